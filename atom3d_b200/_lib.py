@@ -76,6 +76,14 @@ _SIGNATURES: dict[str, tuple] = {
             ctypes.POINTER(SignData), c_vp, c_vp, c_u32, c_vp, c_size, c_vp,
         ],
     ),
+    "a3d_bvh_obbs": (c_int, [c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp]),
+    "a3d_udf_obbs": (
+        c_int,
+        [
+            ctypes.POINTER(BvhView), c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp,
+            ctypes.POINTER(SignData), c_vp, c_vp, c_u32, c_vp, c_size, c_vp,
+        ],
+    ),
     "a3d_udf_backward": (c_int, [c_vp, c_i64, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "a3d_morton_encode": (c_int, [c_vp, c_i64, c_vp, c_vp]),
     "a3d_morton_decode": (c_int, [c_vp, c_i64, c_int, c_vp, c_vp]),
@@ -106,6 +114,7 @@ A3D_ERR_WORKSPACE = 2
 A3D_ERR_CUDA = 3
 A3D_ERR_OVERFLOW = 4
 A3D_ERR_TIMEOUT = 5
+A3D_BVH_OBB_BYTES = 128
 A3D_UDF_SORT_QUERIES = 1
 A3D_UDF_ASSUME_SORTED = 2
 A3D_UDF_NO_REUSE = 4

@@ -18,6 +18,7 @@
 #include <math.h>
 
 #include "bvh_layout.cuh"
+#include "bvh_obb.cuh"
 #include "primitives.cuh"
 #include "tri_math.cuh"
 
@@ -84,6 +85,15 @@ __device__ __forceinline__ void cswap(float& da, uint32_t& ra, float& db, uint32
   }
 }
 
+// the same exchange carrying the pruning value e along
+__device__ __forceinline__ void cswap(float& da, uint32_t& ra, float& ea, float& db, uint32_t& rb, float& eb) {
+  if (child_less(db, rb, da, ra)) {
+    float t = da; da = db; db = t;
+    t = ea; ea = eb; eb = t;
+    uint32_t u = ra; ra = rb; rb = u;
+  }
+}
+
 __device__ __forceinline__ float box_dist_sq(float px, float py, float pz, float lx, float ly, float lz, float hx,
                                              float hy, float hz) {
   const float dx = fmaxf(fmaxf(lx - px, px - hx), 0.f);
@@ -131,6 +141,8 @@ struct TreeT {
   uint32_t num_nodes;
   uint32_t num_tris;
   uint32_t* fault;
+  const ObbNode* __restrict__ obbs;  // nullptr: none
+  uint32_t num_obbs;                  // a node past them has none
   __device__ __forceinline__ const int4* node(uint32_t ref) const {
     if (kGuard && ref >= num_nodes) {
       atomicOr(fault, kFaultNode);
@@ -434,9 +446,12 @@ __global__ void __launch_bounds__(kUdfThreads)
 
 
 
+// Box distance d and reference r of child c, and the value e >= d that prunes
+// it: the larger of the box and the oriented-box distance.  The oriented box
+// is read only for a child whose box still qualifies against `best`.
 template <typename Tree>
-__device__ __forceinline__ void quad_child_box(const Tree& T, uint32_t ref, int c, float px,
-                                               float py, float pz, float& d, uint32_t& r) {
+__device__ __forceinline__ void quad_child_box(const Tree& T, uint32_t ref, int c, float px, float py, float pz,
+                                               float best, float& d, uint32_t& r, float& e) {
   const int4* np = T.node(ref);
   const int4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3);
   const uint32_t meta = (uint32_t)w0.w;
@@ -453,6 +468,10 @@ __device__ __forceinline__ void quad_child_box(const Tree& T, uint32_t ref, int 
   const float hz = dequant((uint32_t)w2.y, c, sz, oz);
   r = c == 0 ? (uint32_t)w2.z : (c == 1 ? (uint32_t)w2.w : (c == 2 ? (uint32_t)w3.x : (uint32_t)w3.y));
   d = c < nch ? box_dist_sq(px, py, pz, lx, ly, lz, hx, hy, hz) : INFINITY;
+  e = d;
+  if (d < best && ref < T.num_obbs) {
+    e = fmaxf(d, obb_dist_sq(T.obbs[ref].child + c, px - ox, py - oy, pz - oz));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -497,10 +516,12 @@ constexpr int kFinCap = 64;
 
 struct TaskSmem {
   uint2 stack[kTaskDepth][32];
-  float4 p[32];  // owners' query points (w unused): one 16-B read per task
+  float4 p[32];  // owners' query points and, in w, the best squared distance
+                 // that prunes children (0 while probing): one 16-B read per task
   uint32_t nref[32];
   uint8_t nown[32];
   uint2 box[32 * kBoxStride];  // (distance bits, child ref) per child-box task
+  float boxe[32 * kBoxStride];  // the value that prunes the child (both boxes)
   uint32_t tidx[kTaskTriCap];
   uint8_t town[kTaskTriCap];  // owner lane | position in its leaf << 5
   float trid[kMaxLeafTris * kTriRow];
@@ -559,7 +580,7 @@ __global__ void __maxnreg__(kTaskMaxRegs)
     qi = perm ? (int64_t)perm[k] : k;
     root = kBatch ? sel.root_of(qi) : 0u;
     px = pts[3 * qi]; py = pts[3 * qi + 1]; pz = pts[3 * qi + 2];
-    S.p[lane] = make_float4(px, py, pz, 0.f);
+    float prune = 0.f;  // a probe or seed item prunes nothing
     bsq = INFINITY;
     if (bound) {
       const float b = bound[qi];
@@ -575,6 +596,7 @@ __global__ void __maxnreg__(kTaskMaxRegs)
     reused = false;
     if ((seeding & kSeedBoundOnly) && bsq < INFINITY) {
       best_sq = bsq;
+      prune = bsq;
       phase = kTrav;
       ref = root;
       have = true;
@@ -588,6 +610,7 @@ __global__ void __maxnreg__(kTaskMaxRegs)
       ref = root;
       have = true;
     }
+    S.p[lane] = make_float4(px, py, pz, prune);
     kprev = k;
     if (kBatch) prev_root = root;
   };
@@ -644,6 +667,7 @@ __global__ void __maxnreg__(kTaskMaxRegs)
       // of handing it to the deep-stack re-run kernel
       bsq = INFINITY;
       best_sq = INFINITY;
+      S.p[lane].w = 0.f;
       sp = 0;
       gsp = 0;
       if (reused) {
@@ -716,11 +740,12 @@ __global__ void __maxnreg__(kTaskMaxRegs)
     for (int t = lane; t < 4 * nnodes; t += 32) {
       const int r = t >> 2, c = t & 3;
       const int o = S.nown[r];
-      float d;
+      float d, e;
       uint32_t cr;
       const float4 q = S.p[o];
-      quad_child_box(T, S.nref[r], c, q.x, q.y, q.z, d, cr);
+      quad_child_box(T, S.nref[r], c, q.x, q.y, q.z, q.w, d, cr, e);
       S.box[r * kBoxStride + c] = make_uint2(__float_as_uint(d), cr);
+      S.boxe[r * kBoxStride + c] = e;
     }
     for (int t = lane; t < ttotal; t += 32) {
       const uint32_t op = S.town[t];
@@ -731,13 +756,14 @@ __global__ void __maxnreg__(kTaskMaxRegs)
     __syncwarp();
     // (d) owners consume their results
     if (is_node) {
-      float d[4];
+      float d[4], e[4];
       uint32_t r[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const uint2 e = S.box[kBoxStride * nrank + c];
-        d[c] = __uint_as_float(e.x);
-        r[c] = e.y;
+        const uint2 b = S.box[kBoxStride * nrank + c];
+        d[c] = __uint_as_float(b.x);
+        r[c] = b.y;
+        e[c] = S.boxe[kBoxStride * nrank + c];
       }
       if (phase == kProbe) {
         // greedy: the (distance, ref)-smallest child
@@ -748,11 +774,17 @@ __global__ void __maxnreg__(kTaskMaxRegs)
           if (child_less(d[c], r[c], bd, br)) { bd = d[c]; br = r[c]; }
         ref = br;
       } else {
-        cswap(d[0], r[0], d[1], r[1]);
-        cswap(d[2], r[2], d[3], r[3]);
-        cswap(d[0], r[0], d[2], r[2]);
-        cswap(d[1], r[1], d[3], r[3]);
-        cswap(d[1], r[1], d[2], r[2]);
+        // a child is dropped by e (both boxes), visited in order of d (the
+        // axis-aligned box alone), so the oriented boxes change which children are visited, never
+        // their order
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (!(e[c] < best_sq)) d[c] = INFINITY;
+        cswap(d[0], r[0], e[0], d[1], r[1], e[1]);
+        cswap(d[2], r[2], e[2], d[3], r[3], e[3]);
+        cswap(d[0], r[0], e[0], d[2], r[2], e[2]);
+        cswap(d[1], r[1], e[1], d[3], r[3], e[3]);
+        cswap(d[1], r[1], e[1], d[2], r[2], e[2]);
         int q = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) q += d[c] < best_sq ? 1 : 0;
@@ -771,7 +803,7 @@ __global__ void __maxnreg__(kTaskMaxRegs)
           } else {
 #pragma unroll
             for (int c = 3; c >= 1; --c)
-              if (c < q) S.stack[sp++][lane] = make_uint2(r[c], __float_as_uint(d[c]));
+              if (c < q) S.stack[sp++][lane] = make_uint2(r[c], __float_as_uint(e[c]));
             ref = r[0];
           }
         } else {
@@ -786,13 +818,18 @@ __global__ void __maxnreg__(kTaskMaxRegs)
         if (dd < dmin) { dmin = dd; imin = f0 + (uint32_t)i; }
       }
       if (phase == kTrav) {
-        if (dmin < best_sq) { best_sq = dmin; best_tri = imin; }
+        if (dmin < best_sq) {
+          best_sq = dmin;
+          best_tri = imin;
+          S.p[lane].w = dmin;
+        }
         have = false;
       } else {
         // probe leaf or seed triangle: radius just above its distance
         float b = dmin < INFINITY ? nextafterf(dmin, INFINITY) : INFINITY;
         if (bsq < b) b = bsq;
         best_sq = b;
+        S.p[lane].w = b;
         phase = kTrav;
         ref = root;
         have = true;
@@ -1019,7 +1056,15 @@ extern "C" size_t a3d_udf_workspace_bytes(int64_t num_points, uint32_t flags) {
 extern "C" int a3d_udf(const a3d_bvh_view* bvh, const float* points, int64_t num_points, float* distances,
                        int32_t* face_ids, float* closest_points, float* uvw, const a3d_sign_data* sign,
                        const float* bound, unsigned long long* stats, uint32_t flags, void* workspace,
-                       size_t workspace_bytes, a3d_stream_t stream_) {
+                       size_t workspace_bytes, a3d_stream_t stream) {
+  return a3d_udf_obbs(bvh, nullptr, points, num_points, distances, face_ids, closest_points, uvw, sign, bound, stats,
+                       flags, workspace, workspace_bytes, stream);
+}
+
+extern "C" int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const float* points, int64_t num_points,
+                             float* distances, int32_t* face_ids, float* closest_points, float* uvw,
+                             const a3d_sign_data* sign, const float* bound, unsigned long long* stats, uint32_t flags,
+                             void* workspace, size_t workspace_bytes, a3d_stream_t stream_) {
   cudaStream_t s = (cudaStream_t)stream_;
   A3D_REQUIRE(bvh && bvh->nodes && bvh->tris && bvh->num_nodes > 0, A3D_ERR_ARGUMENT, "udf: invalid bvh");
   A3D_REQUIRE(num_points >= 0 && num_points < (1ll << 32), A3D_ERR_ARGUMENT, "udf: bad number of points");
@@ -1064,7 +1109,8 @@ extern "C" int a3d_udf(const a3d_bvh_view* bvh, const float* points, int64_t num
                            ((flags & A3D_UDF_BOUND_SEEDS) && bound ? kSeedBoundOnly : 0u);
   A3D_CUDA_TRY(cudaMemsetAsync(w.nrerun, 0, kStatusWords * sizeof(uint32_t), s));
   const TreeT<false> T{(const WideNode*)bvh->nodes, (const TriRec*)bvh->tris, (uint32_t)bvh->num_nodes,
-                       (uint32_t)bvh->num_tris, w.nrerun + 3};
+                       (uint32_t)bvh->num_tris, w.nrerun + 3, (const ObbNode*)obbs,
+                       obbs != nullptr ? (uint32_t)bvh->num_nodes : 0u};
   const MeshSel sel{nullptr, nullptr, 1, 0};
   const TaskShape shape{kTaskPool, 0};
   QueryOut out{distances, face_ids, closest_points, uvw};
@@ -1166,7 +1212,7 @@ size_t batch_udf_bytes(int64_t n) {
   return base + (size_t)spill_owner_bound(c) * kSpillCap * sizeof(uint2) + 512;
 }
 
-int batch_udf(const a3d_bvh_batch* bvh, const float* points, const int64_t* qoff, int64_t n, float* distances,
+int batch_udf(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points, const int64_t* qoff, int64_t n, float* distances,
               int32_t* face_ids, float* closest_points, float* uvw, TaskShape shape, unsigned long long* stats,
               void* workspace, size_t workspace_bytes, cudaStream_t s) {
   A3D_REQUIRE(bvh && bvh->nodes && bvh->tris && bvh->roots && bvh->bounds && bvh->num_meshes > 0 &&
@@ -1195,7 +1241,8 @@ int batch_udf(const a3d_bvh_batch* bvh, const float* points, const int64_t* qoff
   A3D_REQUIRE(points && qoff && distances && face_ids && closest_points, A3D_ERR_ARGUMENT, "batch_udf: null pointer");
   // the node count is only known on the device: guard with the capacity
   const TreeT<true> T{(const WideNode*)bvh->nodes, (const TriRec*)bvh->tris, (uint32_t)bvh->num_faces,
-                      (uint32_t)bvh->num_faces, w.nrerun + 3};
+                      (uint32_t)bvh->num_faces, w.nrerun + 3, (const ObbNode*)obbs,
+                      obbs != nullptr ? (uint32_t)num_obbs : 0u};
   const SignArgs sg{nullptr, nullptr, nullptr, nullptr, nullptr};
   for (int64_t base = 0; base < n; base += kBatchChunk) {
     const int64_t cn = n - base < kBatchChunk ? n - base : kBatchChunk;
@@ -1281,6 +1328,16 @@ extern "C" int a3d_batch_udf(const a3d_bvh_batch* bvh, const float* points, cons
                              int64_t num_queries, float* distances, int32_t* face_ids, float* closest_points,
                              float* uvw, const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
                              size_t workspace_bytes, a3d_stream_t stream) {
+  return a3d_batch_udf_obbs(bvh, nullptr, 0, points, query_offsets, num_queries, distances, face_ids, closest_points,
+                             uvw, tuning, stats, workspace, workspace_bytes, stream);
+}
+
+extern "C" int a3d_batch_udf_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points,
+                                   const int64_t* query_offsets, int64_t num_queries, float* distances,
+                                   int32_t* face_ids, float* closest_points, float* uvw,
+                                   const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
+                                   size_t workspace_bytes, a3d_stream_t stream) {
+  A3D_REQUIRE(num_obbs >= 0 && num_obbs < (1ll << 31), A3D_ERR_ARGUMENT, "batch_udf: bad oriented-box count");
   a3d::TaskShape shape{a3d::kTaskPool, 0};
   if (tuning) {
     A3D_REQUIRE(tuning->pool >= 0 && tuning->pool <= 4096 && tuning->blocks_per_sm >= 0, A3D_ERR_ARGUMENT,
@@ -1288,7 +1345,7 @@ extern "C" int a3d_batch_udf(const a3d_bvh_batch* bvh, const float* points, cons
     if (tuning->pool > 0) shape.pool = tuning->pool;
     shape.blocks_per_sm = tuning->blocks_per_sm;
   }
-  return a3d::batch_udf(bvh, points, query_offsets, num_queries, distances, face_ids, closest_points, uvw, shape,
+  return a3d::batch_udf(bvh, obbs, num_obbs, points, query_offsets, num_queries, distances, face_ids, closest_points, uvw, shape,
                         stats, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -1301,7 +1358,15 @@ extern "C" size_t a3d_batch_autotune_workspace_bytes(int64_t sample_queries, int
 extern "C" int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points, const int64_t* query_offsets,
                                   int64_t num_queries, int64_t sample_queries, void* workspace,
                                   size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,
-                                  a3d_stream_t stream_) {
+                                  a3d_stream_t stream) {
+  return a3d_batch_autotune_obbs(bvh, nullptr, 0, points, query_offsets, num_queries, sample_queries, workspace,
+                                  workspace_bytes, best, best_ms, stream);
+}
+
+extern "C" int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs,
+                                        const float* points, const int64_t* query_offsets, int64_t num_queries,
+                                        int64_t sample_queries, void* workspace, size_t workspace_bytes,
+                                        a3d_udf_tuning* best, float* best_ms, a3d_stream_t stream_) {
   using namespace a3d;
   cudaStream_t s = (cudaStream_t)stream_;
   A3D_REQUIRE(bvh && points && query_offsets && best && num_queries > 0 && sample_queries > 0, A3D_ERR_ARGUMENT,
@@ -1339,7 +1404,7 @@ extern "C" int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points,
       for (int rep = 0; rep < 3 && rc == A3D_OK; ++rep) {
         if (rep == 1 && cudaEventRecord(e0, s) != cudaSuccess) rc = A3D_ERR_CUDA;
         if (rc == A3D_OK)
-          rc = batch_udf(bvh, t.pts, t.qoff, ns, t.dist, t.fid, t.cp, nullptr, shape, nullptr, t.udf_ws, t.udf_bytes,
+          rc = batch_udf(bvh, obbs, num_obbs, t.pts, t.qoff, ns, t.dist, t.fid, t.cp, nullptr, shape, nullptr, t.udf_ws, t.udf_bytes,
                          s);
       }
       float ms = 0.f;

@@ -351,8 +351,8 @@ def main():
     stream = torch.cuda.current_stream(dev)
 
     def step(stats=None):
-        _lib.call("a3d_udf", ctypes.byref(view), qd.data_ptr(), n, dist_o.data_ptr(), fid_o.data_ptr(),
-                  cp_o.data_ptr(), None, None, None, _lib.ptr(stats), flags, ws.data_ptr(), ws.numel(),
+        _lib.call("a3d_udf_obbs", ctypes.byref(view), bvh.obbs.data_ptr(), qd.data_ptr(), n,
+                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, _lib.ptr(stats), flags, ws.data_ptr(), ws.numel(),
                   stream.cuda_stream)
 
     # traversal statistics of our tree (one untimed pass)
@@ -964,8 +964,8 @@ def time_traversal_kernel(bvh, qd, dist_o, fid_o, cp_o, ws, flags, stream, steps
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
 
     def call():
-        _lib.call("a3d_udf", ctypes.byref(view), qs.data_ptr(), n, dist_o.data_ptr(), fid_o.data_ptr(),
-                  cp_o.data_ptr(), None, None, None, None, _lib.A3D_UDF_ASSUME_SORTED | (flags & ~_lib.A3D_UDF_SORT_QUERIES),
+        _lib.call("a3d_udf_obbs", ctypes.byref(view), bvh.obbs.data_ptr(), qs.data_ptr(), n,
+                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, None, _lib.A3D_UDF_ASSUME_SORTED | (flags & ~_lib.A3D_UDF_SORT_QUERIES),
                   ws.data_ptr(), ws.numel(),
                   stream.cuda_stream)
 

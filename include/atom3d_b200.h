@@ -68,6 +68,19 @@ int a3d_bvh_build(const float* vertices, int64_t num_vertices,
                   float* bounds_out /* host, 6 floats: lo xyz, hi xyz */,
                   a3d_stream_t stream);
 
+/* Oriented boxes of a finished tree (no counterpart in the reference): per
+ * child of every node the extent of its triangles in a frame along their mean
+ * normal, a lower bound on the distance that is far tighter than the
+ * axis-aligned box on smooth surfaces.  obbs_out: num_nodes x
+ * A3D_BVH_OBB_BYTES, 16-B aligned.  For a batch, num_nodes is the node
+ * capacity of obbs_out and num_nodes_device (nullable) a3d_batch_build's
+ * device count.  a3d_udf_obbs and a3d_batch_udf_obbs take them; results never
+ * depend on them. */
+#define A3D_BVH_OBB_BYTES 128
+int a3d_bvh_obbs(const void* nodes, const void* tris, int64_t num_nodes,
+                  const int64_t* num_nodes_device, int64_t num_tris, void* obbs_out,
+                  a3d_stream_t stream);
+
 /* ---- pseudo-normal precompute for the SDF sign -------------------------- */
 /* Replaces MeshBVH._precompute_face_normals and
  * MeshBVH._precompute_pseudo_normal_data (atom3d/core/mesh_bvh.py:129-232).
@@ -122,6 +135,14 @@ int a3d_udf(const a3d_bvh_view* bvh, const float* points, int64_t num_points,
             float* uvw, const a3d_sign_data* sign, const float* bound,
             unsigned long long* stats, uint32_t flags,
             void* workspace, size_t workspace_bytes, a3d_stream_t stream);
+
+/* a3d_udf with the tree's oriented boxes (a3d_bvh_obbs; NULL: none): the
+ * same results from fewer tests. */
+int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const float* points, int64_t num_points,
+                  float* distances, int32_t* face_ids, float* closest_points,
+                  float* uvw, const a3d_sign_data* sign, const float* bound,
+                  unsigned long long* stats, uint32_t flags,
+                  void* workspace, size_t workspace_bytes, a3d_stream_t stream);
 
 /* Allocation-free variant of a3d_udf (no counterpart in the reference).
  * For callers that may not call cudaMalloc (a host application owning all
@@ -531,6 +552,13 @@ int a3d_batch_udf(const a3d_bvh_batch* bvh, const float* points, const int64_t* 
                   int64_t num_queries, float* distances, int32_t* face_ids, float* closest_points,
                   float* uvw, const a3d_udf_tuning* tuning, unsigned long long* stats,
                   void* workspace, size_t workspace_bytes, a3d_stream_t stream);
+/* the same with the batch's oriented boxes (num_obbs records; nodes past
+ * them have none) */
+int a3d_batch_udf_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points,
+                        const int64_t* query_offsets, int64_t num_queries, float* distances,
+                        int32_t* face_ids, float* closest_points, float* uvw,
+                        const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
+                        size_t workspace_bytes, a3d_stream_t stream);
 /* Times the traversal's launch shapes on every ceil(Q/sample)-th query
  * (sample <= 16,777,216) and returns the fastest (host-synchronous; not
  * inside stream capture). */
@@ -539,6 +567,11 @@ int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points, const int6
                        int64_t num_queries, int64_t sample_queries, void* workspace,
                        size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,
                        a3d_stream_t stream);
+int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs,
+                             const float* points, const int64_t* query_offsets,
+                             int64_t num_queries, int64_t sample_queries, void* workspace,
+                             size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,
+                             a3d_stream_t stream);
 
 /* ---- learned distance bound (no counterpart in the reference) ----------- */
 /* A Fourier-feature MLP (3 -> 64 -> 128 -> 128 -> 128 -> 1, ReLU) predicts
