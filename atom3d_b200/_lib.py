@@ -76,8 +76,9 @@ _SIGNATURES: dict[str, tuple] = {
             ctypes.POINTER(SignData), c_vp, c_vp, c_u32, c_vp, c_size, c_vp,
         ],
     ),
-    "a3d_bvh_obbs": (c_int, [c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp]),
-    "a3d_udf_obbs": (
+    "a3d_bvh_children_bytes": (c_size, [c_i64, c_i64]),
+    "a3d_bvh_children": (c_int, [c_vp, c_vp, c_i64, c_vp, c_i64, c_vp, c_vp]),
+    "a3d_udf_children": (
         c_int,
         [
             ctypes.POINTER(BvhView), c_vp, c_vp, c_i64, c_vp, c_vp, c_vp, c_vp,
@@ -114,7 +115,6 @@ A3D_ERR_WORKSPACE = 2
 A3D_ERR_CUDA = 3
 A3D_ERR_OVERFLOW = 4
 A3D_ERR_TIMEOUT = 5
-A3D_BVH_OBB_BYTES = 128
 A3D_UDF_SORT_QUERIES = 1
 A3D_UDF_ASSUME_SORTED = 2
 A3D_UDF_NO_REUSE = 4

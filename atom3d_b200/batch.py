@@ -48,11 +48,12 @@ _SIGS = {
     "a3d_batch_build": (ctypes.c_int, [_vp, _vp, _vp, _vp, _i32, _i64, ctypes.c_int, _vp, _vp, _vp, _vp, _vp, _vp,
                                        _vp, _sz, _vp]),
     "a3d_batch_udf_workspace_bytes": (_sz, [_i64, _i32]),
-    "a3d_batch_udf_obbs": (ctypes.c_int, [ctypes.POINTER(BvhBatch), _vp, _i64, _vp, _vp, _i64, _vp, _vp, _vp, _vp,
-                                          ctypes.POINTER(UdfTuning), _vp, _vp, _sz, _vp]),
+    "a3d_batch_udf_children": (ctypes.c_int, [ctypes.POINTER(BvhBatch), _vp, _i64, _vp, _vp, _i64, _vp, _vp, _vp,
+                                              _vp, ctypes.POINTER(UdfTuning), _vp, _vp, _sz, _vp]),
     "a3d_batch_autotune_workspace_bytes": (_sz, [_i64, _i32]),
-    "a3d_batch_autotune_obbs": (ctypes.c_int, [ctypes.POINTER(BvhBatch), _vp, _i64, _vp, _vp, _i64, _i64, _vp, _sz,
-                                               ctypes.POINTER(UdfTuning), ctypes.POINTER(ctypes.c_float), _vp]),
+    "a3d_batch_autotune_children": (ctypes.c_int, [ctypes.POINTER(BvhBatch), _vp, _i64, _vp, _vp, _i64, _i64, _vp,
+                                                   _sz, ctypes.POINTER(UdfTuning), ctypes.POINTER(ctypes.c_float),
+                                                   _vp]),
 }
 
 
@@ -115,12 +116,13 @@ class BatchedMeshBVH:
         dev = self.device
         self.nodes = _aligned(n * 64, 64, dev)
         self.tris = _aligned(n * 64, 64, dev)
-        # oriented boxes (the traversal's second lower bound) for the first
-        # num_obbs nodes: the node count is only known on the device, and
-        # stays well below half the faces at the leaf sizes in use; deeper
+        # child records (decoded boxes and discs for the traversal) of the first
+        # num_children nodes: the node count is only known on the device, and
+        # stays below a quarter of the faces at the leaf sizes in use; deeper
         # nodes go without
-        self.num_obbs = n // 2 + 64
-        self.obbs = torch.empty(self.num_obbs * _lib.A3D_BVH_OBB_BYTES, dtype=torch.uint8, device=dev)
+        self.num_children = n // 4 + 64
+        self.children = torch.empty(_lib.lib().a3d_bvh_children_bytes(self.num_children, n), dtype=torch.uint8,
+                                    device=dev)
         self.roots = torch.zeros(m, dtype=torch.int32, device=dev)
         self.bounds = torch.zeros(m, 6, dtype=torch.float32, device=dev)
         self.num_nodes = torch.zeros(1, dtype=torch.int64, device=dev)
@@ -142,8 +144,8 @@ class BatchedMeshBVH:
             self.num_meshes, self.num_faces, self.leaf_max, self.nodes.data_ptr(), self.tris.data_ptr(),
             self.roots.data_ptr(), self.bounds.data_ptr(), self.num_nodes.data_ptr(), self.build_status.data_ptr(),
             self._build_ws.data_ptr(), self._build_ws.numel(), _lib.stream_ptr(self.device)))
-        _lib.call("a3d_bvh_obbs", self.nodes.data_ptr(), self.tris.data_ptr(), self.num_obbs,
-                  self.num_nodes.data_ptr(), self.num_faces, self.obbs.data_ptr(), _lib.stream_ptr(self.device))
+        _lib.call("a3d_bvh_children", self.nodes.data_ptr(), self.tris.data_ptr(), self.num_children,
+                  self.num_nodes.data_ptr(), self.num_faces, self.children.data_ptr(), _lib.stream_ptr(self.device))
 
     def check(self) -> None:
         """Read the build's device status (synchronises)."""
@@ -169,10 +171,10 @@ class BatchedMeshBVH:
             raise ValueError("points must be contiguous float32 [Q,3]")
         ws = self._workspace(nq)
         t = tuning if tuning is not None else self.tuning
-        _lib.check("a3d_batch_udf", _bind().a3d_batch_udf_obbs(
-            ctypes.byref(self.view), self.obbs.data_ptr(), self.num_obbs, points.data_ptr(), query_offsets.data_ptr(),
-            nq, dist.data_ptr(), fid.data_ptr(), cp.data_ptr(), _lib.ptr(uvw), ctypes.byref(t), _lib.ptr(stats),
-            ws.data_ptr(), ws.numel(), _lib.stream_ptr(self.device)))
+        _lib.check("a3d_batch_udf", _bind().a3d_batch_udf_children(
+            ctypes.byref(self.view), self.children.data_ptr(), self.num_children, points.data_ptr(),
+            query_offsets.data_ptr(), nq, dist.data_ptr(), fid.data_ptr(), cp.data_ptr(), _lib.ptr(uvw),
+            ctypes.byref(t), _lib.ptr(stats), ws.data_ptr(), ws.numel(), _lib.stream_ptr(self.device)))
 
     def query_status(self) -> dict:
         """Status words of the last query (synchronises): queries re-run,
@@ -215,9 +217,10 @@ class BatchedMeshBVH:
             self.check()
             t = UdfTuning()
             ms = ctypes.c_float(0.0)
-            _lib.check("a3d_batch_autotune", lib.a3d_batch_autotune_obbs(
-                ctypes.byref(self.view), self.obbs.data_ptr(), self.num_obbs, points.data_ptr(),
-                query_offsets.data_ptr(), nq, ns, ws.data_ptr(), ws.numel(), ctypes.byref(t), ctypes.byref(ms), _lib.stream_ptr(self.device)))
+            _lib.check("a3d_batch_autotune", lib.a3d_batch_autotune_children(
+                ctypes.byref(self.view), self.children.data_ptr(), self.num_children, points.data_ptr(),
+                query_offsets.data_ptr(), nq, ns, ws.data_ptr(), ws.numel(), ctypes.byref(t), ctypes.byref(ms),
+                _lib.stream_ptr(self.device)))
             t.leaf_max = int(lm)
             seen[int(lm)] = {"sample_ms": float(ms.value), **t.as_dict()}
             if best is None or ms.value < best[0] * self._leaf_margin(int(lm), best[1].leaf_max):
@@ -232,8 +235,8 @@ class BatchedMeshBVH:
     def _leaf_margin(lm: int, best: int) -> float:
         """How much faster a leaf size must be than the best so far: smaller
         leaves mean more nodes, memory and build time, so a difference within
-        the timings' noise (5%) goes to the larger leaf (with the oriented
-        boxes leaves of 2 and 4 are within 2% of each other on small samples,
+        the timings' noise (5%) goes to the larger leaf (with the child
+        records leaves of 2 and 4 are within 2% of each other on small samples,
         0.325 and 0.331 ms)."""
         return 0.95 if lm < best else 1.05 if lm > best else 1.0
 

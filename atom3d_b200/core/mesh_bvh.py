@@ -60,10 +60,11 @@ class WideBVH:
             self.num_nodes = int(nn.value)
             self.nodes = nodes[: self.num_nodes * 64]
             self.tris = tris
-            # oriented boxes: the closest-point traversal's second lower bound
-            self.obbs = torch.empty(self.num_nodes * _lib.A3D_BVH_OBB_BYTES, dtype=torch.uint8, device=dev)
-            _lib.call("a3d_bvh_obbs", self.nodes.data_ptr(), self.tris.data_ptr(), self.num_nodes, None, nf,
-                      self.obbs.data_ptr(), _lib.stream_ptr(dev))
+            # child records: decoded boxes and discs for the closest-point traversal
+            self.children = torch.empty(_lib.lib().a3d_bvh_children_bytes(self.num_nodes, nf), dtype=torch.uint8,
+                                        device=dev)
+            _lib.call("a3d_bvh_children", self.nodes.data_ptr(), self.tris.data_ptr(), self.num_nodes, None, nf,
+                      self.children.data_ptr(), _lib.stream_ptr(dev))
         self.lo = [bounds[0], bounds[1], bounds[2]]
         self.hi = [bounds[3], bounds[4], bounds[5]]
         self._view = _lib.BvhView(
@@ -98,7 +99,7 @@ class WideBVH:
             if b.shape[0] != n:
                 raise ValueError("bound must have one entry per query")
         _lib.call(
-            "a3d_udf_obbs", ctypes.byref(self._view), self.obbs.data_ptr(), p.data_ptr(), n, dist.data_ptr(), fid.data_ptr(), cp.data_ptr(),
+            "a3d_udf_children", ctypes.byref(self._view), self.children.data_ptr(), p.data_ptr(), n, dist.data_ptr(), fid.data_ptr(), cp.data_ptr(),
             _lib.ptr(uvw), ctypes.byref(sign) if sign is not None else None, _lib.ptr(b), _lib.ptr(stats), flags,
             ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev),
         )

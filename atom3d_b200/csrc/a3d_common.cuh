@@ -103,6 +103,19 @@ struct Workspace {
   __host__ bool ok() const { return measuring || used <= size; }
 };
 
+// 32 bytes of read-only global memory in one load (32-byte aligned): half the
+// L1 requests of two 16-byte loads where every lane reads its own record
+__device__ __forceinline__ void ldg256(const void* p, int4& a, int4& b) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+      : "l"(p));
+}
+__device__ __forceinline__ void ldg256(const void* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
 // float <-> order-preserving uint32 (for atomic min/max on floats)
 __device__ __forceinline__ uint32_t float_flip(float f) {
   uint32_t u = __float_as_uint(f);

@@ -6,19 +6,22 @@
 // 759-827).  Design:
 //   * queries are Morton-sorted (30-bit key, in-house radix sort) so a warp
 //     walks neighbouring regions of the tree together;
-//   * one 64-B node = four 16-B loads; the four child boxes are decoded from
-//     8-bit offsets, sorted by distance with a 5-exchange network, the
-//     nearest qualifying child is visited next and the others pushed;
-//   * the traversal stack lives in shared memory ([depth][thread] layout, no
-//     bank conflicts); a query that would overflow it is re-run by a
-//     fallback launch with a deep local-memory stack, never truncated;
+//   * a group of four or two lanes walks the tree for one query: each lane
+//     tests one or two of a node's children, first the box, then the disc
+//     about the child's triangles (bvh_children.cuh); the nearest qualifying
+//     child by box distance is visited next and the others pushed;
+//   * the traversal stack lives in shared memory and continues in the
+//     workspace; a query that would overflow both is re-run by a launch with a
+//     deep local-memory stack, never truncated;
 //   * a per-query bound (learned upper bound on the distance) seeds the
-//     pruning radius; a query whose bound proves too small is re-run
-//     without it, so results are identical with and without the bound.
+//     pruning radius; a query whose bound proves too small is run again
+//     without it, so results are identical with and without the bound;
+//   * the traversal leaves (triangle, squared distance) per query, and a
+//     second kernel makes the closest point, barycentrics and sign of them.
 #include <math.h>
 
 #include "bvh_layout.cuh"
-#include "bvh_obb.cuh"
+#include "bvh_children.cuh"
 #include "primitives.cuh"
 #include "tri_math.cuh"
 
@@ -43,6 +46,14 @@ struct QueryOut {
   int32_t* fid;
   float* cp;
   float* uvw;
+};
+
+// the traversals' results, by the queries' place in the sorted order: closest
+// triangle (0xffffffff: none) and squared distance, turned into the caller's
+// outputs by udf_finish_kernel
+struct Best {
+  uint32_t* tri;
+  float* sq;
 };
 
 struct Counters {
@@ -81,15 +92,6 @@ __device__ __forceinline__ bool child_less(float da, uint32_t ra, float db, uint
 __device__ __forceinline__ void cswap(float& da, uint32_t& ra, float& db, uint32_t& rb) {
   if (child_less(db, rb, da, ra)) {
     float t = da; da = db; db = t;
-    uint32_t u = ra; ra = rb; rb = u;
-  }
-}
-
-// the same exchange carrying the pruning value e along
-__device__ __forceinline__ void cswap(float& da, uint32_t& ra, float& ea, float& db, uint32_t& rb, float& eb) {
-  if (child_less(db, rb, da, ra)) {
-    float t = da; da = db; db = t;
-    t = ea; ea = eb; eb = t;
     uint32_t u = ra; ra = rb; rb = u;
   }
 }
@@ -141,8 +143,8 @@ struct TreeT {
   uint32_t num_nodes;
   uint32_t num_tris;
   uint32_t* fault;
-  const ObbNode* __restrict__ obbs;  // nullptr: none
-  uint32_t num_obbs;                  // a node past them has none
+  ChildRecs children;
+  uint32_t num_children;  // a node past them has no records (0: none at all)
   __device__ __forceinline__ const int4* node(uint32_t ref) const {
     if (kGuard && ref >= num_nodes) {
       atomicOr(fault, kFaultNode);
@@ -258,7 +260,7 @@ __device__ __forceinline__ bool traverse(const Tree& T, float px, float py, floa
   }
 }
 
-__device__ __noinline__ void finish_query(const TriRec* __restrict__ tris, uint32_t num_tris, uint32_t best_tri,
+__device__ __forceinline__ void finish_query(const TriRec* __restrict__ tris, uint32_t num_tris, uint32_t best_tri,
                                           float best_sq,
                                              float px, float py, float pz, int64_t qi, const QueryOut& out,
                                              const SignArgs& sg, bool do_sign) {
@@ -386,12 +388,11 @@ __device__ __forceinline__ void probe(const Tree& T, float px, float py, float p
 // distance some tested triangle already beats or ties earlier in the same
 // nearest-first order.  An external bound, when given, tightens the radius
 // further; if it excludes every triangle the query is re-run unbounded.
-template <bool kSign, bool kStats>
+template <bool kStats>
 __global__ void __launch_bounds__(kUdfThreads)
     udf_kernel(TreeT<false> T, const float* __restrict__ pts,
                int64_t n, int chunk, const uint32_t* __restrict__ perm, const float* __restrict__ bound,
-               QueryOut out, SignArgs sg, unsigned long long* stats, uint32_t* __restrict__ rerun,
-               uint32_t* __restrict__ nrerun) {
+               Best out, unsigned long long* stats, uint32_t* __restrict__ rerun, uint32_t* __restrict__ nrerun) {
   pdl_wait();
   __shared__ uint2 s_stack[kSharedDepth * kUdfThreads];
   __shared__ uint32_t s_next[kUdfThreads / 32];
@@ -430,10 +431,11 @@ __global__ void __launch_bounds__(kUdfThreads)
     if (!ok || best_tri == 0xffffffffu) {
       // stack overflow, or an external bound excluded every triangle
       const uint32_t slot = atomicAdd(nrerun, 1u);
-      rerun[slot] = (uint32_t)qi;
+      rerun[slot] = (uint32_t)k;
       prev = 0xffffffffu;
     } else {
-      finish_query(T.tris, T.num_tris, best_tri, best_sq, px, py, pz, qi, out, sg, kSign);
+      out.tri[k] = best_tri;
+      out.sq[k] = best_sq;
       prev = best_tri;
     }
     k = w0 + (int64_t)atomicAdd(&s_next[warp], 1u);
@@ -446,176 +448,174 @@ __global__ void __launch_bounds__(kUdfThreads)
 
 
 
-// Box distance d and reference r of child c, and the value e >= d that prunes
-// it: the larger of the box and the oriented-box distance.  The oriented box
-// is read only for a child whose box still qualifies against `best`.
-template <typename Tree>
-__device__ __forceinline__ void quad_child_box(const Tree& T, uint32_t ref, int c, float px, float py, float pz,
-                                               float best, float& d, uint32_t& r, float& e) {
-  const int4* np = T.node(ref);
-  const int4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3);
+// Children c0 .. c0 + kC - 1 of a node: box distance d, reference r (0xffffffff
+// for no child) and the value e >= d that prunes the child, the larger of the
+// box and the disc distance.  The disc is read only for a child whose box
+// still qualifies against `best`.  ties: bit x - 1 set when the reference of
+// sibling c ^ x is smaller.
+template <bool kRecords, int kC, typename Tree>
+__device__ __forceinline__ void node_child(const Tree& T, uint32_t ref, int c0, float px, float py, float pz,
+                                           float best, float d[kC], uint32_t r[kC], float e[kC], uint32_t ties[kC]) {
+  if (kRecords && ref < T.num_children) {
+    const BoxRec* rec = T.children.boxes + 4 * (size_t)ref + c0;
+    float4 a[kC], b[kC];
+#pragma unroll
+    for (int j = 0; j < kC; ++j) ldg256(rec + j, a[j], b[j]);
+#pragma unroll
+    for (int j = 0; j < kC; ++j) {
+      r[j] = __float_as_uint(b[j].z);
+      ties[j] = __float_as_uint(b[j].w);
+      d[j] = r[j] != 0xffffffffu ? box_dist_sq(px, py, pz, a[j].x, a[j].y, a[j].z, a[j].w, b[j].x, b[j].y) : INFINITY;
+      e[j] = d[j];
+    }
+#pragma unroll
+    for (int j = 0; j < kC; ++j)
+      if (d[j] < best && (ref_is_leaf(r[j]) || r[j] < T.num_children))
+        e[j] = fmaxf(d[j], disc_dist_sq(ref_is_leaf(r[j]) ? T.children.leaf_discs + leaf_first(r[j])
+                                                          : T.children.node_discs + r[j],
+                                        px, py, pz));
+    return;
+  }
+  const WideNode* nd = reinterpret_cast<const WideNode*>(T.node(ref));
+  const int4 w0 = __ldg(reinterpret_cast<const int4*>(nd)), w1 = __ldg(reinterpret_cast<const int4*>(nd) + 1);
+  const int2 w2 = __ldg(reinterpret_cast<const int2*>(nd) + 4);
   const uint32_t meta = (uint32_t)w0.w;
   const int nch = (int)(meta >> 24);
   const float sx = __uint_as_float((meta & 0xffu) << 23);
   const float sy = __uint_as_float(((meta >> 8) & 0xffu) << 23);
   const float sz = __uint_as_float(((meta >> 16) & 0xffu) << 23);
   const float ox = __int_as_float(w0.x), oy = __int_as_float(w0.y), oz = __int_as_float(w0.z);
-  const float lx = dequant((uint32_t)w1.x, c, sx, ox);
-  const float ly = dequant((uint32_t)w1.y, c, sy, oy);
-  const float lz = dequant((uint32_t)w1.z, c, sz, oz);
-  const float hx = dequant((uint32_t)w1.w, c, sx, ox);
-  const float hy = dequant((uint32_t)w2.x, c, sy, oy);
-  const float hz = dequant((uint32_t)w2.y, c, sz, oz);
-  r = c == 0 ? (uint32_t)w2.z : (c == 1 ? (uint32_t)w2.w : (c == 2 ? (uint32_t)w3.x : (uint32_t)w3.y));
-  d = c < nch ? box_dist_sq(px, py, pz, lx, ly, lz, hx, hy, hz) : INFINITY;
-  e = d;
-  if (d < best && ref < T.num_obbs) {
-    e = fmaxf(d, obb_dist_sq(T.obbs[ref].child + c, px - ox, py - oy, pz - oz));
+#pragma unroll
+  for (int j = 0; j < kC; ++j) {
+    const int c = c0 + j;
+    r[j] = __ldg(nd->ref + c);
+    ties[j] = 0;
+#pragma unroll
+    for (int x = 1; x < 4; ++x) ties[j] |= __ldg(nd->ref + (c ^ x)) < r[j] ? 1u << (x - 1) : 0u;
+    const float lx = dequant((uint32_t)w1.x, c, sx, ox);
+    const float ly = dequant((uint32_t)w1.y, c, sy, oy);
+    const float lz = dequant((uint32_t)w1.z, c, sz, oz);
+    const float hx = dequant((uint32_t)w1.w, c, sx, ox);
+    const float hy = dequant((uint32_t)w2.x, c, sy, oy);
+    const float hz = dequant((uint32_t)w2.y, c, sz, oz);
+    d[j] = c < nch ? box_dist_sq(px, py, pz, lx, ly, lz, hx, hy, hz) : INFINITY;
+    e[j] = d[j];
   }
 }
 
 // ---------------------------------------------------------------------------
-// warp task traversal
+// group traversal
 // ---------------------------------------------------------------------------
-// Each lane owns one query (its point, best distance and a stack in shared
-// memory).  Every round, each owner contributes the work of its current item:
-// four child-box tests for an internal node, one triangle test per triangle
-// of a leaf (or of the seed triangle).  The tasks of all 32 owners are packed
-// into dense lists and evaluated by all lanes in lockstep, then each owner
-// consumes its results: sorts the four children by (distance, ref) and
-// pushes the qualifying ones, or folds its triangle distances in order with a
-// strict "<".  The per-query visiting order is therefore the one of the
-// single-lane traversal above and results are identical; only the lane that
-// evaluates each test changes.
-constexpr int kTaskWarps = 2;
-constexpr int kTaskDepth = 32;
-constexpr int kSpillCap = 96;    // per-owner global overflow stack (entries)
-constexpr int kSpillChunk = 16;  // entries moved per spill / refill
-// A spill happens when a node's q <= 4 qualifying children do not fit, i.e.
-// with at least kTaskDepth - 2 entries on the stack, and moves a whole chunk:
-// the stack must then hold a chunk.
-static_assert(kTaskDepth - 2 >= kSpillChunk, "a spill needs a full chunk on the shared stack");
-constexpr int kTaskTriCap = 32 * kMaxLeafTris;
-constexpr int kTaskPool = 64;  // queries per pool taken from the global counter
-// register cap of the task kernel: each of the SM's four sub-partitions
-// holds 16K registers, so 64-thread blocks reach 8 resident blocks (16
-// warps) at <= 128 registers a thread and 9 (18 warps, also the 24 KB
-// shared-memory limit) at <= 96
-#ifndef A3D_TASK_MAX_REGS
-#define A3D_TASK_MAX_REGS 128
-#endif
-constexpr int kTaskMaxRegs = A3D_TASK_MAX_REGS;
+// kG lanes (4 or 2) walk the tree for one query, 32 / kG queries a warp: at a
+// node each lane tests 4 / kG children (box, then disc) and the group orders
+// and pushes them by shuffles; all lanes of a group hold the query's state,
+// so a warp needs few registers and many warps hide the tree's latency.  A
+// warp alternates two phases: node steps for the queries at an inner node
+// while enough of them are, then one leaf step for those that have reached a
+// leaf (or test their seed triangle).  Every query keeps the nearest-first
+// order of traverse(), so results and ties are those of a single walk.
+constexpr int kGroupWarps = 4;
+constexpr int kGroupDepth = 24;  // stack entries of a query in shared memory
+constexpr int kSpillCap = 64;    // further entries in the workspace
+constexpr int kMaxPool = 64;
+constexpr uint32_t kReuseSpan = 64;  // a group's previous result seeds a query this close in the sorted order
+// resident blocks an SM (48 registers at 4 lanes, 64 at 2, no spills in the
+// loops; one block more at 2 lanes spills and triples the time) and queries at
+// a node below which a warp turns to its leaves (16.8M queries, 2 lanes: 37.0,
+// 34.9 and 34.1 ms at 6, 8 and 10 of 16; 4 lanes: 38.0, 35.9 and 35.4 ms at 3,
+// 4 and 5 of 8)
+template <int kG>
+constexpr int kGroupBlocks = kG == 4 ? 10 : 8;
+template <int kG>
+constexpr int kNodeGroups = kG == 4 ? 5 : 10;
 
-// Per-warp shared state.  Child-box results sit at node rank * 5 + child and
-// triangle results at position-in-leaf * 33 + owner, so that the owners'
-// reads in the consume step fall in distinct banks.  Finished queries wait
-// in fin_* and are written out 32 at a time by the whole warp.
-constexpr int kBoxStride = 5;
-constexpr int kTriRow = 33;
-constexpr int kFinCap = 64;
-
-struct TaskSmem {
-  uint2 stack[kTaskDepth][32];
-  float4 p[32];  // owners' query points and, in w, the best squared distance
-                 // that prunes children (0 while probing): one 16-B read per task
-  uint32_t nref[32];
-  uint8_t nown[32];
-  uint2 box[32 * kBoxStride];  // (distance bits, child ref) per child-box task
-  float boxe[32 * kBoxStride];  // the value that prunes the child (both boxes)
-  uint32_t tidx[kTaskTriCap];
-  uint8_t town[kTaskTriCap];  // owner lane | position in its leaf << 5
-  float trid[kMaxLeafTris * kTriRow];
-  uint32_t fin_q[kFinCap];
-  uint32_t fin_tri[kFinCap];
-  float fin_sq[kFinCap];
+template <int kG>
+struct GroupSmem {
+  uint2 stack[32 / kG][kGroupDepth];
+  uint2 own[32 / kG];                     // a leaf step's queries: first triangle less its first task, first lane
+  float trid[32 / kG * kMaxLeafTris];     // distances by task
 };
 
-enum : int { kIdle = 0, kProbe = 1, kSeed = 2, kTrav = 3, kAbandon = 4 };
-// radius seeding of the task kernel
+enum : int { kIdle = 0, kSeed = 1, kTrav = 2, kAbandon = 3 };
+// radius seeding
 enum : uint32_t { kSeedReuse = 1u, kSeedBoundOnly = 2u };
 
-template <bool kSign, bool kStats, bool kBatch>
-__global__ void __maxnreg__(kTaskMaxRegs)
-    udf_task_kernel(TreeT<kBatch> T, const float* __restrict__ pts, int64_t n, const uint32_t* __restrict__ perm,
-                    const float* __restrict__ bound, QueryOut out, SignArgs sg, unsigned long long* stats,
-                    uint32_t* __restrict__ rerun, uint32_t* __restrict__ nrerun, uint32_t* __restrict__ pool_counter,
-                    uint2* __restrict__ spill, int64_t spill_owners, uint32_t seeding, MeshSel sel, int pool) {
+template <int kG, bool kRecords, bool kStats, bool kBatch>
+__global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
+    udf_group_kernel(TreeT<kBatch> T, const float* __restrict__ pts, uint32_t n, const uint32_t* __restrict__ perm,
+                     const float* __restrict__ bound, Best out, unsigned long long* stats,
+                     uint32_t* __restrict__ rerun, uint32_t* __restrict__ nrerun, uint32_t* __restrict__ pool_counter,
+                     uint2* __restrict__ spill, uint32_t spill_owners, uint32_t seeding, MeshSel sel, uint32_t pool,
+                     int groups) {
   pdl_wait();
-  __shared__ TaskSmem smem[kTaskWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  TaskSmem& S = smem[warp];
+  constexpr int kC = 4 / kG;  // children a lane
+  constexpr unsigned lead = kG == 4 ? 0x11111111u : 0x55555555u, gmask = (1u << kG) - 1u;
+  __shared__ GroupSmem<kG> smem[kGroupWarps];
+  const int lane = threadIdx.x & 31, c = lane & (kG - 1), base = lane & ~(kG - 1);
   const unsigned FULL = 0xffffffffu;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  // persistent warps: pools of kTaskPool consecutive (sorted) queries are
-  // taken from a global counter; inside a pool, lanes take queries as they
-  // finish their previous one
-  int64_t pos = 0, end = 0;
+  GroupSmem<kG>& S = smem[threadIdx.x >> 5];
+  uint2* stack = S.stack[lane / kG];
+  // persistent warps: pools of consecutive (sorted) queries are taken from a
+  // global counter; inside a pool, groups take queries as they finish
+  uint32_t pos = 0, end = 0;
   bool exhausted = false;
   Counters ctr{0, 0};
 
-  // owner state
-  int64_t qi = -1, kprev = -(1ll << 40);
+  uint32_t k = 0;  // the query's place in the sorted order
   int phase = kIdle;
   uint32_t ref = 0, prev = 0xffffffffu, best_tri = 0xffffffffu, root = 0u, prev_root = 0u;
   float best_sq = INFINITY, px = 0.f, py = 0.f, pz = 0.f, bsq = INFINITY;
-  bool have = false;
+  bool have = false;    // ref is the item to process
   bool reused = false;  // the query's radius is seeded by the previous query's triangle
+  bool greedy = false;  // descending to the nearest child's leaf for a seed
   int sp = 0;
-  // overflow stack in global memory (the workspace's spill region), used
-  // when the shared stack is full; owners beyond the region have none
-  const int64_t owner = ((int64_t)blockIdx.x * kTaskWarps + warp) * 32 + lane;
-  uint2* my_spill = (spill != nullptr && owner < spill_owners) ? spill + owner * kSpillCap : nullptr;
-  int gsp = 0;
-  int nfin = 0;  // finished queries waiting in S.fin_* (warp-uniform)
   unsigned long long rounds = 0;
 
-  // writes out finished query e of S.fin_*
-  auto finish_entry = [&](int e) {
-    const int64_t q = (int64_t)S.fin_q[e];
-    finish_query(T.tris, T.num_tris, S.fin_tri[e], S.fin_sq[e], pts[3 * q], pts[3 * q + 1], pts[3 * q + 2], q, out,
-                 sg, kSign);
+  // entry i >= kGroupDepth of the query's stack, in the workspace, and the
+  // stack's capacity: kGroupDepth, and kSpillCap more where the workspace has
+  // room for this group
+  auto spill_at = [&](int i) -> uint2* {
+    const uint32_t owner = (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / kG;
+    return spill + (size_t)owner * kSpillCap + (i - kGroupDepth);
+  };
+  auto capacity = [&]() -> int {
+    const uint32_t owner = (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / kG;
+    return owner < spill_owners ? kGroupDepth + kSpillCap : kGroupDepth;
   };
 
-  auto start = [&](int64_t k) {
-    qi = perm ? (int64_t)perm[k] : k;
+  auto start = [&](uint32_t knew) {
+    const uint32_t qi = perm ? perm[knew] : knew;
     root = kBatch ? sel.root_of(qi) : 0u;
-    px = pts[3 * qi]; py = pts[3 * qi + 1]; pz = pts[3 * qi + 2];
-    float prune = 0.f;  // a probe or seed item prunes nothing
+    px = pts[3 * (int64_t)qi]; py = pts[3 * (int64_t)qi + 1]; pz = pts[3 * (int64_t)qi + 2];
     bsq = INFINITY;
     if (bound) {
       const float b = bound[qi];
       if (b * b >= 0.f) bsq = b * b;
     }
-    best_sq = INFINITY;
+    best_sq = bsq;
     best_tri = 0xffffffffu;
     sp = 0;
-    gsp = 0;
-    // a finite caller bound alone seeds the radius when asked to (no probe
-    // descent); else the previous result seeds it for a nearby query in the
-    // sorted order; otherwise a greedy probe does
-    reused = false;
-    if ((seeding & kSeedBoundOnly) && bsq < INFINITY) {
-      best_sq = bsq;
-      prune = bsq;
-      phase = kTrav;
-      ref = root;
-      have = true;
-    } else if ((seeding & kSeedReuse) && prev != 0xffffffffu && (!kBatch || root == prev_root) &&
-               k - kprev <= 64 && k > kprev) {
+    ref = root;
+    have = true;
+    phase = kTrav;
+    // the previous result seeds the radius of a nearby query in the sorted
+    // order (a greedy descent when that is not wanted), unless a finite
+    // caller bound alone is asked to; a query without a near previous one
+    // starts without a radius, which costs less than a descent for one
+    const bool alone = (seeding & kSeedBoundOnly) && bsq < INFINITY;
+    greedy = !alone && !(seeding & kSeedReuse);
+    reused = !alone && (seeding & kSeedReuse) && prev != 0xffffffffu && (!kBatch || root == prev_root) &&
+             knew - k <= kReuseSpan;
+    if (reused) {
       phase = kSeed;
-      reused = true;
-    } else {
-      prev = 0xffffffffu;
-      phase = kProbe;
-      ref = root;
-      have = true;
+      have = false;
     }
-    S.p[lane] = make_float4(px, py, pz, prune);
-    kprev = k;
+    k = knew;
     if (kBatch) prev_root = root;
   };
 
-  // hands new queries to the lanes in `want` (warp-uniform bookkeeping)
+  // hands new queries to the groups in `want` (bits of their first lanes;
+  // warp-uniform bookkeeping)
   auto distribute = [&](unsigned want) {
     while (want) {
       if (pos >= end) {
@@ -623,223 +623,285 @@ __global__ void __maxnreg__(kTaskMaxRegs)
         uint32_t p = 0;
         if (lane == 0) p = atomicAdd(pool_counter, 1u);
         p = __shfl_sync(FULL, p, 0);
-        const int psize = kBatch ? pool : kTaskPool;
-        pos = (int64_t)p * psize;
-        end = pos + psize < n ? pos + psize : n;
-        if (pos >= n) { exhausted = true; break; }
+        const uint64_t first = (uint64_t)p * pool;
+        if (first >= n) { exhausted = true; break; }
+        pos = (uint32_t)first;
+        end = n - pos < pool ? n : pos + pool;
       }
-      const int64_t avail = end - pos;
-      const int cnt = __popc(want);
-      const int take = (int)(avail < cnt ? avail : cnt);
-      const int rank = __popc(want & lt_mask);
-      const bool mine = ((want >> lane) & 1u) && rank < take;
+      const uint32_t avail = end - pos, cnt = __popc(want);
+      const uint32_t take = avail < cnt ? avail : cnt;
+      const uint32_t rank = __popc(want & ((1u << base) - 1u));
+      const bool mine = ((want >> base) & 1u) && rank < take;
       if (mine) start(pos + rank);
       pos += take;
       want &= ~__ballot_sync(FULL, mine);
     }
   };
-  distribute(FULL);
+
+  // pops an item for every group without one: its lanes look at the top kG
+  // entries at once
+  auto pop = [&]() {
+    bool need = phase == kTrav && !have && sp > 0;
+    while (__any_sync(FULL, need)) {
+      uint2 t = make_uint2(0u, 0x7f800000u);
+      const int i = sp - 1 - c;
+      if (need && i >= 0) t = i < kGroupDepth ? stack[i] : *spill_at(i);
+      const bool good = need && i >= 0 && __uint_as_float(t.y) < best_sq;
+      const unsigned gm = (__ballot_sync(FULL, good) >> base) & gmask;
+      const int f = __ffs(gm) - 1;
+      const uint32_t pr = __shfl_sync(FULL, t.x, base + (f & (kG - 1)));
+      if (need) {
+        if (gm) {
+          ref = pr;
+          have = true;
+          sp -= f + 1;
+        } else {
+          sp = sp > kG ? sp - kG : 0;
+        }
+      }
+      need = phase == kTrav && !have && sp > 0;
+    }
+  };
+
+  distribute(groups >= 32 / kG ? lead : lead & ((1u << (kG * groups)) - 1u));
 
   while (__any_sync(FULL, phase != kIdle)) {
-    ++rounds;
-    // (a) traversing owners without an item pop; finished owners emit and refetch
-    bool done = false;
-    if (phase == kTrav && !have) {
-      for (;;) {
-        while (sp > 0) {
-          --sp;
-          const uint2 e = S.stack[sp][lane];
-          if (__uint_as_float(e.y) < best_sq) { ref = e.x; have = true; break; }
-        }
-        if (have || gsp == 0) break;
-        // shared stack empty: bring back the most recently spilled chunk
-        const int k = gsp < kSpillChunk ? gsp : kSpillChunk;
-        gsp -= k;
-        for (int i = 0; i < k; ++i) S.stack[i][lane] = my_spill[gsp + i];
-        sp = k;
+    if (kStats) ++rounds;
+    // (a) node steps
+    for (;;) {
+      const bool at = phase == kTrav && have && !ref_is_leaf(ref);
+      float d[kC], e[kC];
+      uint32_t r[kC], ties[kC];
+#pragma unroll
+      for (int j = 0; j < kC; ++j) {
+        d[j] = e[j] = INFINITY;
+        r[j] = 0u;
+        ties[j] = 0u;
       }
-      done = !have;
-    }
-    if (done && best_tri == 0xffffffffu && bsq < INFINITY) {
-      // the caller's bound excluded every triangle: run the query again in
-      // place, unbounded, seeded as the plain method seeds it (the previous
-      // query's triangle when that seeded it, else a greedy probe), instead
-      // of handing it to the deep-stack re-run kernel
-      bsq = INFINITY;
-      best_sq = INFINITY;
-      S.p[lane].w = 0.f;
-      sp = 0;
-      gsp = 0;
-      if (reused) {
-        phase = kSeed;
-        have = false;
+      if (at) {
+        if (kStats && c == 0) ++ctr.nodes;
+        node_child<kRecords, kC>(T, ref, c * kC, px, py, pz, best_sq, d, r, e, ties);
+      }
+      // a child is dropped by e (box and disc), visited in order of d (the box
+      // alone), so the discs change which children are visited, never their
+      // order; rank: the child's place in (distance, ref) order among the
+      // qualifying ones, by the distances' bits, which are never negative
+      bool ok[kC];
+      int key[kC], rank[kC], q = 0;
+      uint32_t next = 0u;
+#pragma unroll
+      for (int j = 0; j < kC; ++j) {
+        ok[j] = e[j] < best_sq || (greedy && d[j] < INFINITY);
+        key[j] = ok[j] ? __float_as_int(d[j]) : 0x7f800000;
+        q += __popc((__ballot_sync(FULL, ok[j]) >> base) & gmask);
+      }
+      if (kG == 4) {
+        rank[0] = 0;
+#pragma unroll
+        for (int x = 1; x < 4; ++x)
+          rank[0] += __shfl_xor_sync(FULL, key[0], x) < key[0] + (int)((ties[0] >> (x - 1)) & 1u) ? 1 : 0;
       } else {
-        phase = kProbe;
-        ref = root;
-        have = true;
+        const int o0 = __shfl_xor_sync(FULL, key[0], 1), o1 = __shfl_xor_sync(FULL, key[kC - 1], 1);
+        const uint32_t t0 = ties[0], t1 = ties[kC - 1];
+        const int k0 = key[0], k1 = key[kC - 1];
+        rank[0] = (k1 < k0 + (int)(t0 & 1u)) + (o0 < k0 + (int)((t0 >> 1) & 1u)) + (o1 < k0 + (int)(t0 >> 2));
+        rank[kC - 1] = (k0 < k1 + (int)(t1 & 1u)) + (o1 < k1 + (int)((t1 >> 1) & 1u)) + (o0 < k1 + (int)(t1 >> 2));
       }
-      done = false;
-    }
-    if (phase == kAbandon) done = true;
-    const bool found = done && phase != kAbandon && best_tri != 0xffffffffu;
-    if (done && !found) {
-      rerun[atomicAdd(nrerun, 1u)] = (uint32_t)qi;
-      prev = 0xffffffffu;
-    }
-    {
-      // queue the finished queries; once 32 wait, every lane writes one out
-      const unsigned fmask = __ballot_sync(FULL, found);
-      if (found) {
-        const int at = nfin + __popc(fmask & lt_mask);
-        S.fin_q[at] = (uint32_t)qi;
-        S.fin_tri[at] = best_tri;
-        S.fin_sq[at] = best_sq;
-        prev = best_tri;
-      }
-      nfin += __popc(fmask);
-      if (nfin >= 32) {
-        __syncwarp();
-        finish_entry(nfin - 32 + lane);
-        nfin -= 32;
-        __syncwarp();
-      }
-    }
-    if (done) phase = kIdle;
-    distribute(__ballot_sync(FULL, done));
-    // (b) classify this round's item
-    const bool is_node = (phase == kProbe || phase == kTrav) && have && !ref_is_leaf(ref);
-    const bool is_leaf = (phase == kProbe || phase == kTrav) && have && ref_is_leaf(ref);
-    const bool is_seed = phase == kSeed;
-    const unsigned nmask = __ballot_sync(FULL, is_node);
-    const int nrank = __popc(nmask & lt_mask);
-    const int nnodes = __popc(nmask);
-    if (is_node) {
-      S.nref[nrank] = ref;
-      S.nown[nrank] = (uint8_t)lane;
-      if (kStats) ++ctr.nodes;
-    }
-    const int tcnt = is_leaf ? (int)leaf_count(ref) : (is_seed ? 1 : 0);
-    int toff = tcnt;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(FULL, toff, o);
-      if (lane >= o) toff += v;
-    }
-    const int ttotal = __shfl_sync(FULL, toff, 31);
-    toff -= tcnt;
-    const uint32_t f0 = is_seed ? prev : leaf_first(ref);
-    if (tcnt > 0) {
-      for (int i = 0; i < tcnt; ++i) {
-        S.tidx[toff + i] = f0 + i;
-        S.town[toff + i] = (uint8_t)(lane | (i << 5));
-      }
-      if (kStats) ctr.tris += tcnt;
-    }
-    __syncwarp();
-    // (c) dense evaluation: child boxes, then triangles
-    for (int t = lane; t < 4 * nnodes; t += 32) {
-      const int r = t >> 2, c = t & 3;
-      const int o = S.nown[r];
-      float d, e;
-      uint32_t cr;
-      const float4 q = S.p[o];
-      quad_child_box(T, S.nref[r], c, q.x, q.y, q.z, q.w, d, cr, e);
-      S.box[r * kBoxStride + c] = make_uint2(__float_as_uint(d), cr);
-      S.boxe[r * kBoxStride + c] = e;
-    }
-    for (int t = lane; t < ttotal; t += 32) {
-      const uint32_t op = S.town[t];
-      const int o = (int)(op & 31u);
-      const float4 q = S.p[o];
-      S.trid[(op >> 5) * kTriRow + o] = tri_dist_sq(T.tri(S.tidx[t]), q.x, q.y, q.z);
-    }
-    __syncwarp();
-    // (d) owners consume their results
-    if (is_node) {
-      float d[4], e[4];
-      uint32_t r[4];
+      for (int j = 0; j < kC; ++j) next |= ok[j] && rank[j] == 0 ? r[j] : 0u;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const uint2 b = S.box[kBoxStride * nrank + c];
-        d[c] = __uint_as_float(b.x);
-        r[c] = b.y;
-        e[c] = S.boxe[kBoxStride * nrank + c];
-      }
-      if (phase == kProbe) {
-        // greedy: the (distance, ref)-smallest child
-        float bd = d[0];
-        uint32_t br = r[0];
-#pragma unroll
-        for (int c = 1; c < 4; ++c)
-          if (child_less(d[c], r[c], bd, br)) { bd = d[c]; br = r[c]; }
-        ref = br;
-      } else {
-        // a child is dropped by e (both boxes), visited in order of d (the
-        // axis-aligned box alone), so the oriented boxes change which children are visited, never
-        // their order
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          if (!(e[c] < best_sq)) d[c] = INFINITY;
-        cswap(d[0], r[0], e[0], d[1], r[1], e[1]);
-        cswap(d[2], r[2], e[2], d[3], r[3], e[3]);
-        cswap(d[0], r[0], e[0], d[2], r[2], e[2]);
-        cswap(d[1], r[1], e[1], d[3], r[3], e[3]);
-        cswap(d[1], r[1], e[1], d[2], r[2], e[2]);
-        int q = 0;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) q += d[c] < best_sq ? 1 : 0;
-        if (q > 0) {
-          if (sp + (q - 1) > kTaskDepth && my_spill != nullptr && gsp + kSpillChunk <= kSpillCap) {
-            // move the oldest entries (visited last) to the global overflow stack
-            for (int i = 0; i < kSpillChunk; ++i) my_spill[gsp + i] = S.stack[i][lane];
-            for (int i = kSpillChunk; i < sp; ++i) S.stack[i - kSpillChunk][lane] = S.stack[i][lane];
-            gsp += kSpillChunk;
-            sp -= kSpillChunk;
-          }
-          if (sp + (q - 1) > kTaskDepth) {
-            // still no room: the deep-stack kernel re-runs the query
+      for (int x = 1; x < kG; x <<= 1) next |= __shfl_xor_sync(FULL, next, x);
+      if (at) {
+        if (greedy) {
+          ref = next;
+        } else if (q > 0) {
+          if (sp + q - 1 > kGroupDepth && sp + q - 1 > capacity()) {
+            // no room: the deep-stack kernel re-runs the query
             phase = kAbandon;
             have = false;
           } else {
 #pragma unroll
-            for (int c = 3; c >= 1; --c)
-              if (c < q) S.stack[sp++][lane] = make_uint2(r[c], __float_as_uint(e[c]));
-            ref = r[0];
+            for (int j = 0; j < kC; ++j) {
+              const int i = sp + q - 1 - rank[j];
+              if (ok[j] && rank[j] > 0) {
+                if (i < kGroupDepth) stack[i] = make_uint2(r[j], __float_as_uint(e[j]));
+                else *spill_at(i) = make_uint2(r[j], __float_as_uint(e[j]));
+              }
+            }
+            sp += q - 1;
+            ref = next;
           }
         } else {
           have = false;
         }
       }
-    } else if (is_leaf || is_seed) {
+      __syncwarp();
+      pop();
+      const unsigned at_node = __ballot_sync(FULL, phase == kTrav && have && !ref_is_leaf(ref));
+      if (__popc(at_node) >= kG * kNodeGroups<kG>) continue;
+      if (at_node == 0) break;
+      // few queries at nodes: go on only if none waits for a leaf step or its end
+      if (__any_sync(FULL, phase == kSeed || phase == kAbandon || (phase == kTrav && (!have || ref_is_leaf(ref)))))
+        break;
+    }
+    // (b) leaf step
+    uint32_t cnt = phase == kSeed ? 1u : (phase == kTrav && have && ref_is_leaf(ref) ? leaf_count(ref) : 0u);
+    if (__any_sync(FULL, cnt > 0u)) {
+      if (kStats && c == 0) ctr.tris += cnt;
       float dmin = INFINITY;
       uint32_t imin = 0xffffffffu;
-      for (int i = 0; i < tcnt; ++i) {
-        const float dd = S.trid[i * kTriRow + lane];
-        if (dd < dmin) { dmin = dd; imin = f0 + (uint32_t)i; }
-      }
-      if (phase == kTrav) {
-        if (dmin < best_sq) {
-          best_sq = dmin;
-          best_tri = imin;
-          S.p[lane].w = dmin;
+      if (kG == 4) {
+        // every fourth triangle a lane
+        for (uint32_t i = c; i < cnt; i += 4) {
+          const uint32_t ti = (phase == kSeed ? prev : leaf_first(ref)) + i;
+          const TriRec tr = T.tri(ti);
+          float dd;
+          if (tr.c.w < 0.f) {
+            // near-degenerate: the FP64 evaluation is a call, and what stays
+            // live across a call is spilled in the hot loops as well; so the
+            // state is put aside by hand here and dead until it is read back
+            volatile uint32_t keep[20];
+            keep[0] = k; keep[1] = (uint32_t)phase; keep[2] = ref; keep[3] = prev; keep[4] = best_tri;
+            keep[5] = root; keep[6] = prev_root; keep[7] = __float_as_uint(best_sq); keep[8] = __float_as_uint(px);
+            keep[9] = __float_as_uint(py); keep[10] = __float_as_uint(pz); keep[11] = __float_as_uint(bsq);
+            keep[12] = (uint32_t)sp; keep[13] = pos; keep[14] = end; keep[15] = i;
+            keep[16] = __float_as_uint(dmin); keep[17] = imin; keep[18] = cnt;
+            keep[19] = (have ? 1u : 0u) | (reused ? 2u : 0u) | (exhausted ? 4u : 0u) | (greedy ? 8u : 0u);
+            dd = tri_dist_sq_f64(tr.a.x, tr.a.y, tr.a.z, tr.b.x, tr.b.y, tr.b.z, tr.c.x, tr.c.y, tr.c.z, px, py, pz);
+            k = keep[0]; phase = (int)keep[1]; ref = keep[2]; prev = keep[3]; best_tri = keep[4];
+            root = keep[5]; prev_root = keep[6]; best_sq = __uint_as_float(keep[7]); px = __uint_as_float(keep[8]);
+            py = __uint_as_float(keep[9]); pz = __uint_as_float(keep[10]); bsq = __uint_as_float(keep[11]);
+            sp = (int)keep[12]; pos = keep[13]; end = keep[14]; i = keep[15];
+            dmin = __uint_as_float(keep[16]); imin = keep[17]; cnt = keep[18];
+            const uint32_t fl = keep[19];
+            have = (fl & 1u) != 0u; reused = (fl & 2u) != 0u; exhausted = (fl & 4u) != 0u; greedy = (fl & 8u) != 0u;
+          } else {
+            dd = dist_sq_bary(mk(px, py, pz), mk(tr.a.x, tr.a.y, tr.a.z), mk(tr.b.x, tr.b.y, tr.b.z),
+                              mk(tr.c.x, tr.c.y, tr.c.z), tr.c.w, tr.b.w, tr.r.w, tr.r.x, tr.r.y, tr.r.z);
+          }
+          if (dd < dmin) { dmin = dd; imin = (phase == kSeed ? prev : leaf_first(ref)) + i; }
         }
-        have = false;
       } else {
-        // probe leaf or seed triangle: radius just above its distance
-        float b = dmin < INFINITY ? nextafterf(dmin, INFINITY) : INFINITY;
-        if (bsq < b) b = bsq;
-        best_sq = b;
-        S.p[lane].w = b;
-        phase = kTrav;
-        ref = root;
-        have = true;
+        // the triangles of all waiting queries as one list of tasks, a lane each
+        uint32_t off = cnt;  // tasks up to and with this query's
+#pragma unroll
+        for (int o = kG; o < 32; o <<= 1) {
+          const uint32_t v = __shfl_up_sync(FULL, off, o);
+          if (lane >= o) off += v;
+        }
+        uint32_t total = __shfl_sync(FULL, off, 31);
+        off -= cnt;
+        const unsigned owners = __ballot_sync(FULL, cnt > 0u) & lead;
+        if (c == 0 && cnt > 0u)
+          S.own[__popc(owners & ((1u << base) - 1u))] =
+              make_uint2((phase == kSeed ? prev : leaf_first(ref)) - off, (uint32_t)lane);
+        __syncwarp();
+        int before = -1;  // owners whose first task lies before this group of 32
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+          const unsigned firsts =
+              __reduce_or_sync(FULL, cnt > 0u && (off >> 5) == (t0 >> 5) ? 1u << (off & 31u) : 0u);
+          const uint2 w = S.own[before + __popc(firsts & (0xffffffffu >> (31 - lane)))];
+          before += __popc(firsts);
+          const float qx = __shfl_sync(FULL, px, w.y), qy = __shfl_sync(FULL, py, w.y),
+                      qz = __shfl_sync(FULL, pz, w.y);
+          const uint32_t t = t0 + (uint32_t)lane;
+          if (t < total) {
+            const TriRec tr = T.tri(w.x + t);
+            if (tr.c.w < 0.f) {
+              // as above
+              volatile uint32_t keep[21];
+              keep[0] = k; keep[1] = (uint32_t)phase; keep[2] = ref; keep[3] = prev; keep[4] = best_tri;
+              keep[5] = root; keep[6] = prev_root; keep[7] = __float_as_uint(best_sq); keep[8] = __float_as_uint(px);
+              keep[9] = __float_as_uint(py); keep[10] = __float_as_uint(pz); keep[11] = __float_as_uint(bsq);
+              keep[12] = (uint32_t)sp; keep[13] = pos; keep[14] = end; keep[15] = t0;
+              keep[16] = off; keep[17] = total; keep[18] = (uint32_t)before; keep[19] = cnt;
+              keep[20] = (have ? 1u : 0u) | (reused ? 2u : 0u) | (exhausted ? 4u : 0u) | (greedy ? 8u : 0u);
+              S.trid[t0 + lane] = tri_dist_sq_f64(tr.a.x, tr.a.y, tr.a.z, tr.b.x, tr.b.y, tr.b.z, tr.c.x, tr.c.y,
+                                                  tr.c.z, qx, qy, qz);
+              k = keep[0]; phase = (int)keep[1]; ref = keep[2]; prev = keep[3]; best_tri = keep[4];
+              root = keep[5]; prev_root = keep[6]; best_sq = __uint_as_float(keep[7]); px = __uint_as_float(keep[8]);
+              py = __uint_as_float(keep[9]); pz = __uint_as_float(keep[10]); bsq = __uint_as_float(keep[11]);
+              sp = (int)keep[12]; pos = keep[13]; end = keep[14]; t0 = keep[15];
+              off = keep[16]; total = keep[17]; before = (int)keep[18]; cnt = keep[19];
+              const uint32_t fl = keep[20];
+              have = (fl & 1u) != 0u; reused = (fl & 2u) != 0u; exhausted = (fl & 4u) != 0u; greedy = (fl & 8u) != 0u;
+            } else {
+              S.trid[t] = dist_sq_bary(mk(qx, qy, qz), mk(tr.a.x, tr.a.y, tr.a.z), mk(tr.b.x, tr.b.y, tr.b.z),
+                                       mk(tr.c.x, tr.c.y, tr.c.z), tr.c.w, tr.b.w, tr.r.w, tr.r.x, tr.r.y, tr.r.z);
+            }
+          }
+        }
+        __syncwarp();
+        const uint32_t f0 = phase == kSeed ? prev : leaf_first(ref);
+        for (uint32_t i = c; i < cnt; i += kG) {
+          const float dd = S.trid[off + i];
+          if (dd < dmin) { dmin = dd; imin = f0 + i; }
+        }
       }
+      // the first of the smallest, as one lane testing them in order finds it
+#pragma unroll
+      for (int x = 1; x < kG; x <<= 1) {
+        const float od = __shfl_xor_sync(FULL, dmin, x);
+        const uint32_t oi = __shfl_xor_sync(FULL, imin, x);
+        if (child_less(od, oi, dmin, imin)) { dmin = od; imin = oi; }
+      }
+      if (cnt > 0u) {
+        if (phase == kTrav && !greedy) {
+          if (dmin < best_sq) {
+            best_sq = dmin;
+            best_tri = imin;
+          }
+          have = false;
+        } else {
+          // radius just above the seed triangle's distance
+          float b = dmin < INFINITY ? nextafterf(dmin, INFINITY) : INFINITY;
+          if (bsq < b) b = bsq;
+          best_sq = b;
+          reused = true;
+          greedy = false;
+          phase = kTrav;
+          ref = root;
+          have = true;
+        }
+      }
+      __syncwarp();
     }
-    __syncwarp();
+    pop();
+    // (c) finished queries emit, their groups take new ones
+    bool done = phase == kTrav && !have;
+    if (done && best_tri == 0xffffffffu && (bsq < INFINITY || reused)) {
+      // the caller's bound excluded every triangle, or the seed triangle's own
+      // box rounds to beyond it (flat axis-aligned faces): run the query again
+      // in place, without the bound, then without the seed
+      const bool again = reused && bsq < INFINITY && prev != 0xffffffffu && (seeding & kSeedReuse);
+      bsq = INFINITY;
+      best_sq = INFINITY;
+      reused = again;
+      sp = 0;
+      ref = root;
+      have = !again;
+      phase = again ? kSeed : kTrav;
+      done = false;
+    }
+    if (phase == kAbandon) done = true;
+    const unsigned dmask = __ballot_sync(FULL, done);
+    if (dmask) {
+      if (done) {
+        if (phase != kAbandon && best_tri != 0xffffffffu) {
+          if (c == 0) {
+            out.tri[k] = best_tri;
+            out.sq[k] = best_sq;
+          }
+          prev = best_tri;
+        } else {
+          if (c == 0) rerun[atomicAdd(nrerun, 1u)] = k;
+          prev = 0xffffffffu;
+        }
+        phase = kIdle;
+      }
+      distribute(dmask & lead);
+    }
   }
-  // queries still waiting to be written out
-  __syncwarp();
-  if (lane < nfin) finish_entry(lane);
   if (kStats) {
     flush_counters(ctr, stats);
     if (lane == 0) atomicAdd(stats + 3, rounds);
@@ -847,17 +909,19 @@ __global__ void __maxnreg__(kTaskMaxRegs)
 }
 
 
-template <bool kSign, bool kStats, bool kBatch>
+template <bool kStats, bool kBatch>
 __global__ void __launch_bounds__(64)
-    udf_rerun_kernel(TreeT<kBatch> T, const float* __restrict__ pts, const uint32_t* __restrict__ rerun,
-                     const uint32_t* __restrict__ nrerun, QueryOut out, SignArgs sg, unsigned long long* stats,
-                     uint32_t* __restrict__ overflow, uint32_t* __restrict__ total_reruns, MeshSel sel) {
+    udf_rerun_kernel(TreeT<kBatch> T, const float* __restrict__ pts, const uint32_t* __restrict__ perm,
+                     const uint32_t* __restrict__ rerun, const uint32_t* __restrict__ nrerun, Best out,
+                     unsigned long long* stats, uint32_t* __restrict__ overflow, uint32_t* __restrict__ total_reruns,
+                     MeshSel sel) {
   pdl_wait();
   const uint32_t m = *nrerun;
   if (blockIdx.x == 0 && threadIdx.x == 0 && m > 0) atomicAdd(total_reruns, m);
   Counters ctr{0, 0};
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t qi = rerun[t];
+    const uint32_t k = rerun[t];
+    const int64_t qi = perm ? perm[k] : k;
     const float px = pts[3 * qi], py = pts[3 * qi + 1], pz = pts[3 * qi + 2];
     uint32_t seed_tri;
     float seed_sq;
@@ -867,13 +931,38 @@ __global__ void __launch_bounds__(64)
     uint32_t best_tri = 0xffffffffu;
     LocalStack st;
     st.sp = 0;
-    if (!traverse(T, px, py, pz, st, best_sq, best_tri, ctr, root)) atomicExch(overflow, 1u);
-    finish_query(T.tris, T.num_tris, best_tri, best_sq, px, py, pz, qi, out, sg, kSign);
+    bool ok = traverse(T, px, py, pz, st, best_sq, best_tri, ctr, root);
+    if (ok && best_tri == 0xffffffffu) {
+      // the probed triangle's own box rounds to beyond it: no radius
+      best_sq = INFINITY;
+      st.sp = 0;
+      ok = traverse(T, px, py, pz, st, best_sq, best_tri, ctr, root);
+    }
+    if (!ok) atomicExch(overflow, 1u);
+    out.tri[k] = best_tri;
+    out.sq[k] = best_sq;
   }
   if (kStats && (ctr.nodes | ctr.tris)) {
     atomicAdd(stats, ctr.nodes);
     atomicAdd(stats + 1, ctr.tris);
   }
+}
+
+// The caller's outputs from the traversal's results, one thread per query in
+// sorted order (neighbouring threads read the same triangle records; outputs
+// scatter to the queries' own places).  A kernel of its own because the
+// closest point, barycentrics and sign would cost the traversal its registers
+// (in it: 192 B of spills a lane, which with 24 warps an SM overflow L1).
+template <bool kSign>
+__global__ void __launch_bounds__(256)
+    udf_finish_kernel(const TriRec* __restrict__ tris, uint32_t num_tris, const float* __restrict__ pts, int64_t n,
+                      const uint32_t* __restrict__ perm, Best best, QueryOut out, SignArgs sg) {
+  pdl_wait();
+  const int64_t k = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (k >= n) return;
+  const int64_t qi = perm ? perm[k] : k;
+  finish_query(tris, num_tris, best.tri[k], best.sq[k], pts[3 * qi], pts[3 * qi + 1], pts[3 * qi + 2], qi, out, sg,
+               kSign);
 }
 
 __global__ void query_morton_kernel(const float* __restrict__ pts, int64_t n, float lox, float loy, float loz,
@@ -905,6 +994,7 @@ struct UdfWs {
   uint32_t* rerun;
   uint32_t* nrerun;  // status words: [0] re-run list length, [1] deep-stack overflow, [2] pool counter,
                      // [3] guard faults, [4] queries re-run in total
+  Best best;         // the traversal's results; with a query sort in its key buffers, free after it
   uint2* spill;      // optional overflow stacks (trailing workspace)
   int64_t spill_owners;
 };
@@ -918,18 +1008,21 @@ size_t carve_udf(UdfWs& w, Workspace& ws, int64_t n, uint32_t flags) {
     w.vals = ws.take<uint32_t>(n);
     w.vals_alt = ws.take<uint32_t>(n);
     w.rs_scratch = ws.take<uint32_t>((int64_t)radix_sort_scratch_elems(n));
+    w.best = Best{w.keys, reinterpret_cast<float*>(w.keys_alt)};
   } else {
     w.keys = w.keys_alt = w.vals = w.vals_alt = w.rs_scratch = nullptr;
+    w.best.tri = ws.take<uint32_t>(n);
+    w.best.sq = ws.take<float>(n);
   }
   w.rerun = ws.take<uint32_t>(n);
   return ws.used;
 }
 
-// owners of the persistent traversal that get an overflow stack when the
-// workspace has room for it (bounded: 148 SMs x 10 blocks x 64 lanes)
+// queries in flight (four lanes each) that get an overflow stack when the
+// workspace has room for it (bounded: 148 SMs x 64 warps)
 int64_t spill_owner_bound(int64_t n) {
-  const int64_t cap = (int64_t)148 * 10 * 64;  // overflow stacks for the resident owners of a 148-SM part
-  return n + 128 < cap ? n + 128 : cap;
+  const int64_t cap = (int64_t)148 * 32 * 16;
+  return (n + kGroupWarps) * 16 < cap ? (n + kGroupWarps) * 16 : cap;  // a warp may take one query only
 }
 
 // launch shape of the persistent traversal: queries per pool, resident
@@ -939,8 +1032,8 @@ struct TaskShape {
   int blocks_per_sm;
 };
 
-template <bool kSign, bool kStats, bool kBatch>
-int task_blocks_per_sm(int* out) {
+template <int kG, bool kRecords, bool kStats, bool kBatch>
+int group_blocks_per_sm(int* out) {
   // per device: a process may drive GPUs of different kinds
   static int cached[kMaxDevices] = {0};
   int dev = 0;
@@ -950,44 +1043,73 @@ int task_blocks_per_sm(int* out) {
     return A3D_OK;
   }
   int b = 0;
-  A3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, udf_task_kernel<kSign, kStats, kBatch>,
-                                                             kTaskWarps * 32, 0));
+  A3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, udf_group_kernel<kG, kRecords, kStats, kBatch>,
+                                                             kGroupWarps * 32, 0));
   b = b < 1 ? 1 : b;
   if (dev >= 0 && dev < kMaxDevices) cached[dev] = b;
   *out = b;
   return A3D_OK;
 }
 
+template <int kG, bool kRecords, bool kStats, bool kBatch>
+int launch_groups(const TreeT<kBatch>& T, const float* pts, int64_t n, const uint32_t* perm, const float* bound,
+                  unsigned long long* stats, UdfWs& w, uint32_t seeding, const MeshSel& sel, TaskShape shape,
+                  cudaStream_t s) {
+  int bps = 0;
+  A3D_TRY((group_blocks_per_sm<kG, kRecords, kStats, kBatch>(&bps)));
+  if (shape.blocks_per_sm > 0 && shape.blocks_per_sm < bps) bps = shape.blocks_per_sm;
+  const int64_t warps = (int64_t)num_sms() * bps * kGroupWarps;
+  // few queries: as few a warp as the resident warps allow
+  const int64_t per_warp = ceil_div(n, warps);
+  const int groups = per_warp < 32 / kG ? (int)per_warp : 32 / kG;
+  int64_t pool = shape.pool;
+  if (pool <= 0) {
+    pool = per_warp / 4;
+    pool = pool < groups ? groups : (pool > kMaxPool ? kMaxPool : pool);
+  }
+  const int64_t want_blocks = ceil_div(ceil_div(n, pool), kGroupWarps);
+  const int64_t grid = want_blocks < warps / kGroupWarps ? want_blocks : warps / kGroupWarps;
+  const int64_t owners = w.spill == nullptr ? 0 : (w.spill_owners < 0x7fffffff ? w.spill_owners : 0x7fffffff);
+  A3D_PDL((udf_group_kernel<kG, kRecords, kStats, kBatch>), dim3((unsigned)grid), dim3(kGroupWarps * 32), 0, s, T, pts,
+          (uint32_t)n, perm, bound, w.best, stats, w.rerun, w.nrerun, w.nrerun + 2, w.spill, (uint32_t)owners, seeding,
+          sel, (uint32_t)pool, groups);
+  return A3D_OK;
+}
+
+// From this many queries on two lanes a query, below it four: four take fewer
+// steps a query, which counts while the queries in flight do not fill the
+// chip, two execute less per query (16.8M queries: 34.1 against 36.6 ms; 24
+// meshes with 8.7M: 23.8 against 25.0 with their build; 300k: 0.86 against
+// 0.83; 100k: 0.44 against 0.38).
+constexpr int64_t kPairMin = 2 << 20;
+
 template <bool kSign, bool kStats, bool kBatch>
 int launch_udf(const TreeT<kBatch>& T, const float* pts, int64_t n, const uint32_t* perm, bool coherent,
                const float* bound, const QueryOut& out, const SignArgs& sg, unsigned long long* stats, UdfWs& w,
                uint32_t seeding, const MeshSel& sel, TaskShape shape, cudaStream_t s) {
   if (coherent) {
-    int bps = 0;
-    A3D_TRY((task_blocks_per_sm<kSign, kStats, kBatch>(&bps)));
-    if (shape.blocks_per_sm > 0 && shape.blocks_per_sm < bps) bps = shape.blocks_per_sm;
-    const int pool = shape.pool > 0 ? shape.pool : kTaskPool;
-    const int sms = num_sms();
-    const int64_t pools = ceil_div(n, pool);
-    const int64_t want_blocks = ceil_div(pools, kTaskWarps);
-    const int64_t grid = want_blocks < (int64_t)sms * bps ? want_blocks : (int64_t)sms * bps;
-    A3D_PDL((udf_task_kernel<kSign, kStats, kBatch>), dim3((unsigned)grid), dim3(kTaskWarps * 32), 0, s, T, pts, n,
-            perm, bound, out, sg, stats, w.rerun, w.nrerun, w.nrerun + 2, w.spill, w.spill_owners, seeding, sel, pool);
+    if (T.num_children > 0u) {
+      A3D_TRY(n >= kPairMin
+                  ? (launch_groups<2, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
+                  : (launch_groups<4, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s)));
+    } else {
+      A3D_TRY((launch_groups<4, false, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s)));
+    }
   } else {
     if constexpr (!kBatch) {
-      A3D_PDL((udf_kernel<kSign, kStats>), dim3((unsigned)ceil_div(n, kUdfThreads)), dim3(kUdfThreads), 0, s, T, pts, n,
-              1, perm, bound, out, sg, stats, w.rerun, w.nrerun);
+      A3D_PDL((udf_kernel<kStats>), dim3((unsigned)ceil_div(n, kUdfThreads)), dim3(kUdfThreads), 0, s, T, pts, n, 1,
+              perm, bound, w.best, stats, w.rerun, w.nrerun);
     } else {
       A3D_REQUIRE(false, A3D_ERR_ARGUMENT, "udf: batches are always sorted");
     }
   }
   A3D_LAUNCH_CHECK();
-  // the re-run list length is only known on the device: launch enough
-  // threads for a few percent of the queries, each thread strides
-  const int64_t rr_min = (int64_t)num_sms() * 256;
-  const int64_t rr_threads = n / 16 > rr_min ? n / 16 : rr_min;
-  A3D_PDL((udf_rerun_kernel<kSign, kStats, kBatch>), dim3((unsigned)ceil_div(rr_threads, 64)), dim3(64), 0, s, T, pts,
-          w.rerun, w.nrerun, out, sg, stats, w.nrerun + 1, w.nrerun + 4, sel);
+  // the re-run list length is only known on the device (and nearly always 0)
+  const int64_t rr_threads = (int64_t)num_sms() * 256;
+  A3D_PDL((udf_rerun_kernel<kStats, kBatch>), dim3((unsigned)ceil_div(rr_threads, 64)), dim3(64), 0, s, T, pts, perm,
+          w.rerun, w.nrerun, w.best, stats, w.nrerun + 1, w.nrerun + 4, sel);
+  A3D_PDL(udf_finish_kernel<kSign>, dim3((unsigned)ceil_div(n, 256)), dim3(256), 0, s, T.tris, T.num_tris, pts, n, perm,
+          w.best, out, sg);
   return A3D_OK;
 }
 
@@ -1057,11 +1179,11 @@ extern "C" int a3d_udf(const a3d_bvh_view* bvh, const float* points, int64_t num
                        int32_t* face_ids, float* closest_points, float* uvw, const a3d_sign_data* sign,
                        const float* bound, unsigned long long* stats, uint32_t flags, void* workspace,
                        size_t workspace_bytes, a3d_stream_t stream) {
-  return a3d_udf_obbs(bvh, nullptr, points, num_points, distances, face_ids, closest_points, uvw, sign, bound, stats,
-                       flags, workspace, workspace_bytes, stream);
+  return a3d_udf_children(bvh, nullptr, points, num_points, distances, face_ids, closest_points, uvw, sign, bound,
+                          stats, flags, workspace, workspace_bytes, stream);
 }
 
-extern "C" int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const float* points, int64_t num_points,
+extern "C" int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, const float* points, int64_t num_points,
                              float* distances, int32_t* face_ids, float* closest_points, float* uvw,
                              const a3d_sign_data* sign, const float* bound, unsigned long long* stats, uint32_t flags,
                              void* workspace, size_t workspace_bytes, a3d_stream_t stream_) {
@@ -1109,10 +1231,10 @@ extern "C" int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const flo
                            ((flags & A3D_UDF_BOUND_SEEDS) && bound ? kSeedBoundOnly : 0u);
   A3D_CUDA_TRY(cudaMemsetAsync(w.nrerun, 0, kStatusWords * sizeof(uint32_t), s));
   const TreeT<false> T{(const WideNode*)bvh->nodes, (const TriRec*)bvh->tris, (uint32_t)bvh->num_nodes,
-                       (uint32_t)bvh->num_tris, w.nrerun + 3, (const ObbNode*)obbs,
-                       obbs != nullptr ? (uint32_t)bvh->num_nodes : 0u};
+                       (uint32_t)bvh->num_tris, w.nrerun + 3, ChildRecs(children, bvh->num_nodes),
+                       children != nullptr ? (uint32_t)bvh->num_nodes : 0u};
   const MeshSel sel{nullptr, nullptr, 1, 0};
-  const TaskShape shape{kTaskPool, 0};
+  const TaskShape shape{0, 0};
   QueryOut out{distances, face_ids, closest_points, uvw};
   SignArgs sg{nullptr, nullptr, nullptr, nullptr, nullptr};
   if (sign) {
@@ -1121,11 +1243,19 @@ extern "C" int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const flo
                   pn ? sign->he_edge_idx : nullptr, sign->faces};
   }
   if (sign) {
-    if (stats) A3D_TRY((launch_udf<true, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel, shape, s)));
-    else A3D_TRY((launch_udf<true, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel, shape, s)));
+    if (stats)
+      A3D_TRY((launch_udf<true, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+                                             shape, s)));
+    else
+      A3D_TRY((launch_udf<true, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+                                              shape, s)));
   } else {
-    if (stats) A3D_TRY((launch_udf<false, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel, shape, s)));
-    else A3D_TRY((launch_udf<false, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel, shape, s)));
+    if (stats)
+      A3D_TRY((launch_udf<false, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+                                              shape, s)));
+    else
+      A3D_TRY((launch_udf<false, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+                                               shape, s)));
   }
   if (stats) {
     // reruns are reported as bound misses / spills (same counter: re-run queries)
@@ -1212,8 +1342,9 @@ size_t batch_udf_bytes(int64_t n) {
   return base + (size_t)spill_owner_bound(c) * kSpillCap * sizeof(uint2) + 512;
 }
 
-int batch_udf(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points, const int64_t* qoff, int64_t n, float* distances,
-              int32_t* face_ids, float* closest_points, float* uvw, TaskShape shape, unsigned long long* stats,
+int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_children, const float* points,
+              const int64_t* qoff, int64_t n, float* distances, int32_t* face_ids, float* closest_points,
+              float* uvw, TaskShape shape, unsigned long long* stats,
               void* workspace, size_t workspace_bytes, cudaStream_t s) {
   A3D_REQUIRE(bvh && bvh->nodes && bvh->tris && bvh->roots && bvh->bounds && bvh->num_meshes > 0 &&
                   bvh->num_faces > 0 && bvh->num_faces < (1ll << 28),
@@ -1241,8 +1372,8 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, cons
   A3D_REQUIRE(points && qoff && distances && face_ids && closest_points, A3D_ERR_ARGUMENT, "batch_udf: null pointer");
   // the node count is only known on the device: guard with the capacity
   const TreeT<true> T{(const WideNode*)bvh->nodes, (const TriRec*)bvh->tris, (uint32_t)bvh->num_faces,
-                      (uint32_t)bvh->num_faces, w.nrerun + 3, (const ObbNode*)obbs,
-                      obbs != nullptr ? (uint32_t)num_obbs : 0u};
+                      (uint32_t)bvh->num_faces, w.nrerun + 3, ChildRecs(children, num_children),
+                      children != nullptr ? (uint32_t)num_children : 0u};
   const SignArgs sg{nullptr, nullptr, nullptr, nullptr, nullptr};
   for (int64_t base = 0; base < n; base += kBatchChunk) {
     const int64_t cn = n - base < kBatchChunk ? n - base : kBatchChunk;
@@ -1328,25 +1459,25 @@ extern "C" int a3d_batch_udf(const a3d_bvh_batch* bvh, const float* points, cons
                              int64_t num_queries, float* distances, int32_t* face_ids, float* closest_points,
                              float* uvw, const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
                              size_t workspace_bytes, a3d_stream_t stream) {
-  return a3d_batch_udf_obbs(bvh, nullptr, 0, points, query_offsets, num_queries, distances, face_ids, closest_points,
-                             uvw, tuning, stats, workspace, workspace_bytes, stream);
+  return a3d_batch_udf_children(bvh, nullptr, 0, points, query_offsets, num_queries, distances, face_ids,
+                                closest_points, uvw, tuning, stats, workspace, workspace_bytes, stream);
 }
 
-extern "C" int a3d_batch_udf_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points,
-                                   const int64_t* query_offsets, int64_t num_queries, float* distances,
-                                   int32_t* face_ids, float* closest_points, float* uvw,
-                                   const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
-                                   size_t workspace_bytes, a3d_stream_t stream) {
-  A3D_REQUIRE(num_obbs >= 0 && num_obbs < (1ll << 31), A3D_ERR_ARGUMENT, "batch_udf: bad oriented-box count");
-  a3d::TaskShape shape{a3d::kTaskPool, 0};
+extern "C" int a3d_batch_udf_children(const a3d_bvh_batch* bvh, const void* children, int64_t num_children,
+                                      const float* points, const int64_t* query_offsets, int64_t num_queries,
+                                      float* distances, int32_t* face_ids, float* closest_points, float* uvw,
+                                      const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
+                                      size_t workspace_bytes, a3d_stream_t stream) {
+  A3D_REQUIRE(num_children >= 0 && num_children < (1ll << 31), A3D_ERR_ARGUMENT, "batch_udf: bad child-record count");
+  a3d::TaskShape shape{0, 0};
   if (tuning) {
     A3D_REQUIRE(tuning->pool >= 0 && tuning->pool <= 4096 && tuning->blocks_per_sm >= 0, A3D_ERR_ARGUMENT,
                 "batch_udf: bad tuning");
     if (tuning->pool > 0) shape.pool = tuning->pool;
     shape.blocks_per_sm = tuning->blocks_per_sm;
   }
-  return a3d::batch_udf(bvh, obbs, num_obbs, points, query_offsets, num_queries, distances, face_ids, closest_points, uvw, shape,
-                        stats, workspace, workspace_bytes, (cudaStream_t)stream);
+  return a3d::batch_udf(bvh, children, num_children, points, query_offsets, num_queries, distances, face_ids,
+                        closest_points, uvw, shape, stats, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" size_t a3d_batch_autotune_workspace_bytes(int64_t sample_queries, int32_t num_meshes) {
@@ -1359,11 +1490,11 @@ extern "C" int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points,
                                   int64_t num_queries, int64_t sample_queries, void* workspace,
                                   size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,
                                   a3d_stream_t stream) {
-  return a3d_batch_autotune_obbs(bvh, nullptr, 0, points, query_offsets, num_queries, sample_queries, workspace,
+  return a3d_batch_autotune_children(bvh, nullptr, 0, points, query_offsets, num_queries, sample_queries, workspace,
                                   workspace_bytes, best, best_ms, stream);
 }
 
-extern "C" int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs,
+extern "C" int a3d_batch_autotune_children(const a3d_bvh_batch* bvh, const void* children, int64_t num_children,
                                         const float* points, const int64_t* query_offsets, int64_t num_queries,
                                         int64_t sample_queries, void* workspace, size_t workspace_bytes,
                                         a3d_udf_tuning* best, float* best_ms, a3d_stream_t stream_) {
@@ -1386,14 +1517,14 @@ extern "C" int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obb
   A3D_PDL(sample_queries_kernel, dim3((unsigned)ceil_div(th, 256)), dim3(256), 0, s, points, stride, query_offsets,
           bvh->num_meshes, t.pts, ns, t.qoff);
   int occ = 0;
-  A3D_TRY((task_blocks_per_sm<false, false, true>(&occ)));
+  A3D_TRY((group_blocks_per_sm<2, true, false, true>(&occ)));
   const int pools[4] = {32, 64, 128, 256};
   const int bpss[3] = {occ, occ * 3 / 4, occ / 2};
   cudaEvent_t e0, e1;
   A3D_CUDA_TRY(cudaEventCreate(&e0));
   A3D_CUDA_TRY(cudaEventCreate(&e1));
   float best_t = INFINITY;
-  a3d_udf_tuning bt{kTaskPool, occ, 0, 0};
+  a3d_udf_tuning bt{64, occ, 0, 0};
   int rc = A3D_OK;
   for (int pi = 0; pi < 4 && rc == A3D_OK; ++pi) {
     for (int bi = 0; bi < 3 && rc == A3D_OK; ++bi) {
@@ -1404,8 +1535,8 @@ extern "C" int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obb
       for (int rep = 0; rep < 3 && rc == A3D_OK; ++rep) {
         if (rep == 1 && cudaEventRecord(e0, s) != cudaSuccess) rc = A3D_ERR_CUDA;
         if (rc == A3D_OK)
-          rc = batch_udf(bvh, obbs, num_obbs, t.pts, t.qoff, ns, t.dist, t.fid, t.cp, nullptr, shape, nullptr, t.udf_ws, t.udf_bytes,
-                         s);
+          rc = batch_udf(bvh, children, num_children, t.pts, t.qoff, ns, t.dist, t.fid, t.cp, nullptr, shape, nullptr,
+                         t.udf_ws, t.udf_bytes, s);
       }
       float ms = 0.f;
       if (rc == A3D_OK && (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||

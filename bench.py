@@ -351,9 +351,9 @@ def main():
     stream = torch.cuda.current_stream(dev)
 
     def step(stats=None):
-        _lib.call("a3d_udf_obbs", ctypes.byref(view), bvh.obbs.data_ptr(), qd.data_ptr(), n,
-                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, _lib.ptr(stats), flags, ws.data_ptr(), ws.numel(),
-                  stream.cuda_stream)
+        _lib.call("a3d_udf_children", ctypes.byref(view), bvh.children.data_ptr(), qd.data_ptr(), n,
+                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, _lib.ptr(stats), flags,
+                  ws.data_ptr(), ws.numel(), stream.cuda_stream)
 
     # traversal statistics of our tree (one untimed pass)
     st = torch.zeros(4, dtype=torch.int64, device=dev)
@@ -934,9 +934,9 @@ def l2_read_peak(dev, mib=48, passes=40, reps=5):
 
 
 def launches_per_udf():
-    # query Morton keys (1) + 4 radix passes x (upsweep, 3 scan kernels,
-    # downsweep) + traversal + re-run kernel
-    return 1 + 4 * 5 + 2
+    # query Morton keys (1) + 4 radix passes x (upsweep, 2 scan kernels,
+    # downsweep) + traversal + re-run kernel + outputs
+    return 1 + 4 * 4 + 3
 
 
 def time_traversal_kernel(bvh, qd, dist_o, fid_o, cp_o, ws, flags, stream, steps):
@@ -964,9 +964,9 @@ def time_traversal_kernel(bvh, qd, dist_o, fid_o, cp_o, ws, flags, stream, steps
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
 
     def call():
-        _lib.call("a3d_udf_obbs", ctypes.byref(view), bvh.obbs.data_ptr(), qs.data_ptr(), n,
-                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, None, _lib.A3D_UDF_ASSUME_SORTED | (flags & ~_lib.A3D_UDF_SORT_QUERIES),
-                  ws.data_ptr(), ws.numel(),
+        _lib.call("a3d_udf_children", ctypes.byref(view), bvh.children.data_ptr(), qs.data_ptr(), n,
+                  dist_o.data_ptr(), fid_o.data_ptr(), cp_o.data_ptr(), None, None, None, None,
+                  _lib.A3D_UDF_ASSUME_SORTED | (flags & ~_lib.A3D_UDF_SORT_QUERIES), ws.data_ptr(), ws.numel(),
                   stream.cuda_stream)
 
     for _ in range(3):

@@ -68,17 +68,17 @@ int a3d_bvh_build(const float* vertices, int64_t num_vertices,
                   float* bounds_out /* host, 6 floats: lo xyz, hi xyz */,
                   a3d_stream_t stream);
 
-/* Oriented boxes of a finished tree (no counterpart in the reference): per
- * child of every node the extent of its triangles in a frame along their mean
- * normal, a lower bound on the distance that is far tighter than the
- * axis-aligned box on smooth surfaces.  obbs_out: num_nodes x
- * A3D_BVH_OBB_BYTES, 16-B aligned.  For a batch, num_nodes is the node
- * capacity of obbs_out and num_nodes_device (nullable) a3d_batch_build's
- * device count.  a3d_udf_obbs and a3d_batch_udf_obbs take them; results never
- * depend on them. */
-#define A3D_BVH_OBB_BYTES 128
-int a3d_bvh_obbs(const void* nodes, const void* tris, int64_t num_nodes,
-                  const int64_t* num_nodes_device, int64_t num_tris, void* obbs_out,
+/* Child records of a finished tree (no counterpart in the reference): per
+ * child of every node its box and reference decoded and a disc about its
+ * triangles along their mean normal, a lower bound on the distance that is far
+ * tighter than the axis-aligned box on smooth surfaces.  children_out:
+ * a3d_bvh_children_bytes(num_nodes, num_tris) bytes, 32-B aligned.  For a
+ * batch, num_nodes is a capacity (nodes past it go without) and
+ * num_nodes_device (nullable) a3d_batch_build's device count.  a3d_udf_children and
+ * a3d_batch_udf_children take them; results never depend on them. */
+size_t a3d_bvh_children_bytes(int64_t num_nodes, int64_t num_tris);
+int a3d_bvh_children(const void* nodes, const void* tris, int64_t num_nodes,
+                  const int64_t* num_nodes_device, int64_t num_tris, void* children_out,
                   a3d_stream_t stream);
 
 /* ---- pseudo-normal precompute for the SDF sign -------------------------- */
@@ -123,10 +123,10 @@ typedef struct a3d_sign_data {
 #define A3D_UDF_ASSUME_SORTED 2u  /* queries already spatially coherent: skip the sort */
 /* radius seeding (results never depend on it): by default a query's pruning
  * radius starts just above the distance to the closest triangle of the
- * previous query in the sorted order, or of a greedy descent, capped by
- * `bound`.  NO_REUSE drops the previous-query seed; BOUND_SEEDS lets a
- * finite `bound` alone seed the radius (no greedy descent).  A query with
- * no triangle inside a too-small bound is re-run without it. */
+ * previous query in the sorted order when that is near, capped by `bound`.
+ * NO_REUSE takes a greedy descent's triangle instead; BOUND_SEEDS lets a
+ * finite `bound` alone seed the radius.  A query with no triangle inside a
+ * too-small bound is re-run without it. */
 #define A3D_UDF_NO_REUSE 4u
 #define A3D_UDF_BOUND_SEEDS 8u
 size_t a3d_udf_workspace_bytes(int64_t num_points, uint32_t flags);
@@ -136,9 +136,9 @@ int a3d_udf(const a3d_bvh_view* bvh, const float* points, int64_t num_points,
             unsigned long long* stats, uint32_t flags,
             void* workspace, size_t workspace_bytes, a3d_stream_t stream);
 
-/* a3d_udf with the tree's oriented boxes (a3d_bvh_obbs; NULL: none): the
+/* a3d_udf with the tree's child records (a3d_bvh_children; NULL: none): the
  * same results from fewer tests. */
-int a3d_udf_obbs(const a3d_bvh_view* bvh, const void* obbs, const float* points, int64_t num_points,
+int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, const float* points, int64_t num_points,
                   float* distances, int32_t* face_ids, float* closest_points,
                   float* uvw, const a3d_sign_data* sign, const float* bound,
                   unsigned long long* stats, uint32_t flags,
@@ -552,9 +552,9 @@ int a3d_batch_udf(const a3d_bvh_batch* bvh, const float* points, const int64_t* 
                   int64_t num_queries, float* distances, int32_t* face_ids, float* closest_points,
                   float* uvw, const a3d_udf_tuning* tuning, unsigned long long* stats,
                   void* workspace, size_t workspace_bytes, a3d_stream_t stream);
-/* the same with the batch's oriented boxes (num_obbs records; nodes past
+/* the same with the batch's child records (of num_children nodes; nodes past
  * them have none) */
-int a3d_batch_udf_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs, const float* points,
+int a3d_batch_udf_children(const a3d_bvh_batch* bvh, const void* children, int64_t num_children, const float* points,
                         const int64_t* query_offsets, int64_t num_queries, float* distances,
                         int32_t* face_ids, float* closest_points, float* uvw,
                         const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
@@ -567,7 +567,7 @@ int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points, const int6
                        int64_t num_queries, int64_t sample_queries, void* workspace,
                        size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,
                        a3d_stream_t stream);
-int a3d_batch_autotune_obbs(const a3d_bvh_batch* bvh, const void* obbs, int64_t num_obbs,
+int a3d_batch_autotune_children(const a3d_bvh_batch* bvh, const void* children, int64_t num_children,
                              const float* points, const int64_t* query_offsets,
                              int64_t num_queries, int64_t sample_queries, void* workspace,
                              size_t workspace_bytes, a3d_udf_tuning* best, float* best_ms,

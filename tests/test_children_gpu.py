@@ -1,5 +1,5 @@
-"""The oriented boxes only skip work: a3d_udf_obbs returns what a3d_udf (no
-boxes) returns, bit for bit, because a child is skipped only when none of its
+"""The child records only skip work: a3d_udf_children returns what a3d_udf
+(no records) returns, bit for bit, because a child is skipped only when none of its
 triangles' computed distances can be below the best one."""
 
 import ctypes
@@ -70,7 +70,7 @@ def mesh(kind):
 @pytest.mark.parametrize("kind", ["smooth", "one triangle", "cube", "soup", "infinite vertex", "far from the origin",
                                   "flattened"])
 @pytest.mark.parametrize("leaf_max", [1, 8])
-def test_oriented_boxes_change_no_result(kind, leaf_max):
+def test_child_records_change_no_result(kind, leaf_max):
     v, f = mesh(kind)
     b = WideBVH(v.cuda(), f.cuda(), leaf_max=leaf_max)
     g = torch.Generator().manual_seed(5)
@@ -89,3 +89,19 @@ def test_oriented_boxes_change_no_result(kind, leaf_max):
         for x, y in zip((*ref[:3], ref[3][has]), (*got[:3], got[3][has])):
             same = (x == y) | ((x != x) & (y != y))
             assert bool(same.all()), (kind, leaf_max, int((~same).sum()))
+
+
+@pytest.mark.parametrize("kind", ["one triangle", "cube"])
+def test_flat_boxes_still_give_every_query_its_face(kind):
+    """A flat box can round to just beyond its own triangle: a query whose
+    radius that triangle seeds must not come back empty."""
+    v, f = mesh(kind)
+    if kind == "one triangle":
+        v = torch.tensor([[0.0, 0, 0], [1, 0, 0], [0, 1, 0]])
+    b = WideBVH(v.cuda(), f.cuda())
+    q = torch.rand(50000, 3, generator=torch.Generator().manual_seed(2)).cuda() * 3 - 1
+    first = b.query(q)
+    assert int(first[1].min()) >= 0
+    for _ in range(3):
+        for x, y in zip(first, b.query(q)):
+            assert torch.equal(x, y)
