@@ -15,8 +15,9 @@
 //      nodes s..e-2 with root s, leaf j at N + j (duplicate codes
 //      disambiguated by index)
 //   4b. SAH refinement: every subtree of at most 16384 triangles below the
-//      top of the tree is rebuilt top-down with binned SAH by one thread
-//      block (bvh_sah.cuh), in place and within its own index range
+//      top of the tree is rebuilt top-down with binned SAH, its upper nodes by
+//      one thread block, the rest by the chip's warps (bvh_sah.cuh), in place
+//      and within its own index range
 //   5. bottom-up refit (second arriving child computes the union box)
 //   6. SAH-optimal collapse into 4-wide quantised nodes: the refit also
 //      computes, bottom-up, the cheapest cover of every subtree by 1..4 wide
@@ -81,11 +82,12 @@ struct BuildWs {
   uint32_t* newidx;     // [N] slot -> final node index
   int64_t* count;       // single-mesh builds: node count
   int32_t* clusters;    // [N] roots of the subtrees the SAH pass rebuilds
-  uint32_t* ncl;        // their count
+  uint32_t* ncl;        // their count, and the small nodes'
   float4* dp_cost;      // [N] collapse cost of each internal node spread over 1..4 wide slots
   uint32_t* dp_dec;     // [N] the decisions behind dp_cost (see refit_kernel)
   uint32_t* sah_tmp;    // [N] partition scratch of the SAH pass
-  SahNode* sah_small;   // [N] its lists of small nodes
+  SahSmall* sah_small;  // [N] its list of small nodes
+  int32_t* sah_nat;     // [N / 3 + 1] where each cluster's new root would have been
 };
 
 size_t carve(BuildWs& w, Workspace& ws, int64_t n, int64_t m) {
@@ -121,11 +123,12 @@ size_t carve(BuildWs& w, Workspace& ws, int64_t n, int64_t m) {
   w.newidx = ws.take<uint32_t>(n);
   w.count = ws.take<int64_t>(1);
   w.clusters = ws.take<int32_t>(n);
-  w.ncl = ws.take<uint32_t>(1);
+  w.ncl = ws.take<uint32_t>(2);
   w.dp_cost = ws.take<float4>(n);
   w.dp_dec = ws.take<uint32_t>(n);
   w.sah_tmp = ws.take<uint32_t>(n);
-  w.sah_small = ws.take<SahNode>(n);
+  w.sah_small = ws.take<SahSmall>(n);
+  w.sah_nat = ws.take<int32_t>(n / 3 + 1);
   return ws.used;
 }
 
@@ -688,7 +691,12 @@ int launch_sah(int64_t n, BuildWs& w, const uint32_t* order, cudaStream_t s) {
   A3D_PDL(sah_cluster_kernel<kThreads>, dim3((unsigned)(max_clusters < sah_grid ? max_clusters : sah_grid)),
           dim3(kThreads), sizeof(SahSmem<kThreads>), s, w.clusters, w.ncl,
           SahTree{w.left, w.right, w.parent, w.first, w.last, n}, const_cast<uint32_t*>(order), w.sah_tmp,
-          w.sah_small, SahPrims{w.centroid, w.tri_lo, w.tri_hi});
+          w.sah_small, w.ncl + 1, w.sah_nat, n >= kSahWideFrom ? kSahWarpWide : kSahWarpMin,
+          SahPrims{w.centroid, w.tri_lo, w.tri_hi});
+  const int64_t want = ceil_div(n / 2 + 1, kSahSmallThreads / 32), cap = (int64_t)num_sms() * 8;
+  A3D_PDL(sah_small_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(kSahSmallThreads), 0, s, w.sah_small,
+          w.ncl + 1, w.clusters, w.sah_nat, SahTree{w.left, w.right, w.parent, w.first, w.last, n},
+          const_cast<uint32_t*>(order), w.sah_tmp, SahPrims{w.centroid, w.tri_lo, w.tri_hi});
   return A3D_OK;
 }
 
@@ -725,7 +733,7 @@ int build_wide_bvh(const float* V, const int64_t* vert_off, const int32_t* F, co
   // 64 clusters for the SMs
   int sah_max = kSahMax;
   while (sah_max > 2048 && (int64_t)sah_max * 64 > n) sah_max >>= 1;
-  A3D_CUDA_TRY(cudaMemsetAsync(w.ncl, 0, sizeof(uint32_t), s));
+  A3D_CUDA_TRY(cudaMemsetAsync(w.ncl, 0, 2 * sizeof(uint32_t), s));
   A3D_PDL(sah_find_kernel, dim3(g), dim3(kThreads), 0, s, face_off, nmesh, n, w.parent, w.first, w.last, sah_max,
           w.clusters, w.ncl);
   A3D_TRY(n <= (int64_t)kSahMax * num_sms()

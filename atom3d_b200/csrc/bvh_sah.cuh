@@ -6,10 +6,13 @@
 // is rebuilt top-down with a binned surface-area heuristic (16 bins per
 // axis, centroid binning, cost = A_left N_left + A_right N_right, ties to
 // the lower axis and bin), down to single triangles:
-//   * nodes of more than kSahWarpMax triangles are split by the whole block
-//     (shared-memory bins, block scans for a stable partition);
-//   * smaller nodes are handed to the block's warps, each building its
-//     subtrees alone (warp shuffles and ballots, per-warp bins).
+//   * nodes of more than warp_max triangles are split by one block per
+//     cluster (sah_cluster_kernel: shared-memory bins, block scans for a
+//     stable partition);
+//   * smaller nodes go on a list that all warps of the chip share
+//     (sah_small_kernel); a warp splits them with bins of its own down to 32
+//     triangles and builds the rest of the subtree, all its nodes of a level
+//     at once, with one triangle a lane.
 // The triangles' centroids and boxes are read from global memory (L2
 // resident); the cluster's slice of the sorted face order is partitioned in
 // place.  Partitions are stable, reductions are min/max/integer sums, so the
@@ -34,7 +37,14 @@ namespace {
 
 constexpr int kSahMax = 16384;
 constexpr int kSahBins = 16;
-constexpr int kSahWarpMax = 128;
+// largest node handed to a warp (warp_max): 256, from kSahWideFrom triangles in
+// all on 512.  A block splits a cluster's larger nodes one after the other,
+// about 12 us each whatever their size, while a warp's chain of 512 triangles
+// takes longer than the rest of a small build (whole builds, at 128 / 256 /
+// 512 / 1024: 20,480 triangles 861 / 869 / 1004 / 1394 us, 327,680: 1.57 /
+// 1.47 / 1.53 / 1.87 ms, 1,310,720: 4.77 / 4.05 / 3.80 / 3.83 ms)
+constexpr int kSahWarpMin = 256, kSahWarpWide = 512;
+constexpr int64_t kSahWideFrom = 1 << 19;
 // block size of the cluster kernel: 1024 threads when the clusters are
 // about as many as the SMs (one mesh up to kSahMax x SMs triangles: each
 // block's 32 warps share out its small nodes), 256 when there are many
@@ -49,8 +59,11 @@ constexpr int kSahMaxDepth = 48;
 constexpr int kSahTiny = 2;
 constexpr int kSahCand = 3 * (kSahBins - 1);            // 45 split candidates
 constexpr int kBinWords = 3 * kSahBins * 7;              // count, lo xyz, hi xyz
-constexpr int kSahWarpStack = kSahWarpMax / 2;           // disjoint ranges of >= 2
-constexpr int kSahBlockStack = kSahMax / (kSahWarpMax + 1) + 2;
+// a warp's pending nodes: one per level, at most kSahMaxDepth levels and the
+// median splits of what is left below them
+constexpr int kSahWarpStack = kSahMaxDepth + 16;
+static_assert(kSahWarpWide <= (1 << 15), "median splits end within the stack");
+constexpr int kSahBlockStack = kSahMax / (kSahWarpMin + 1) + 2;  // disjoint ranges above warp_max
 
 // a node to split: local range [b, e) of its cluster, parent index (-1 for
 // the cluster root), side in the parent, depth inside the cluster
@@ -58,16 +71,21 @@ struct SahNode {
   int b, e, parent, sd;  // sd = side | depth << 1
 };
 
+// a node of at most warp_max triangles waiting for a warp
+struct SahSmall {
+  SahNode node;
+  int cluster;
+};
+
 template <int kThreads>
 struct SahSmem {
   static constexpr int kWarps = kThreads / 32;
-  uint32_t bins[kWarps + 1][kBinWords];  // per warp, then the block's
-  SahNode wstack[kWarps][kSahWarpStack];
+  uint32_t bins[kBinWords];
   SahNode bstack[kSahBlockStack];
   float red[kWarps][6];
   uint32_t wsum[kWarps];
   float cb[6];
-  int nsmall, nb, m, axis, kk, root_nat;
+  int nb, m, axis, kk, root_nat;
 };
 
 struct SahTree {
@@ -212,16 +230,16 @@ __device__ __forceinline__ void sah_emit(const SahTree& T, int f, int b, int m, 
   }
 }
 
-// One block per cluster (grid-stride over the device-side cluster list).
-// The cluster's slice of the sorted face order is partitioned in place
-// (tmp: a scratch slice of the same positions); small nodes waiting for the
-// warps are listed in `small` at the cluster's positions (a cluster of n
-// triangles has fewer than n of them).
+// One block per cluster (grid-stride over the device-side cluster list): the
+// nodes above warp_max.  The cluster's slice of the sorted face order is
+// partitioned in place (tmp: a scratch slice of the same positions); smaller
+// nodes are appended to `small` (a cluster of n triangles has fewer than n of
+// them), and root_nat[cluster] keeps the position its root would have had.
 template <int kThreads>
 __global__ void __launch_bounds__(kThreads)
     sah_cluster_kernel(const int32_t* __restrict__ clusters, const uint32_t* __restrict__ ncl, SahTree T,
-                       uint32_t* __restrict__ order, uint32_t* __restrict__ tmp_all, SahNode* __restrict__ small_all,
-                       SahPrims P) {
+                       uint32_t* __restrict__ order, uint32_t* __restrict__ tmp_all, SahSmall* __restrict__ small,
+                       uint32_t* __restrict__ nsmall, int32_t* __restrict__ root_nat, int warp_max, SahPrims P) {
   pdl_wait();
   extern __shared__ __align__(16) unsigned char sah_raw[];
   constexpr int kWarps = kThreads / 32;
@@ -236,16 +254,13 @@ __global__ void __launch_bounds__(kThreads)
     const int shift = (R == l) ? 1 : 0;
     uint32_t* ord = order + f;
     uint32_t* tmp = tmp_all + f;
-    SahNode* small = small_all + f;
     if (tid == 0) {
-      S.nsmall = 0;
       S.nb = 0;
       const SahNode root{0, n, -1, 0};
-      if (n > kSahWarpMax) S.bstack[S.nb++] = root;
-      else small[S.nsmall++] = root;
+      if (n > warp_max) S.bstack[S.nb++] = root;
+      else small[atomicAdd(nsmall, 1u)] = SahSmall{root, (int)ci};
     }
     __syncthreads();
-    // ---- stage A: nodes above kSahWarpMax, split by the whole block
     for (;;) {
       __syncthreads();
       const int nb = S.nb;
@@ -270,7 +285,7 @@ __global__ void __launch_bounds__(kThreads)
         }
       if (lane == 0)
         for (int a = 0; a < 3; ++a) { S.red[warp][a] = mn[a]; S.red[warp][3 + a] = mx[a]; }
-      sah_clear_bins(S.bins[kWarps], tid, kThreads);
+      sah_clear_bins(S.bins, tid, kThreads);
       __syncthreads();
       if (tid < 6) {
         float v = S.red[0][tid];
@@ -285,11 +300,11 @@ __global__ void __launch_bounds__(kThreads)
       for (int a = 0; a < 3; ++a) scale[a] = cb[3 + a] > cb[a] ? (float)kSahBins / (cb[3 + a] - cb[a]) : 0.f;
       const bool median = depth >= kSahMaxDepth;
       if (!median)
-        for (int i = b + tid; i < e; i += kThreads) sah_bin_prim(S.bins[kWarps], P, ord[i], cb, scale);
+        for (int i = b + tid; i < e; i += kThreads) sah_bin_prim(S.bins, P, ord[i], cb, scale);
       __syncthreads();
       if (warp == 0) {
         int axis = 0, kk = 0, nl = 0;
-        if (!median) nl = sah_pick(S.bins[kWarps], cb, lane, axis, kk);
+        if (!median) nl = sah_pick(S.bins, cb, lane, axis, kk);
         if (lane == 0) {
           S.m = nl > 0 ? b + nl : b + (e - b) / 2;
           S.axis = nl > 0 ? axis : -1;
@@ -334,104 +349,283 @@ __global__ void __launch_bounds__(kThreads)
       __syncthreads();
       if (tid == 0) {
         --S.nb;
-        if (is_root) S.root_nat = f + m - 1 + shift;
+        if (is_root) {
+          S.root_nat = f + m - 1 + shift;
+          root_nat[ci] = S.root_nat;
+        }
         const int label = sah_label(f, m, shift, R, S.root_nat, is_root);
         sah_emit(T, f, b, m, e, label, plabel, side, [&](int cb0, int ce0, int cs) {
           const SahNode ch{cb0, ce0, label, cs | ((depth + 1) << 1)};
-          if (ce0 - cb0 > kSahWarpMax) S.bstack[S.nb++] = ch;
-          else small[S.nsmall++] = ch;
+          if (ce0 - cb0 > warp_max) S.bstack[S.nb++] = ch;
+          else small[atomicAdd(nsmall, 1u)] = SahSmall{ch, (int)ci};
         });
       }
     }
     __syncthreads();
-    // ---- stage B: each warp builds the subtrees of its small nodes
-    uint32_t* wb = S.bins[warp];
-    SahNode* ws = S.wstack[warp];
-    const int nsmall = S.nsmall;
-    for (int si = warp; si < nsmall; si += kWarps) {
-      if (lane == 0) ws[0] = small[si];
-      int sp = 1;
-      __syncwarp();
-      while (sp > 0) {
-        const SahNode en = ws[sp - 1];
-        --sp;
-        __syncwarp();
-        const int b = en.b, e = en.e, side = en.sd & 1, depth = en.sd >> 1;
-        const int plabel = en.parent;
-        const bool is_root = plabel < 0;
-        int m = b + 1;
-        // at most kSahTiny triangles: split at the median position
-        if (e - b > kSahTiny) {
-          float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-          for (int i = b + lane; i < e; i += 32) {
-            const float4 c = __ldg(P.cen + ord[i]);
-            mn[0] = fminf(mn[0], c.x); mn[1] = fminf(mn[1], c.y); mn[2] = fminf(mn[2], c.z);
-            mx[0] = fmaxf(mx[0], c.x); mx[1] = fmaxf(mx[1], c.y); mx[2] = fmaxf(mx[2], c.z);
-          }
-          float cb[6], scale[3];
+  }
+}
+
+constexpr int kSahSmallThreads = 128;
+
+struct SahWarpSmem {
+  uint32_t bins[kBinWords];
+  SahNode stack[kSahWarpStack];
+  // the triangles of a subtree of at most 32, one a lane: box corners (lo.w:
+  // the bins per axis, 8 bits each), centroids (w: face id), and each lane's
+  // best split
+  float4 lo[32], hi[32], cen[32];
+  float cost[32];
+  int cand[32];  // candidate | left count << 8
+};
+
+// Builds the subtree of one node of 2..32 triangles, one triangle a lane, all
+// its nodes of a level at once.  The splits are those of the binned search: a
+// split after bin k keeps apart the same triangles as one after the highest
+// occupied bin up to k, so each lane evaluates, per axis, the split after its
+// own triangle's bin, over its node's triangles, and the node takes the
+// lowest (cost, candidate).  Bound by its instructions, about 48 per
+// (triangle, triangle) pair of a node; the bins of a warp-wide pass per node
+// took ten times as many, half of them on nodes of 3 or 4 triangles.
+__device__ __forceinline__ void sah_build32(SahWarpSmem& S, const SahTree& T, const SahPrims& P,
+                                            uint32_t* __restrict__ ord, int f, int shift, int R, int& root_nat,
+                                            const SahNode& en, int lane) {
+  const unsigned FULL = 0xffffffffu;
+  const int n = en.e - en.b;
+  int s = 0, e = n, plabel = en.parent, side = en.sd & 1, depth = en.sd >> 1;
+  uint32_t id = 0;
+  if (lane < n) {
+    id = ord[en.b + lane];
+    float4 c = __ldg(P.cen + id);
+    c.w = __uint_as_float(id);
+    S.cen[lane] = c;
+    S.lo[lane] = __ldg(P.lo + id);
+    S.hi[lane] = __ldg(P.hi + id);
+  } else {
+    s = e = lane;  // no triangle: an empty node
+  }
+  __syncwarp();
+  int longest = n;
+  while (longest > 1) {
+    const int len = e - s;
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    int bin[3] = {0, 0, 0};
+    bool flat[3] = {true, true, true};
+    if (len > kSahTiny && depth < kSahMaxDepth) {
+      // centroid bounds of the lane's node and the bins of its own centroid
+      float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+      for (int j = s; j < e; ++j) {
+        const float4 o = S.cen[j];
+        mn[0] = fminf(mn[0], o.x); mn[1] = fminf(mn[1], o.y); mn[2] = fminf(mn[2], o.z);
+        mx[0] = fmaxf(mx[0], o.x); mx[1] = fmaxf(mx[1], o.y); mx[2] = fmaxf(mx[2], o.z);
+      }
+      c = S.cen[lane];
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1)
+      for (int a = 0; a < 3; ++a) {
+        flat[a] = !(mx[a] > mn[a]);
+        if (!flat[a]) bin[a] = sah_bin(sah_c(c, a), mn[a], (float)kSahBins / (mx[a] - mn[a]));
+      }
+      S.lo[lane].w = __int_as_float(bin[0] | (bin[1] << 8) | (bin[2] << 16));
+    }
+    __syncwarp();
+    float cost = INFINITY;
+    int cand = 0x7fffffff, nl = 0;
+    if (len > kSahTiny && depth < kSahMaxDepth) {
+      float l[3][6], r[3][6];
+      int cl[3] = {0, 0, 0};
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-              mn[a] = fminf(mn[a], __shfl_xor_sync(FULL, mn[a], o));
-              mx[a] = fmaxf(mx[a], __shfl_xor_sync(FULL, mx[a], o));
-            }
+      for (int a = 0; a < 3; ++a)
 #pragma unroll
-          for (int a = 0; a < 3; ++a) {
-            cb[a] = mn[a];
-            cb[3 + a] = mx[a];
-            scale[a] = mx[a] > mn[a] ? (float)kSahBins / (mx[a] - mn[a]) : 0.f;
-          }
-          int nl = 0, axis = 0, kk = 0;
-          if (depth < kSahMaxDepth) {
-            sah_clear_bins(wb, lane, 32);
-            __syncwarp();
-            for (int i = b + lane; i < e; i += 32) sah_bin_prim(wb, P, ord[i], cb, scale);
-            __syncwarp();
-            nl = sah_pick(wb, cb, lane, axis, kk);
-            __syncwarp();
-          }
-          if (nl > 0) {
-            m = b + nl;
-            int lbase = b, rbase = m;
-            for (int i0 = b; i0 < e; i0 += 32) {
-              const int i = i0 + lane;
-              uint32_t p = 0;
-              bool lft = false;
-              if (i < e) {
-                p = ord[i];
-                lft = sah_bin(sah_c(__ldg(P.cen + p), axis), cb[axis], scale[axis]) < kk;
-              }
-              const unsigned bl = __ballot_sync(FULL, lft), br = __ballot_sync(FULL, i < e && !lft);
-              const unsigned below = (1u << lane) - 1u;
-              if (i < e) {
-                if (lft) tmp[lbase + __popc(bl & below)] = p;
-                else tmp[rbase + __popc(br & below)] = p;
-              }
-              lbase += __popc(bl);
-              rbase += __popc(br);
-            }
-            __syncwarp();
-            for (int i = b + lane; i < e; i += 32) ord[i] = tmp[i];
-            __syncwarp();
+        for (int x = 0; x < 3; ++x) {
+          l[a][x] = r[a][x] = INFINITY;
+          l[a][3 + x] = r[a][3 + x] = -INFINITY;
+        }
+      for (int j = s; j < e; ++j) {
+        const float4 lo = S.lo[j], hi = S.hi[j];
+        const int ob = __float_as_int(lo.w);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          if (((ob >> (8 * a)) & 0xff) <= bin[a]) {
+            ++cl[a];
+            l[a][0] = fminf(l[a][0], lo.x); l[a][1] = fminf(l[a][1], lo.y); l[a][2] = fminf(l[a][2], lo.z);
+            l[a][3] = fmaxf(l[a][3], hi.x); l[a][4] = fmaxf(l[a][4], hi.y); l[a][5] = fmaxf(l[a][5], hi.z);
           } else {
-            m = b + (e - b) / 2;
+            r[a][0] = fminf(r[a][0], lo.x); r[a][1] = fminf(r[a][1], lo.y); r[a][2] = fminf(r[a][2], lo.z);
+            r[a][3] = fmaxf(r[a][3], hi.x); r[a][4] = fmaxf(r[a][4], hi.y); r[a][5] = fmaxf(r[a][5], hi.z);
           }
-        } else {
-          m = b + (e - b) / 2;
         }
-        if (lane == 0) {
-          if (is_root) S.root_nat = f + m - 1 + shift;
-          const int label = sah_label(f, m, shift, R, S.root_nat, is_root);
-          sah_emit(T, f, b, m, e, label, plabel, side, [&](int cb0, int ce0, int cs) {
-            ws[sp++] = SahNode{cb0, ce0, label, cs | ((depth + 1) << 1)};
-          });
+      }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        if (flat[a] || cl[a] == len) continue;
+        const float v = sah_half_area(l[a][0], l[a][1], l[a][2], l[a][3], l[a][4], l[a][5]) * (float)cl[a] +
+                        sah_half_area(r[a][0], r[a][1], r[a][2], r[a][3], r[a][4], r[a][5]) * (float)(len - cl[a]);
+        if (v < cost) {
+          cost = v;
+          cand = a * (kSahBins - 1) + bin[a];
+          nl = cl[a];
         }
-        sp = __shfl_sync(FULL, sp, 0);
-        __syncwarp();
       }
     }
-    __syncthreads();
+    S.cost[lane] = cost;
+    S.cand[lane] = cand < 0x7fffffff ? (cand | (nl << 8)) : 0x7fffffff;
+    __syncwarp();
+    // the node's split: the lowest (cost, candidate) of its lanes
+    int best = 0x7fffffff;
+    if (len > kSahTiny && depth < kSahMaxDepth) {
+      float bc = INFINITY;
+      for (int j = s; j < e; ++j) {
+        const float oc = S.cost[j];
+        const int o = S.cand[j];
+        if (oc < bc || (oc == bc && (o & 0xff) < (best & 0xff))) {
+          bc = oc;
+          best = o;
+        }
+      }
+      if (!(bc < INFINITY)) best = 0x7fffffff;
+    }
+    bool left;
+    int m;
+    if (best != 0x7fffffff) {
+      const int axis = (best & 0xff) / (kSahBins - 1), kk = (best & 0xff) % (kSahBins - 1);
+      left = bin[axis == 0 ? 0 : (axis == 1 ? 1 : 2)] <= kk;
+      m = s + (best >> 8);
+    } else {
+      m = s + len / 2;
+      left = lane < m;
+    }
+    // stable partition: each triangle to its lane in the children's order
+    const unsigned seg = len > 0 ? (0xffffffffu >> (32 - len)) << s : 0u;
+    const unsigned lm = __ballot_sync(FULL, left) & seg;
+    const unsigned below = (1u << lane) - 1u;
+    const int to = left ? s + __popc(lm & below) : m + __popc(seg & ~lm & below);
+    const float4 mylo = S.lo[lane], myhi = S.hi[lane], myc = S.cen[lane];
+    __syncwarp();
+    if (len > 1) {
+      S.lo[to] = mylo;
+      S.hi[to] = myhi;
+      S.cen[to] = myc;
+    }
+    int label = 0;
+    if (len > 1) {
+      const bool is_root = plabel < 0;
+      if (is_root) root_nat = f + en.b + m - 1 + shift;
+      label = sah_label(f, en.b + m, shift, R, root_nat, is_root);
+      if (lane == s)
+        sah_emit(T, f, en.b + s, en.b + m, en.b + e, label, plabel, side, [](int, int, int) {});
+      plabel = label;
+      side = lane < m ? 0 : 1;
+      ++depth;
+      if (lane < m) e = m;
+      else s = m;
+    }
+    __syncwarp();
+    longest = __reduce_max_sync(FULL, e - s);
+  }
+  if (lane < n) ord[en.b + lane] = __float_as_uint(S.cen[lane].w);
+  __syncwarp();
+}
+
+// One warp per node of the small list (grid-stride; the nodes' order in the
+// list does not matter, each owns its range of the face order).
+__global__ void __launch_bounds__(kSahSmallThreads)
+    sah_small_kernel(const SahSmall* __restrict__ small, const uint32_t* __restrict__ nsmall,
+                     const int32_t* __restrict__ clusters, const int32_t* __restrict__ root_nats, SahTree T,
+                     uint32_t* __restrict__ order, uint32_t* __restrict__ tmp_all, SahPrims P) {
+  pdl_wait();
+  __shared__ SahWarpSmem smem[kSahSmallThreads / 32];
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  SahWarpSmem& S = smem[threadIdx.x >> 5];
+  uint32_t* wb = S.bins;
+  const uint32_t count = *nsmall, warps = gridDim.x * (kSahSmallThreads / 32);
+  for (uint32_t si = blockIdx.x * (kSahSmallThreads / 32) + (threadIdx.x >> 5); si < count; si += warps) {
+    const SahSmall it = small[si];
+    const int R = clusters[it.cluster];
+    // the cluster's range: a root of this list still has the radix tree's own
+    // first and last; a split cluster's root was given the same ones
+    const int f = T.first[R], l = T.last[R];
+    const int shift = (R == l) ? 1 : 0;
+    uint32_t* ord = order + f;
+    uint32_t* tmp = tmp_all + f;
+    int root_nat = it.node.parent < 0 ? 0 : root_nats[it.cluster];
+    if (lane == 0) S.stack[0] = it.node;
+    int sp = 1;
+    __syncwarp();
+    while (sp > 0) {
+      const SahNode en = S.stack[sp - 1];
+      --sp;
+      __syncwarp();
+      if (en.e - en.b <= 32) {
+        sah_build32(S, T, P, ord, f, shift, R, root_nat, en, lane);
+        continue;
+      }
+      const int b = en.b, e = en.e, side = en.sd & 1, depth = en.sd >> 1;
+      const int plabel = en.parent;
+      const bool is_root = plabel < 0;
+      int m = b + (e - b) / 2;
+      float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+      for (int i = b + lane; i < e; i += 32) {
+        const float4 c = __ldg(P.cen + ord[i]);
+        mn[0] = fminf(mn[0], c.x); mn[1] = fminf(mn[1], c.y); mn[2] = fminf(mn[2], c.z);
+        mx[0] = fmaxf(mx[0], c.x); mx[1] = fmaxf(mx[1], c.y); mx[2] = fmaxf(mx[2], c.z);
+      }
+      float cb[6], scale[3];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+          mn[a] = fminf(mn[a], __shfl_xor_sync(FULL, mn[a], o));
+          mx[a] = fmaxf(mx[a], __shfl_xor_sync(FULL, mx[a], o));
+        }
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        cb[a] = mn[a];
+        cb[3 + a] = mx[a];
+        scale[a] = mx[a] > mn[a] ? (float)kSahBins / (mx[a] - mn[a]) : 0.f;
+      }
+      int nl = 0, axis = 0, kk = 0;
+      if (depth < kSahMaxDepth) {
+        sah_clear_bins(wb, lane, 32);
+        __syncwarp();
+        for (int i = b + lane; i < e; i += 32) sah_bin_prim(wb, P, ord[i], cb, scale);
+        __syncwarp();
+        nl = sah_pick(wb, cb, lane, axis, kk);
+        __syncwarp();
+      }
+      if (nl > 0) {
+        m = b + nl;
+        int lbase = b, rbase = m;
+        for (int i0 = b; i0 < e; i0 += 32) {
+          const int i = i0 + lane;
+          uint32_t p = 0;
+          bool lft = false;
+          if (i < e) {
+            p = ord[i];
+            lft = sah_bin(sah_c(__ldg(P.cen + p), axis), cb[axis], scale[axis]) < kk;
+          }
+          const unsigned bl = __ballot_sync(FULL, lft), br = __ballot_sync(FULL, i < e && !lft);
+          const unsigned below = (1u << lane) - 1u;
+          if (i < e) {
+            if (lft) tmp[lbase + __popc(bl & below)] = p;
+            else tmp[rbase + __popc(br & below)] = p;
+          }
+          lbase += __popc(bl);
+          rbase += __popc(br);
+        }
+        __syncwarp();
+        for (int i = b + lane; i < e; i += 32) ord[i] = tmp[i];
+        __syncwarp();
+      }
+      if (is_root) root_nat = f + m - 1 + shift;
+      if (lane == 0) {
+        const int label = sah_label(f, m, shift, R, root_nat, is_root);
+        sah_emit(T, f, b, m, e, label, plabel, side, [&](int cb0, int ce0, int cs) {
+          S.stack[sp++] = SahNode{cb0, ce0, label, cs | ((depth + 1) << 1)};
+        });
+      }
+      sp = __shfl_sync(FULL, sp, 0);
+      __syncwarp();
+    }
   }
 }
 
