@@ -210,81 +210,205 @@ int fill_async(T* p, int64_t n, T v, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // stable LSD radix sort of (key, uint32 value) pairs, 8-bit digits
 // ---------------------------------------------------------------------------
+// Per digit an upsweep (the digit counts of each tile) and a downsweep.  The
+// downsweep ranks a tile's keys warp by warp with ballots against counters
+// of the warp's own, so it needs three block barriers a tile, then brings the
+// tile into digit order in shared memory and writes it in runs of consecutive
+// addresses.  (Ranking and scattering 256 keys at a time took 64 barriers a
+// tile of 4,096 keys and one sector per key.)  Tiles are 4,096 keys, fewer
+// while there would be less than two tiles an SM.
 constexpr int kRsThreads = 256;
-constexpr int kRsItems = 16;
-constexpr int kRsTile = kRsThreads * kRsItems;
+constexpr int kRsWarps = kRsThreads / 32;
+constexpr int kRsMaxItems = 16;
+// up to this many tiles a downsweep block adds up the tiles' counts itself
+// (kRsFuseTiles x 1 KB from L2) instead of a scan launched in between
+constexpr int64_t kRsFuseTiles = 128;
 
-template <typename K>
-__global__ void __launch_bounds__(kRsThreads) rs_upsweep_kernel(const K* __restrict__ keys, int64_t n, int shift,
-                                                                uint32_t* __restrict__ hist, int64_t num_tiles) {
-  pdl_wait();
-  __shared__ uint32_t s_hist[256];
-  s_hist[threadIdx.x] = 0;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kRsTile;
-  const int lane = threadIdx.x & 31;
-#pragma unroll 4
-  for (int i = 0; i < kRsItems; ++i) {
-    int64_t idx = base + (int64_t)i * kRsThreads + threadIdx.x;
-    uint32_t d = idx < n ? (uint32_t)((keys[idx] >> shift) & 0xff) : 0x100u;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    if (d < 256u && lane == __ffs(peers) - 1) atomicAdd(&s_hist[d], (uint32_t)__popc(peers));
+// the lanes whose 8-bit digit equals this lane's, by one ballot a bit (in a
+// quarter of the time of match_any, whose rate falls with the distinct values)
+__device__ __forceinline__ unsigned rs_peers(uint32_t d) {
+  unsigned peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const unsigned ones = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+    peers &= (d >> b) & 1u ? ones : ~ones;
   }
-  __syncthreads();
-  hist[(int64_t)threadIdx.x * num_tiles + blockIdx.x] = s_hist[threadIdx.x];
+  return peers;
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kRsThreads)
-    rs_downsweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
-                        uint32_t* __restrict__ vals_out, int64_t n, int shift, const uint32_t* __restrict__ offsets,
-                        int64_t num_tiles) {
-  pdl_wait();
-  __shared__ uint32_t s_base[256];
-  __shared__ uint32_t s_warp[kRsThreads / 32][256];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  s_base[t] = offsets[(int64_t)t * num_tiles + blockIdx.x];
-  const int64_t base = (int64_t)blockIdx.x * kRsTile;
-  for (int c = 0; c < kRsItems; ++c) {
-#pragma unroll
-    for (int w = 0; w < kRsThreads / 32; ++w) s_warp[w][t] = 0;
-    __syncthreads();
-    const int64_t idx = base + (int64_t)c * kRsThreads + t;
-    const bool valid = idx < n;
-    K k = 0;
-    uint32_t v = 0, d = 0x100u;
-    if (valid) {
-      k = keys_in[idx];
-      v = vals_in[idx];
-      d = (uint32_t)((k >> shift) & 0xff);
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int rank = __popc(peers & ((1u << lane) - 1u));
-    if (valid && lane == __ffs(peers) - 1) s_warp[warp][d] = (uint32_t)__popc(peers);
-    __syncthreads();
-    uint32_t run = s_base[t];
-#pragma unroll
-    for (int w = 0; w < kRsThreads / 32; ++w) {
-      uint32_t cnt = s_warp[w][t];
-      s_warp[w][t] = run;
-      run += cnt;
-    }
-    s_base[t] = run;
-    __syncthreads();
-    if (valid) {
-      const uint32_t pos = s_warp[warp][d] + (uint32_t)rank;
-      keys_out[pos] = k;
-      vals_out[pos] = v;
-    }
-    __syncthreads();
-  }
+// keys a thread of a sort of n keys: the fused form's tiles up to 131,072
+// keys, above it two tiles an SM up to 16
+inline int radix_items(int64_t n) {
+  if (n <= kRsFuseTiles * 2 * kRsThreads) return 2;
+  int items = kRsMaxItems;
+  while (items > 4 && n < (int64_t)items * kRsThreads * 296) items >>= 1;
+  return items;
 }
-
-inline int64_t radix_num_tiles(int64_t n) { return ceil_div(n > 0 ? n : 1, kRsTile); }
+inline int64_t radix_num_tiles(int64_t n) {
+  return ceil_div(n > 0 ? n : 1, (int64_t)radix_items(n) * kRsThreads);
+}
 // uint32 elements of scratch needed by radix_sort_pairs
 inline size_t radix_sort_scratch_elems(int64_t n) {
   const int64_t h = 256 * radix_num_tiles(n);
   return (size_t)h + scan_workspace_elems(h);
+}
+
+// hist: [digit][tile] for the scanned form, [tile][digit] for the fused one
+template <typename K, int kItems, bool kFused>
+__global__ void __launch_bounds__(kRsThreads)
+    rs_upsweep_kernel(const K* __restrict__ keys, int64_t n, int shift, uint32_t* __restrict__ hist,
+                      int64_t num_tiles) {
+  pdl_wait();
+  __shared__ uint32_t s_hist[256];
+  s_hist[threadIdx.x] = 0;
+  const int64_t base = (int64_t)blockIdx.x * (kItems * kRsThreads);
+  const int lane = threadIdx.x & 31;
+  uint32_t d[kItems];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int64_t idx = base + (int64_t)i * kRsThreads + threadIdx.x;
+    d[i] = idx < n ? (uint32_t)((keys[idx] >> shift) & 0xff) : 0x100u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    // a warp of one digit (sorted or narrow keys) adds once
+    const uint32_t d0 = __shfl_sync(0xffffffffu, d[i], 0);
+    if (__all_sync(0xffffffffu, d[i] == d0)) {
+      if (lane == 0 && d0 < 256u) atomicAdd(&s_hist[d0], 32u);
+    } else if (d[i] < 256u) {
+      atomicAdd(&s_hist[d[i]], 1u);
+    }
+  }
+  __syncthreads();
+  hist[kFused ? (int64_t)blockIdx.x * 256 + threadIdx.x : (int64_t)threadIdx.x * num_tiles + blockIdx.x] =
+      s_hist[threadIdx.x];
+}
+
+template <typename K, int kItems>
+struct RsSmem {
+  uint32_t warp[kRsWarps][256];  // digit counts, then the warps' offsets in the digit
+  uint32_t start[256];           // where a digit starts in the tile
+  uint32_t out[256];             // where it goes, less that
+  uint32_t scan[kBlockScanSlots];
+  K buf[kItems * kRsThreads];    // the tile in digit order: keys, then values
+};
+
+// resident blocks an SM: more would spill the 16 keys a thread holds
+template <typename K>
+constexpr int kRsBlocks = sizeof(K) == 8 ? 3 : 4;
+
+template <typename K, int kItems, bool kFused>
+__global__ void __launch_bounds__(kRsThreads, kRsBlocks<K>)
+    rs_downsweep_kernel(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
+                        uint32_t* __restrict__ vals_out, int64_t n, int shift, const uint32_t* __restrict__ hist,
+                        int64_t num_tiles) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char rs_raw[];
+  RsSmem<K, kItems>& S = *reinterpret_cast<RsSmem<K, kItems>*>(rs_raw);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+#pragma unroll
+  for (int w = 0; w < kRsWarps; ++w) S.warp[w][t] = 0;
+  // a warp's keys are consecutive, 32 a step, so ranks follow the input order
+  const int64_t base = (int64_t)blockIdx.x * (kItems * kRsThreads);
+  const int64_t mine = base + (int64_t)warp * (kItems * 32) + lane;
+  K key[kItems];
+  uint32_t rank[kItems];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int64_t idx = mine + i * 32;
+    key[i] = idx < n ? keys_in[idx] : ~K(0);  // past the end: after every other key of digit 255
+  }
+  // this block's place in each digit's output
+  uint32_t before = 0, total = 0;
+  if constexpr (kFused) {
+    for (int64_t j = 0; j < num_tiles; ++j) {
+      const uint32_t c = hist[j * 256 + t];
+      before += j < (int64_t)blockIdx.x ? c : 0u;
+      total += c;
+    }
+  } else {
+    before = hist[(int64_t)t * num_tiles + blockIdx.x];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const uint32_t d = (uint32_t)((key[i] >> shift) & 0xff);
+    const unsigned peers = rs_peers(d);
+    const uint32_t c = S.warp[warp][d];
+    rank[i] = c + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+    if (lane == __ffs(peers) - 1) S.warp[warp][d] = c + (uint32_t)__popc(peers);
+    __syncwarp();
+  }
+  if constexpr (kFused) before += block_exclusive_scan<uint32_t>(total, S.scan, nullptr);
+  __syncthreads();
+  uint32_t run = 0;
+#pragma unroll
+  for (int w = 0; w < kRsWarps; ++w) {
+    const uint32_t c = S.warp[w][t];
+    S.warp[w][t] = run;
+    run += c;
+  }
+  const uint32_t start = block_exclusive_scan<uint32_t>(run, S.scan, nullptr);
+  S.start[t] = start;
+  S.out[t] = before - start;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const uint32_t d = (uint32_t)((key[i] >> shift) & 0xff);
+    rank[i] += S.start[d] + S.warp[warp][d];
+    S.buf[rank[i]] = key[i];
+  }
+  __syncthreads();
+  const int64_t left = n - base;
+  const int count = left < kItems * kRsThreads ? (int)left : kItems * kRsThreads;
+  uint32_t to[kItems];
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int at = i * kRsThreads + t;
+    to[i] = 0;
+    if (at < count) {
+      const K k = S.buf[at];
+      to[i] = S.out[(uint32_t)((k >> shift) & 0xff)] + (uint32_t)at;
+      keys_out[to[i]] = k;
+    }
+  }
+  __syncthreads();
+  uint32_t* vbuf = reinterpret_cast<uint32_t*>(S.buf);
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int64_t idx = mine + i * 32;
+    vbuf[rank[i]] = idx < n ? vals_in[idx] : 0u;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kItems; ++i) {
+    const int at = i * kRsThreads + t;
+    if (at < count) vals_out[to[i]] = vbuf[at];
+  }
+}
+
+template <typename K, int kItems, bool kFused>
+int radix_pass(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, int64_t n, int shift, uint32_t* hist,
+               uint32_t* tmp, int64_t nt, cudaStream_t s) {
+  const size_t smem = sizeof(RsSmem<K, kItems>);
+  if (smem > 48 * 1024) {
+    // opt in above 48 KB, once per device
+    static bool done[kMaxDevices] = {false};
+    int dev = 0;
+    A3D_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxDevices || !done[dev]) {
+      A3D_CUDA_TRY(cudaFuncSetAttribute(rs_downsweep_kernel<K, kItems, kFused>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (dev >= 0 && dev < kMaxDevices) done[dev] = true;
+    }
+  }
+  A3D_PDL((rs_upsweep_kernel<K, kItems, kFused>), dim3((unsigned)nt), dim3(kRsThreads), 0, s, kin, n, shift, hist, nt);
+  if (!kFused) A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(hist, hist, 256 * nt, tmp, (uint32_t*)nullptr, s)));
+  A3D_PDL((rs_downsweep_kernel<K, kItems, kFused>), dim3((unsigned)nt), dim3(kRsThreads), smem, s, kin, vin, kout,
+          vout, n, shift, (const uint32_t*)hist, nt);
+  return A3D_OK;
 }
 
 // Sorts (keys, vals) by bits [begin_bit, end_bit) of the key.  Ping-pongs
@@ -296,16 +420,22 @@ int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, i
   *result_in_alt = false;
   if (n <= 1) return A3D_OK;
   A3D_REQUIRE(n < (int64_t)0xffffffffll, A3D_ERR_ARGUMENT, "radix sort: too many elements");
+  const int items = radix_items(n);
   const int64_t nt = radix_num_tiles(n);
   uint32_t* hist = scratch;
   uint32_t* tmp = scratch + 256 * nt;
   K *kin = keys, *kout = keys_alt;
   uint32_t *vin = vals, *vout = vals_alt;
   for (int shift = begin_bit; shift < end_bit; shift += 8) {
-    A3D_PDL(rs_upsweep_kernel<K>, dim3((unsigned)nt), dim3(kRsThreads), 0, s, (const K*)kin, n, shift, hist, nt);
-    A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(hist, hist, 256 * nt, tmp, (uint32_t*)nullptr, s)));
-    A3D_PDL(rs_downsweep_kernel<K>, dim3((unsigned)nt), dim3(kRsThreads), 0, s, (const K*)kin, (const uint32_t*)vin,
-            kout, vout, n, shift, (const uint32_t*)hist, nt);
+    switch (items) {
+      case 16: A3D_TRY((radix_pass<K, 16, false>(kin, vin, kout, vout, n, shift, hist, tmp, nt, s))); break;
+      case 8: A3D_TRY((radix_pass<K, 8, false>(kin, vin, kout, vout, n, shift, hist, tmp, nt, s))); break;
+      case 4:
+        A3D_TRY(nt <= kRsFuseTiles ? (radix_pass<K, 4, true>(kin, vin, kout, vout, n, shift, hist, tmp, nt, s))
+                                   : (radix_pass<K, 4, false>(kin, vin, kout, vout, n, shift, hist, tmp, nt, s)));
+        break;
+      default: A3D_TRY((radix_pass<K, 2, true>(kin, vin, kout, vout, n, shift, hist, tmp, nt, s)));
+    }
     K* tk = kin; kin = kout; kout = tk;
     uint32_t* tv = vin; vin = vout; vout = tv;
     *result_in_alt = !*result_in_alt;

@@ -4,8 +4,8 @@
 // Replaces bvh_udf_kernel (atom3d/kernels/bvh_kernels.cu:363-463) and the
 // PyTorch sign gathers of MeshBVH._compute_sign (atom3d/core/mesh_bvh.py:
 // 759-827).  Design:
-//   * queries are Morton-sorted (30-bit key, in-house radix sort) so a warp
-//     walks neighbouring regions of the tree together;
+//   * many queries are Morton-sorted (in-house radix sort) so a warp walks
+//     neighbouring regions of the tree together;
 //   * a group of four or two lanes walks the tree for one query: each lane
 //     tests one or two of a node's children, first the box, then the disc
 //     about the child's triangles (bvh_children.cuh); the nearest qualifying
@@ -966,16 +966,16 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void query_morton_kernel(const float* __restrict__ pts, int64_t n, float lox, float loy, float loz,
-                                    float ix, float iy, float iz, uint32_t* __restrict__ keys,
+                                    float inv, float qmax, uint32_t* __restrict__ keys,
                                     uint32_t* __restrict__ vals) {
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float q[3] = {(pts[3 * i] - lox) * ix, (pts[3 * i + 1] - loy) * iy, (pts[3 * i + 2] - loz) * iz};
+  const float q[3] = {(pts[3 * i] - lox) * inv, (pts[3 * i + 1] - loy) * inv, (pts[3 * i + 2] - loz) * inv};
   uint32_t code = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    float t = fminf(fmaxf(q[a], 0.f), 1023.f);
+    float t = fminf(fmaxf(q[a], 0.f), qmax);
     if (!(t == t)) t = 0.f;
     code |= (uint32_t)spread3_21((uint64_t)t) << a;
   }
@@ -984,6 +984,16 @@ __global__ void query_morton_kernel(const float* __restrict__ pts, int64_t n, fl
 }
 
 constexpr int kStatusWords = 8;
+
+// Queries are Morton-sorted from kSortMin on.  Below it what the sorted order
+// saves (L1 misses, a seed from the neighbour) does not pay for the sort, even
+// for queries in random order: 100,000 / 1M / 2M / 4M queries in random order
+// against 1,310,720 triangles take 0.59 / 3.14 / 5.77 / 10.8 ms unsorted and
+// 0.75 / 3.26 / 5.55 / 8.85 ms sorted, against 20,480 rough triangles 0.25 /
+// 1.49 / 2.85 / 5.07 and 0.28 / 1.46 / 2.66 / 4.23.  Below kSortFine 8 bits an
+// axis (three passes) order as well as 10 (four), above 10 gain about 1%.
+constexpr int64_t kSortMin = 3 << 19;
+constexpr int64_t kSortFine = 8 << 20;
 
 struct UdfWs {
   uint32_t* keys;
@@ -1212,21 +1222,24 @@ extern "C" int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, c
   }
   const int64_t n = num_points;
   const uint32_t* perm = nullptr;
-  if (flags & A3D_UDF_SORT_QUERIES) {
+  const bool sort = (flags & A3D_UDF_SORT_QUERIES) != 0 && n >= kSortMin;
+  if (sort) {
     const float ext[3] = {bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2]};
     float emax = fmaxf(ext[0], fmaxf(ext[1], ext[2]));
     emax = emax > 0.f ? emax : 1.f;
     // queries may lie outside the mesh box: use a cube of twice its extent
     const float lo[3] = {0.5f * (bvh->lo[0] + bvh->hi[0]) - emax, 0.5f * (bvh->lo[1] + bvh->hi[1]) - emax,
                          0.5f * (bvh->lo[2] + bvh->hi[2]) - emax};
-    const float inv = 1023.0f / (2.0f * emax);
-    A3D_PDL(query_morton_kernel, dim3((unsigned)ceil_div(n, 256)), dim3(256), 0, s, points, n, lo[0], lo[1], lo[2], inv,
-            inv, inv, w.keys, w.vals);
+    const int bits = n < kSortFine ? 8 : 10;
+    const float qmax = (float)((1 << bits) - 1);
+    A3D_PDL(query_morton_kernel, dim3((unsigned)ceil_div(n, 256)), dim3(256), 0, s, points, n, lo[0], lo[1], lo[2],
+            qmax / (2.0f * emax), qmax, w.keys, w.vals);
     bool alt = false;
-    A3D_TRY(radix_sort_pairs<uint32_t>(w.keys, w.vals, w.keys_alt, w.vals_alt, n, 0, 32, w.rs_scratch, &alt, s));
+    A3D_TRY(radix_sort_pairs<uint32_t>(w.keys, w.vals, w.keys_alt, w.vals_alt, n, 0, 3 * bits, w.rs_scratch, &alt, s));
     perm = alt ? w.vals_alt : w.vals;
   }
-  const bool coherent = perm != nullptr || (flags & A3D_UDF_ASSUME_SORTED) != 0;
+  // in the caller's order when there are few: the same traversal, no sort
+  const bool coherent = (flags & A3D_UDF_SORT_QUERIES) != 0 || (flags & A3D_UDF_ASSUME_SORTED) != 0;
   const uint32_t seeding = ((flags & A3D_UDF_NO_REUSE) ? 0u : kSeedReuse) |
                            ((flags & A3D_UDF_BOUND_SEEDS) && bound ? kSeedBoundOnly : 0u);
   A3D_CUDA_TRY(cudaMemsetAsync(w.nrerun, 0, kStatusWords * sizeof(uint32_t), s));
@@ -1378,12 +1391,15 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_childr
   for (int64_t base = 0; base < n; base += kBatchChunk) {
     const int64_t cn = n - base < kBatchChunk ? n - base : kBatchChunk;
     const float* pts = points + 3 * base;
-    A3D_PDL(batch_query_morton_kernel, dim3((unsigned)ceil_div(cn, 256)), dim3(256), 0, s, pts, cn, base, qoff,
-            bvh->num_meshes, bvh->bounds, bits, w.keys, w.vals);
-    bool alt = false;
-    A3D_TRY(radix_sort_pairs<uint32_t>(w.keys, w.vals, w.keys_alt, w.vals_alt, cn, 0, 3 * bits + mbits,
-                                       w.rs_scratch, &alt, s));
-    const uint32_t* perm = alt ? w.vals_alt : w.vals;
+    const uint32_t* perm = nullptr;  // the caller's order (mesh by mesh) when there are few
+    if (cn >= kSortMin) {
+      A3D_PDL(batch_query_morton_kernel, dim3((unsigned)ceil_div(cn, 256)), dim3(256), 0, s, pts, cn, base, qoff,
+              bvh->num_meshes, bvh->bounds, bits, w.keys, w.vals);
+      bool alt = false;
+      A3D_TRY(radix_sort_pairs<uint32_t>(w.keys, w.vals, w.keys_alt, w.vals_alt, cn, 0, 3 * bits + mbits,
+                                         w.rs_scratch, &alt, s));
+      perm = alt ? w.vals_alt : w.vals;
+    }
     // per chunk: the re-run list and the pool counter start at zero
     A3D_CUDA_TRY(cudaMemsetAsync(w.nrerun, 0, sizeof(uint32_t), s));
     A3D_CUDA_TRY(cudaMemsetAsync(w.nrerun + 2, 0, sizeof(uint32_t), s));

@@ -115,7 +115,8 @@ typedef struct a3d_sign_data {
  * uvw may be NULL.  bound (nullable) is a per-query upper bound on the
  * unsigned distance that seeds the pruning radius; queries whose bound proves
  * too small are re-run unbounded, so results never depend on it.
- * flags: A3D_UDF_SORT_QUERIES (Morton-sort queries for warp coherence),
+ * flags: A3D_UDF_SORT_QUERIES (Morton-sort queries for warp coherence where
+ * there are enough of them for it to pay),
  * A3D_UDF_ASSUME_SORTED (caller's order is already coherent).
  * stats (nullable, device, 4 x uint64): node visits, triangle tests,
  * bound misses, stack spills.  */
