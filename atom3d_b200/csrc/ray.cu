@@ -24,12 +24,9 @@ namespace a3d {
 namespace {
 
 constexpr int kRayThreads = 128;
-// shared-memory stack entries per ray: 20 KB per 128-thread block, and the
-// nearest-hit kernel bounded to 48 registers, so that 10 blocks (40 warps)
-// are resident per SM; a ray that needs more entries is re-run with a deep
-// local stack
+// shared-memory stack entries per ray; a ray that needs more is re-run with a
+// deep local stack
 constexpr int kRayShared = 20;
-constexpr int kRayBlocksPerSm = 10;
 constexpr int kRayDeep = 256;    // local-memory stack of the re-run kernel
 constexpr int kAllDepth = 192;   // node stack of the all-hit traversals
 constexpr int kParityCap = 256;  // hits per (point, direction) kept by the parity kernel
@@ -71,13 +68,25 @@ __device__ __forceinline__ float ray_tri(const Tri& t, V3 ro, V3 rd) {
   const V3 e1 = vsub(t.b, t.a), e2 = vsub(t.c, t.a);
   const V3 h = vcross(rd, e2);
   const float det = vdot(e1, h);
-  if (fabsf(det) < 1e-8f) return INFINITY;
-  const float f = __fdiv_rn(1.0f, det);
+  const float ad = fabsf(det);
+  if (ad < 1e-8f) return INFINITY;
+  // Nearly every triangle tested is missed, most of them clearly: u and v
+  // against |det| with margins far above the rounding of f and the products,
+  // before the divide and the FP64 comparisons that decide the rest.  (An
+  // overflow to inf or NaN passes no rejection that the exact test would not
+  // make.)
   const V3 s = vsub(ro, t.a);
-  const double u = __dmul_rn((double)f, (double)vdot(s, h));
-  if (u < -eps_edge || u > 1.0 + eps_edge) return INFINITY;
+  const float su = vdot(s, h);
+  const float au = det < 0.f ? -su : su;
+  if (au < -1e-5f * ad || au > 1.00001f * ad) return INFINITY;
   const V3 q = vcross(s, e1);
-  const double v = __dmul_rn((double)f, (double)vdot(rd, q));
+  const float sv = vdot(rd, q);
+  const float av = det < 0.f ? -sv : sv;
+  if (av < -1e-5f * ad || av > 1.00001f * ad) return INFINITY;
+  const float f = __fdiv_rn(1.0f, det);
+  const double u = __dmul_rn((double)f, (double)su);
+  if (u < -eps_edge || u > 1.0 + eps_edge) return INFINITY;
+  const double v = __dmul_rn((double)f, (double)sv);
   if (v < -eps_edge || __dadd_rn(u, v) > 1.0 + eps_edge) return INFINITY;
   const float tt = __fmul_rn(f, vdot(e2, q));
   return tt > 1e-8f ? tt : INFINITY;
@@ -121,7 +130,9 @@ __device__ __forceinline__ Ray make_ray(V3 o, V3 d) {
 __device__ __forceinline__ void child_entries(const WideNode* __restrict__ nodes, uint32_t ref, const Ray& r,
                                               float* tc, uint32_t* rc) {
   const int4* np = reinterpret_cast<const int4*>(nodes + ref);
-  const int4 w0 = __ldg(np), w1 = __ldg(np + 1), w2 = __ldg(np + 2), w3 = __ldg(np + 3);
+  int4 w0, w1, w2, w3;
+  ldg256(np, w0, w1);
+  ldg256(np + 2, w2, w3);
   const float ox = __int_as_float(w0.x), oy = __int_as_float(w0.y), oz = __int_as_float(w0.z);
   const uint32_t meta = (uint32_t)w0.w;
   const float sx = __uint_as_float((meta & 0xffu) << 23);
@@ -161,20 +172,6 @@ __device__ __forceinline__ void cswap(float& ta, uint32_t& ra, float& tb, uint32
     rb = x;
   }
 }
-
-struct SharedStack {
-  uint2* base;
-  int sp;
-  static constexpr int kDepth = kRayShared;
-  __device__ __forceinline__ void push(uint32_t ref, float t) {
-    base[sp * kRayThreads] = make_uint2(ref, __float_as_uint(t));
-    ++sp;
-  }
-  __device__ __forceinline__ uint2 pop() {
-    --sp;
-    return base[sp * kRayThreads];
-  }
-};
 
 struct LocalStack {
   uint2 s[kRayDeep];
@@ -247,17 +244,217 @@ struct RayOut {
   float* uvw;
 };
 
-__device__ void write_nearest(const TriRec* __restrict__ tris, const float* __restrict__ face_normals, const Ray& r,
-                              int64_t i, float mint, uint32_t best, const RayOut& out) {
+// The nearest-hit traversal: one ray a lane, persistent warps that hand new
+// rays to lanes as they finish.  A warp alternates node steps, while at least
+// kNodeLanes of its rays are at an inner node, with one leaf step in which the
+// triangles of all rays at a leaf are spread evenly over the lanes.  The order
+// of each ray's visits is that of nearest().  Writes each ray's t and, for
+// ray_finish_kernel, the triangle's record in place of the face.
+// Bound by its instructions: with a ray a thread from start to end, node and
+// leaf in one loop and the divide and FP64 comparisons on every triangle, 7 of
+// 32 lanes were active and 4.2M rays (half a camera's, half scattered) took
+// 2.00 ms; now 0.96.
+constexpr int kRayWarps = kRayThreads / 32;
+// rays at a node below which a warp turns to its leaves, resident blocks an SM,
+// most rays a warp takes at a time (4.2M rays, 1.31M triangles: 1066, 1024,
+// 1008 and 1010 us at 12, 16, 20 and 24 lanes; pools of 128 / 64 / 32: 1012 /
+// 961 / 966 us at 8 blocks)
+constexpr int kNodeLanes = 20;
+constexpr int kRayBlocks = 8;
+constexpr int kParityBlocks = 7;
+constexpr int64_t kRayPool = 64;
+constexpr int kTriRow = 33;  // results at position-in-leaf * 33 + owner: distinct banks
+constexpr uint32_t kNoItem = 0xffffffffu;  // no node or leaf; no reference has this value
+
+struct RaySmem {
+  uint2 stack[kRayShared][32];
+  uint2 own[32];  // a leaf step's rays in lane order: first triangle less its first task, lane | first task << 8
+  float trid[kMaxLeafTris * kTriRow];
+};
+
+__global__ void __launch_bounds__(kRayThreads, kRayBlocks)
+    ray_nearest_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
+                       const float* __restrict__ ro, const float* __restrict__ rd, uint32_t n, float max_t,
+                       float* __restrict__ t_out, int32_t* __restrict__ tri_out, uint32_t* __restrict__ rerun,
+                       uint32_t* __restrict__ nrerun, uint32_t* __restrict__ pool_counter, uint32_t pool) {
+  pdl_wait();
+  __shared__ RaySmem smem[kRayWarps];
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  RaySmem& S = smem[threadIdx.x >> 5];
+  uint32_t pos = 0, end = 0;
+  bool exhausted = false;
+  bool live = false;
+  uint32_t i = 0, ref = kNoItem, best = 0xffffffffu;
+  float mint = max_t;
+  int sp = 0;
+  Ray r{};
+
+  auto distribute = [&](unsigned want) {
+    while (want) {
+      if (pos >= end) {
+        if (exhausted) break;
+        uint32_t p = 0;
+        if (lane == 0) p = atomicAdd(pool_counter, 1u);
+        p = __shfl_sync(FULL, p, 0);
+        const uint64_t first = (uint64_t)p * pool;
+        if (first >= n) { exhausted = true; break; }
+        pos = (uint32_t)first;
+        end = n - pos < pool ? n : pos + pool;
+      }
+      const uint32_t avail = end - pos, cnt = __popc(want);
+      const uint32_t take = avail < cnt ? avail : cnt;
+      const uint32_t rank = __popc(want & ((1u << lane) - 1u));
+      const bool mine = ((want >> lane) & 1u) && rank < take;
+      if (mine) {
+        i = pos + rank;
+        r = make_ray(ld3(ro, i), ld3(rd, i));
+        mint = max_t;
+        best = 0xffffffffu;
+        sp = 0;
+        ref = 0u;
+        live = true;
+      }
+      pos += take;
+      want &= ~__ballot_sync(FULL, mine);
+    }
+  };
+  auto pop = [&]() {
+    ref = kNoItem;
+    while (sp > 0) {
+      --sp;
+      const uint2 e = S.stack[sp][lane];
+      if (__uint_as_float(e.y) <= mint * kPruneSlack) {
+        ref = e.x;
+        break;
+      }
+    }
+  };
+
+  distribute(FULL);
+  while (__any_sync(FULL, live)) {
+    // (a) node steps
+    for (;;) {
+      const unsigned at_node = __ballot_sync(FULL, (int)ref >= 0);
+      if (__popc(at_node) < kNodeLanes &&
+          (at_node == 0u || __any_sync(FULL, live && (int)ref < 0)))
+        break;
+      if ((int)ref >= 0) {
+        float tc[4];
+        uint32_t rc[4];
+        child_entries(nodes, ref, r, tc, rc);
+        cswap(tc[0], rc[0], tc[1], rc[1]);
+        cswap(tc[2], rc[2], tc[3], rc[3]);
+        cswap(tc[0], rc[0], tc[2], rc[2]);
+        cswap(tc[1], rc[1], tc[3], rc[3]);
+        cswap(tc[1], rc[1], tc[2], rc[2]);
+        const float lim = mint * kPruneSlack;
+        int q = 0;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) q += tc[c] <= lim ? 1 : 0;
+        if (q == 0) {
+          pop();
+        } else if (sp + (q - 1) > kRayShared) {
+          rerun[atomicAdd(nrerun, 1u)] = i;  // no room: re-run with a deep stack
+          live = false;
+          ref = kNoItem;
+        } else {
+#pragma unroll
+          for (int c = 3; c >= 1; --c)
+            if (c < q) S.stack[sp++][lane] = make_uint2(rc[c], __float_as_uint(tc[c]));
+          ref = rc[0];
+        }
+      }
+    }
+    // (b) leaf step
+    const uint32_t cnt = live && (int)ref < 0 && ref != kNoItem ? leaf_count(ref) : 0u;
+    const unsigned owners = __ballot_sync(FULL, cnt > 0u);
+    if (owners) {
+      const unsigned lt = (1u << lane) - 1u;
+      uint32_t off = 0, total = 0;  // first task of this lane, tasks in all
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const unsigned m = __ballot_sync(FULL, (cnt >> b) & 1u);
+        off += (uint32_t)__popc(m & lt) << b;
+        total += (uint32_t)__popc(m) << b;
+      }
+      if (cnt > 0u) S.own[__popc(owners & lt)] = make_uint2(leaf_first(ref) - off, (uint32_t)lane | (off << 8));
+      __syncwarp();
+      int before = -1;  // owners whose first task lies before this group of 32
+      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const unsigned firsts = __reduce_or_sync(FULL, cnt > 0u && (off >> 5) == (t0 >> 5) ? 1u << (off & 31u) : 0u);
+        const uint2 w = S.own[before + __popc(firsts & (0xffffffffu >> (31 - lane)))];
+        before += __popc(firsts);
+        const int o = (int)(w.y & 31u);
+        const V3 qo{__shfl_sync(FULL, r.o.x, o), __shfl_sync(FULL, r.o.y, o), __shfl_sync(FULL, r.o.z, o)};
+        const V3 qd{__shfl_sync(FULL, r.d.x, o), __shfl_sync(FULL, r.d.y, o), __shfl_sync(FULL, r.d.z, o)};
+        const uint32_t t = t0 + (uint32_t)lane;
+        if (t < total) S.trid[(t - (w.y >> 8)) * kTriRow + o] = ray_tri(load_tri(tris, w.x + t), qo, qd);
+      }
+      __syncwarp();
+      if (cnt > 0u) {
+        const uint32_t f0 = leaf_first(ref);
+        for (uint32_t k = 0; k < cnt; ++k) {
+          const float t = S.trid[k * kTriRow + lane];
+          if (t < mint) {
+            mint = t;
+            best = f0 + k;
+          }
+        }
+        pop();
+      }
+      __syncwarp();
+    }
+    // (c) finished rays, new ones
+    const bool done = live && ref == kNoItem;
+    if (done) {
+      t_out[i] = mint;
+      tri_out[i] = (int32_t)best;
+      live = false;
+    }
+    const unsigned free_lanes = __ballot_sync(FULL, !live);
+    if (!exhausted || pos < end) distribute(free_lanes);
+  }
+}
+
+__global__ void __launch_bounds__(64)
+    ray_nearest_rerun_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
+                             const float* __restrict__ ro, const float* __restrict__ rd, float max_t,
+                             float* __restrict__ t_out, int32_t* __restrict__ tri_out,
+                             const uint32_t* __restrict__ rerun, const uint32_t* __restrict__ nrerun,
+                             uint32_t* __restrict__ overflow) {
+  pdl_wait();
+  const uint32_t m = *nrerun;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = rerun[k];
+    const Ray r = make_ray(ld3(ro, i), ld3(rd, i));
+    float mint = max_t;
+    uint32_t best = 0xffffffffu;
+    LocalStack st;
+    st.sp = 0;
+    if (!nearest(nodes, tris, r, mint, best, st)) atomicExch(overflow, 1u);
+    t_out[i] = mint;
+    tri_out[i] = (int32_t)best;
+  }
+}
+
+// The remaining outputs of each ray; out.t holds t and out.face the triangle
+// record on entry.
+__global__ void __launch_bounds__(256)
+    ray_finish_kernel(const TriRec* __restrict__ tris, const float* __restrict__ face_normals,
+                      const float* __restrict__ ro, const float* __restrict__ rd, int64_t n, RayOut out) {
+  pdl_wait();
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t best = (uint32_t)out.face[i];
   const bool hit = best != 0xffffffffu;
   out.hit[i] = hit ? 1 : 0;
-  out.t[i] = mint;
   V3 p{0.f, 0.f, 0.f}, nrm{0.f, 0.f, 0.f}, bc{0.f, 0.f, 0.f};
   int32_t face = -1;
   if (hit) {
     const Tri t = load_tri(tris, best);
     face = t.face;
-    p = vpoint(r.o, r.d, mint);
+    p = vpoint(ld3(ro, i), ld3(rd, i), out.t[i]);
     if (out.uvw) bc = tri_bary(t, p, true);
     if (face_normals) nrm = ld3(face_normals, face);
   }
@@ -276,46 +473,6 @@ __device__ void write_nearest(const TriRec* __restrict__ tris, const float* __re
     out.uvw[3 * i] = bc.x;
     out.uvw[3 * i + 1] = bc.y;
     out.uvw[3 * i + 2] = bc.z;
-  }
-}
-
-__global__ void __launch_bounds__(kRayThreads, kRayBlocksPerSm)
-    ray_nearest_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
-                       const float* __restrict__ face_normals, const float* __restrict__ ro,
-                       const float* __restrict__ rd, int64_t n, float max_t, RayOut out, uint32_t* __restrict__ rerun,
-                       uint32_t* __restrict__ nrerun) {
-  pdl_wait();
-  __shared__ uint2 s_stack[kRayShared * kRayThreads];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const Ray r = make_ray(ld3(ro, i), ld3(rd, i));
-  float mint = max_t;
-  uint32_t best = 0xffffffffu;
-  SharedStack st{s_stack + threadIdx.x, 0};
-  if (!nearest(nodes, tris, r, mint, best, st)) {
-    rerun[atomicAdd(nrerun, 1u)] = (uint32_t)i;
-    return;
-  }
-  write_nearest(tris, face_normals, r, i, mint, best, out);
-}
-
-__global__ void __launch_bounds__(64)
-    ray_nearest_rerun_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
-                             const float* __restrict__ face_normals, const float* __restrict__ ro,
-                             const float* __restrict__ rd, float max_t, RayOut out,
-                             const uint32_t* __restrict__ rerun, const uint32_t* __restrict__ nrerun,
-                             uint32_t* __restrict__ overflow) {
-  pdl_wait();
-  const uint32_t m = *nrerun;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = rerun[k];
-    const Ray r = make_ray(ld3(ro, i), ld3(rd, i));
-    float mint = max_t;
-    uint32_t best = 0xffffffffu;
-    LocalStack st;
-    st.sp = 0;
-    if (!nearest(nodes, tris, r, mint, best, st)) atomicExch(overflow, 1u);
-    write_nearest(tris, face_normals, r, i, mint, best, out);
   }
 }
 
@@ -410,61 +567,239 @@ __global__ void ray_all_collect_kernel(const WideNode* __restrict__ nodes, const
   });
 }
 
-// Per point: for each direction, the signed crossing count of the ray with
-// near-coincident hits (|dt| < coalesce, after sorting by t) merged -- a
-// group whose hits all share a sign counts as one crossing of that sign, a
-// mixed group as (|sum| mod 2) * sign(sum) -- and a vote when it is odd.
-__global__ void __launch_bounds__(64)
-    ray_parity_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
-                      const float* __restrict__ pts, int64_t n, const float* __restrict__ dirs, int ndir, float max_t,
-                      float coalesce, int32_t* __restrict__ votes, uint32_t* __restrict__ overflow) {
-  pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const V3 o = ld3(pts, i);
+// Signed crossing count of a ray from its k hits, sorted by t (sign: the hit's
+// side): near-coincident hits (|dt| < coalesce) are merged -- a group whose
+// hits all share a sign counts as one crossing of that sign, a mixed group as
+// (|sum| mod 2) * sign(sum) -- and the ray votes when the count is odd.
+template <typename Hit>
+__device__ __forceinline__ int parity_vote(int k, float coalesce, Hit hit) {
+  int32_t sc = 0;
+  int a = 0;
+  while (a < k) {
+    int b = a + 1;
+    float tb;
+    int sg;
+    hit(a, tb, sg);
+    int32_t cnt = 1, sum = sg;
+    while (b < k) {
+      float t;
+      hit(b, t, sg);
+      if (!(fabsf(__fsub_rn(t, tb)) < coalesce)) break;
+      ++cnt;
+      sum += sg;
+      tb = t;
+      ++b;
+    }
+    const int32_t sgn = sum > 0 ? 1 : (sum < 0 ? -1 : 0);
+    const int32_t asum = sum < 0 ? -sum : sum;
+    sc += asum == cnt ? sgn : (asum % 2) * sgn;
+    a = b;
+  }
+  return ((sc < 0 ? -sc : sc) % 2) == 1 ? 1 : 0;
+}
+
+// one ray with deep local buffers, for the rays that outgrow the shared ones
+__device__ __noinline__ int parity_slow(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris, V3 o,
+                                        V3 d, float max_t, float coalesce, uint32_t* __restrict__ overflow) {
   float ts[kParityCap];
   int8_t sg[kParityCap];
-  int32_t vote = 0;
-  for (int d = 0; d < ndir; ++d) {
-    const Ray r = make_ray(o, ld3(dirs, d));
-    int k = 0;
-    bool lost = false;
-    if (!all_hits(nodes, tris, r, max_t, [&](float th, const Tri&, int s) {
-          // insertion by t keeps the buffer sorted (stable for equal t)
-          if (k >= kParityCap) {
-            lost = true;
-            return;
+  const Ray r = make_ray(o, d);
+  int k = 0;
+  bool lost = false;
+  if (!all_hits(nodes, tris, r, max_t, [&](float th, const Tri&, int s) {
+        // insertion by t keeps the buffer sorted
+        if (k >= kParityCap) {
+          lost = true;
+          return;
+        }
+        int j = k;
+        while (j > 0 && ts[j - 1] > th) {
+          ts[j] = ts[j - 1];
+          sg[j] = sg[j - 1];
+          --j;
+        }
+        ts[j] = th;
+        sg[j] = (int8_t)s;
+        ++k;
+      }))
+    lost = true;
+  if (lost) atomicExch(overflow, 1u);
+  return parity_vote(k, coalesce, [&](int j, float& t, int& s) {
+    t = ts[j];
+    s = sg[j];
+  });
+}
+
+// One (direction, point) ray a lane, directions outermost so that a warp's rays
+// are parallel; phases as in ray_nearest_kernel, visits in any order.  A ray's
+// hits (t, the sign bit for hits from the front) and stack stay in shared
+// memory; one that outgrows either is done again by parity_slow.  votes[i]
+// (zeroed before) counts the point's odd rays.  100,000 points, 8 directions,
+// 200,000 triangles: 1.38 ms with a thread per point and its directions in
+// turn, 0.55 ms so.
+constexpr int kParityHits = 12;
+constexpr int kParityStack = 24;
+
+struct ParitySmem {
+  uint32_t stack[kParityStack][32];
+  float hits[kParityHits][32];
+  uint2 own[32];
+  float trid[kMaxLeafTris * kTriRow];
+};
+
+__global__ void __launch_bounds__(kRayThreads, kParityBlocks)
+    ray_parity_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
+                      const float* __restrict__ pts, int64_t n, const float* __restrict__ dirs, int ndir, float max_t,
+                      float coalesce, int32_t* __restrict__ votes, uint32_t* __restrict__ overflow,
+                      unsigned long long* __restrict__ pool_counter, int64_t pool) {
+  pdl_wait();
+  __shared__ ParitySmem smem[kRayWarps];
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  ParitySmem& S = smem[threadIdx.x >> 5];
+  const int64_t rays = n * ndir;
+  const float lim = max_t * kPruneSlack;
+  int64_t pos = 0, end = 0;
+  bool exhausted = false, live = false, slow = false;
+  int64_t i = 0;
+  int dir = 0, sp = 0, nh = 0;
+  uint32_t ref = kNoItem;
+  Ray r{};
+
+  auto distribute = [&](unsigned want) {
+    while (want) {
+      if (pos >= end) {
+        if (exhausted) break;
+        unsigned long long p = 0;
+        if (lane == 0) p = atomicAdd(pool_counter, 1ull);
+        p = __shfl_sync(FULL, p, 0);
+        if (p >= (unsigned long long)ceil_div(rays, pool)) { exhausted = true; break; }
+        pos = (int64_t)p * pool;
+        end = rays - pos < pool ? rays : pos + pool;
+      }
+      const int64_t avail = end - pos;
+      const int cnt = __popc(want);
+      const int take = (int)(avail < cnt ? avail : cnt);
+      const int rank = __popc(want & ((1u << lane) - 1u));
+      const bool mine = ((want >> lane) & 1u) && rank < take;
+      if (mine) {
+        const int64_t j = pos + rank;
+        dir = (int)(j / n);
+        i = j - dir * n;
+        r = make_ray(ld3(pts, i), ld3(dirs, dir));
+        sp = 0;
+        nh = 0;
+        slow = false;
+        ref = 0u;
+        live = true;
+      }
+      pos += take;
+      want &= ~__ballot_sync(FULL, mine);
+    }
+  };
+
+  distribute(FULL);
+  while (__any_sync(FULL, live)) {
+    // (a) node steps
+    for (;;) {
+      const unsigned at_node = __ballot_sync(FULL, (int)ref >= 0);
+      if (__popc(at_node) < kNodeLanes && (at_node == 0u || __any_sync(FULL, live && (int)ref < 0))) break;
+      if ((int)ref >= 0) {
+        float tc[4];
+        uint32_t rc[4];
+        child_entries(nodes, ref, r, tc, rc);
+        uint32_t next = kNoItem;
+#pragma unroll
+        for (int c = 3; c >= 0; --c)
+          if (tc[c] <= lim) {
+            if (next != kNoItem) {
+              if (sp < kParityStack) S.stack[sp++][lane] = next;
+              else slow = true;
+            }
+            next = rc[c];
           }
+        if (next == kNoItem && sp > 0) next = S.stack[--sp][lane];
+        ref = slow ? kNoItem : next;
+      }
+    }
+    // (b) leaf step
+    const uint32_t cnt = live && (int)ref < 0 && ref != kNoItem ? leaf_count(ref) : 0u;
+    const unsigned owners = __ballot_sync(FULL, cnt > 0u);
+    if (owners) {
+      const unsigned lt = (1u << lane) - 1u;
+      uint32_t off = 0, total = 0;  // first task of this lane, tasks in all
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const unsigned m = __ballot_sync(FULL, (cnt >> b) & 1u);
+        off += (uint32_t)__popc(m & lt) << b;
+        total += (uint32_t)__popc(m) << b;
+      }
+      if (cnt > 0u) S.own[__popc(owners & lt)] = make_uint2(leaf_first(ref) - off, (uint32_t)lane | (off << 8));
+      __syncwarp();
+      int before = -1;  // owners whose first task lies before this group of 32
+      for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const unsigned firsts = __reduce_or_sync(FULL, cnt > 0u && (off >> 5) == (t0 >> 5) ? 1u << (off & 31u) : 0u);
+        const uint2 w = S.own[before + __popc(firsts & (0xffffffffu >> (31 - lane)))];
+        before += __popc(firsts);
+        const int o = (int)(w.y & 31u);
+        const V3 qo{__shfl_sync(FULL, r.o.x, o), __shfl_sync(FULL, r.o.y, o), __shfl_sync(FULL, r.o.z, o)};
+        const V3 qd{__shfl_sync(FULL, r.d.x, o), __shfl_sync(FULL, r.d.y, o), __shfl_sync(FULL, r.d.z, o)};
+        const uint32_t t = t0 + (uint32_t)lane;
+        if (t < total) {
+          const Tri tr = load_tri(tris, w.x + t);
+          float th = ray_tri(tr, qo, qd);
+          if (th > 0.0f && th < max_t) {
+            const float ndotd = vdot(tri_normal(tr), qd);
+            if (ndotd > -1e-4f && ndotd < 1e-4f) th = INFINITY;  // grazing
+            else if (!(ndotd > 0.0f)) th = -th;
+          } else {
+            th = INFINITY;
+          }
+          S.trid[(t - (w.y >> 8)) * kTriRow + o] = th;
+        }
+      }
+      __syncwarp();
+      if (cnt > 0u) {
+        for (uint32_t k = 0; k < cnt; ++k) {
+          const float t = S.trid[k * kTriRow + lane];
+          if (t < INFINITY) {
+            if (nh < kParityHits) S.hits[nh++][lane] = t;
+            else slow = true;
+          }
+        }
+        ref = !slow && sp > 0 ? S.stack[--sp][lane] : kNoItem;
+      }
+      __syncwarp();
+    }
+    // (c) finished rays vote, new ones
+    if (live && ref == kNoItem) {
+      int vote;
+      if (slow) {
+        vote = parity_slow(nodes, tris, r.o, r.d, max_t, coalesce, overflow);
+      } else {
+        // insertion sort by t
+        for (int k = 1; k < nh; ++k) {
+          const float t = S.hits[k][lane];
           int j = k;
-          while (j > 0 && ts[j - 1] > th) {
-            ts[j] = ts[j - 1];
-            sg[j] = sg[j - 1];
+          while (j > 0 && fabsf(S.hits[j - 1][lane]) > fabsf(t)) {
+            S.hits[j][lane] = S.hits[j - 1][lane];
             --j;
           }
-          ts[j] = th;
-          sg[j] = (int8_t)s;
-          ++k;
-        }))
-      lost = true;
-    if (lost) atomicExch(overflow, 1u);
-    int32_t sc = 0;
-    int a = 0;
-    while (a < k) {
-      int b = a + 1;
-      int32_t cnt = 1, sum = sg[a];
-      while (b < k && fabsf(__fsub_rn(ts[b], ts[b - 1])) < coalesce) {
-        ++cnt;
-        sum += sg[b];
-        ++b;
+          S.hits[j][lane] = t;
+        }
+        vote = parity_vote(nh, coalesce, [&](int j, float& t, int& sg) {
+          const float h = S.hits[j][lane];
+          t = fabsf(h);
+          sg = h < 0.f ? -1 : 1;
+        });
       }
-      const int32_t sgn = sum > 0 ? 1 : (sum < 0 ? -1 : 0);
-      const int32_t asum = sum < 0 ? -sum : sum;
-      sc += asum == cnt ? sgn : (asum % 2) * sgn;
-      a = b;
+      if (vote) atomicAdd(&votes[i], 1);
+      live = false;
+      slow = false;
     }
-    vote += ((sc < 0 ? -sc : sc) % 2) == 1 ? 1 : 0;
+    const unsigned free_lanes = __ballot_sync(FULL, !live);
+    if (!exhausted || pos < end) distribute(free_lanes);
   }
-  votes[i] = vote;
 }
 
 }  // namespace
@@ -483,8 +818,34 @@ extern "C" size_t a3d_ray_workspace_bytes(int64_t num_rays) {
 }
 
 namespace {
+// resident blocks of a persistent kernel, queried once per device; slot: one
+// per kernel
+template <typename Kernel>
+int blocks_per_sm(Kernel kernel, int* out, int slot) {
+  static int cached[2][kMaxDevices] = {};
+  int dev = 0;
+  A3D_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev >= 0 && dev < kMaxDevices && cached[slot][dev] > 0) {
+    *out = cached[slot][dev];
+    return A3D_OK;
+  }
+  int b = 0;
+  A3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kRayThreads, 0));
+  b = b < 1 ? 1 : b;
+  if (dev >= 0 && dev < kMaxDevices) cached[slot][dev] = b;
+  *out = b;
+  return A3D_OK;
+}
+
+// rays a warp takes at a time: 32 while that is under four pools a warp, at
+// most kRayPool
+int64_t ray_pool(int64_t rays, int64_t warps) {
+  const int64_t pool = rays / (warps * 4) / 32 * 32;
+  return pool < 32 ? 32 : (pool > kRayPool ? kRayPool : pool);
+}
+
 struct RayWs {
-  uint32_t* status;  // [0] re-run count, [1] stack / buffer overflow
+  uint32_t* status;  // [0] re-run count, [1] stack / buffer overflow, [2] pools taken
   uint32_t* rerun;
   int32_t* counts;
   int64_t* scan_tmp;
@@ -516,10 +877,17 @@ extern "C" int a3d_ray_nearest(const a3d_bvh_view* bvh, const float* rays_o, con
   const WideNode* nodes = (const WideNode*)bvh->nodes;
   const TriRec* tris = (const TriRec*)bvh->tris;
   const RayOut out{hit, t, face_ids, hit_points, normals, uvw};
-  A3D_PDL(ray_nearest_kernel, dim3((unsigned)ceil_div(num_rays, kRayThreads)), dim3(kRayThreads), 0, s, nodes, tris,
-          face_normals, rays_o, rays_d, num_rays, max_t, out, w.rerun, w.status);
-  A3D_PDL(ray_nearest_rerun_kernel, dim3(num_sms() * 4), dim3(64), 0, s, nodes, tris, face_normals, rays_o, rays_d,
-          max_t, out, w.rerun, w.status, w.status + 1);
+  int bps = 0;
+  A3D_TRY(blocks_per_sm(ray_nearest_kernel, &bps, 0));
+  const int64_t warps = (int64_t)num_sms() * bps * kRayWarps;
+  const int64_t pool = ray_pool(num_rays, warps);
+  const int64_t want = ceil_div(ceil_div(num_rays, pool), kRayWarps), cap = warps / kRayWarps;
+  A3D_PDL(ray_nearest_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(kRayThreads), 0, s, nodes, tris, rays_o,
+          rays_d, (uint32_t)num_rays, max_t, t, face_ids, w.rerun, w.status, w.status + 2, (uint32_t)pool);
+  A3D_PDL(ray_nearest_rerun_kernel, dim3(num_sms() * 4), dim3(64), 0, s, nodes, tris, rays_o, rays_d, max_t, t,
+          face_ids, w.rerun, w.status, w.status + 1);
+  A3D_PDL(ray_finish_kernel, dim3((unsigned)ceil_div(num_rays, 256)), dim3(256), 0, s, tris, face_normals, rays_o,
+          rays_d, num_rays, out);
   return A3D_OK;
 }
 
@@ -568,8 +936,15 @@ extern "C" int a3d_ray_parity_votes(const a3d_bvh_view* bvh, const float* points
   A3D_CUDA_TRY(cudaMemsetAsync(w.status, 0, 4 * sizeof(uint32_t), s));
   if (num_points == 0) return A3D_OK;
   A3D_REQUIRE(points && dirs && votes, A3D_ERR_ARGUMENT, "ray_parity: null pointer");
-  A3D_PDL(ray_parity_kernel, dim3((unsigned)ceil_div(num_points, 64)), dim3(64), 0, s, (const WideNode*)bvh->nodes,
-          (const TriRec*)bvh->tris, points, num_points, dirs, num_dirs, max_t, coalesce_t, votes, w.status + 1);
+  A3D_CUDA_TRY(cudaMemsetAsync(votes, 0, (size_t)num_points * sizeof(int32_t), s));
+  int bps = 0;
+  A3D_TRY(blocks_per_sm(ray_parity_kernel, &bps, 1));
+  const int64_t rays = num_points * num_dirs, warps = (int64_t)num_sms() * bps * kRayWarps;
+  const int64_t pool = ray_pool(rays, warps);
+  const int64_t want = ceil_div(ceil_div(rays, pool), kRayWarps), cap = warps / kRayWarps;
+  A3D_PDL(ray_parity_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(kRayThreads), 0, s,
+          (const WideNode*)bvh->nodes, (const TriRec*)bvh->tris, points, num_points, dirs, num_dirs, max_t, coalesce_t,
+          votes, w.status + 1, reinterpret_cast<unsigned long long*>(w.status + 2), pool);
   return A3D_OK;
 }
 
