@@ -17,12 +17,13 @@
 //     order, so extraction in word order is the reference's lexicographic
 //     (x, y, z) nonzero order;
 //   * W grows by monotone relaxation over 32x32-row bricks: a CTA loads its
-//     brick and a one-row halo into shared memory and iterates (dilate in
-//     x/y, flood whole free runs along z with a Kogge-Stone prefix) until
-//     the brick is stable, then marks its neighbours dirty if it changed.
+//     brick and a one-row halo into shared memory, takes what flows in, and
+//     fills whole free runs along z, y and x (Kogge-Stone prefixes) until the
+//     brick is stable, then queues the neighbours its changes can reach.
 //     Bits only ever get set, so reading a neighbour's word while it is
 //     being updated is safe; rounds repeat until no brick is dirty;
-//   * labels and the k-ring dilation are word-parallel passes; one pass
+//   * labels and the k-ring dilation are word-parallel passes over runs of
+//     rows (the last ring decides its labels itself); one pass
 //     counts every label per tile of kTileWords words (and in total), and a
 //     label's coordinates are written by one block per tile after a scan of
 //     that label's tile counts (words are ranked inside the tile).
@@ -149,89 +150,185 @@ __global__ void set_bits_kernel(const int64_t* __restrict__ ijk, int64_t n, Geom
   atomicOr(&vol[widx(g, x, y, z >> 5)], 1u << (z & 31));
 }
 
+// all free bits connected to a bit of r along the lanes' axis, for 32 columns
+// (bits) at a time: r a subset of f.  A lane without a partner reads its own
+// word, which adds nothing.
+__device__ __forceinline__ uint32_t fill_lanes(uint32_t r, uint32_t f) {
+  uint32_t u = r, m = f;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    u |= __shfl_up_sync(0xffffffffu, u, d) & m;
+    m &= __shfl_up_sync(0xffffffffu, m, d);
+  }
+  m = f;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    u |= __shfl_down_sync(0xffffffffu, u, d) & m;
+    m &= __shfl_down_sync(0xffffffffu, m, d);
+  }
+  return u;
+}
+
+struct BrickSmem {
+  uint32_t r[3][kBX + 2][kBY + 2];  // water words w-1, w, w+1 of the rows with halo, as loaded
+  uint32_t t[kBX][kBY + 1];         // the brick's words while they change
+  uint32_t queue[2];                // neighbour bricks to queue, of this visit and the one before
+};
+
+// bits that a change c in a row may set in a row l1 steps (x and y) away, word
+// for word
+__device__ __forceinline__ uint32_t spread(uint32_t c, int l1, int conn) {
+  if (l1 == 2 && conn == 6) return 0u;
+  return (l1 == 1 && conn != 6) || (l1 == 2 && conn == 26) ? c | (c << 1) | (c >> 1) : c;
+}
+// whether it reaches the words above and below there
+__device__ __forceinline__ bool spreads_z(int l1, int conn) {
+  return l1 == 0 || conn == 26 || (conn == 18 && l1 == 1);
+}
+
 // One relaxation round over the bricks queued for it: list `cur` with
-// cnt[round % 3] entries, which the blocks stride over.  A brick whose water
-// changed queues its 27 neighbours (itself included) for the next round,
-// each once: mark[b] is the last round b was queued for, raised with
-// atomicMax, and the first raiser appends b to `nxt` (count cnt[(round + 1)
-// % 3]).  Block 0 clears cnt[(round + 2) % 3], the input count of the
-// previous round, for the round after this one.  Rounds run back to back
+// cnt[round % 3] entries, which the blocks stride over.  A brick takes the
+// water of its halo once and then fills whole free runs along z (bits), y
+// (lanes) and x (lanes, transposed through shared memory) in turn until nothing
+// changes, so open space takes two or three sweeps and not a step per voxel; a
+// brick without any obstacle is filled at once.  It queues the neighbours in
+// which its changes can set a bit -- those whose voxels beside a change were
+// not water when the halo was read -- and itself if the sweeps were cut short,
+// for the next round, each once: mark[b] is the last round b was queued for,
+// raised with atomicMax, and the first raiser appends b to `nxt` (count
+// cnt[(round + 1) % 3]).  Block 0 clears cnt[(round + 2) % 3], the input count
+// of the previous round, for the round after this one.  Rounds run back to back
 // inside one kernel, so everything another block may have written in an
 // earlier round (queue, counts, water) is read through L2 (ld.global.cg),
 // never from a stale L1 line.
+// Bound by the latency of a visit (its loads, then block barriers) at one brick
+// an SM.  923^3 crop of a 1024^3 grid, 26-connected: 4.26 ms with steps of one
+// voxel and all 27 bricks queued on any change, 1.84 ms with runs and the
+// reached neighbours alone, 1.57 ms with a thread's loads in flight together
+// (43 rounds).  Two bricks an SM (32 registers a thread, spills) took longer.
 __device__ __forceinline__ void relax_round(const Geom& g, const uint32_t* __restrict__ occ, uint32_t* water,
                                             const uint32_t* cur, uint32_t* nxt, uint32_t* __restrict__ mark,
-                                            uint32_t* cnt, int round, int nbx, int nby, int max_iters,
-                                            uint32_t (*s_r)[kBX + 2][kBY + 2]) {
+                                            uint32_t* cnt, int round, int nbx, int nby, int max_iters, BrickSmem& S) {
   const uint32_t nbricks = (uint32_t)nbx * (uint32_t)nby * (uint32_t)g.nw;
   const uint32_t n_cur = min(__ldcg(cnt + round % 3), nbricks);
   if (blockIdx.x == 0 && threadIdx.x == 0) cnt[(round + 2) % 3] = 0u;
   const uint32_t next_round = (uint32_t)round + 1u;
-  for (uint32_t item = blockIdx.x; item < n_cur; item += gridDim.x) {
-    const int bid = (int)__ldcg(cur + item);
+  const int tx = threadIdx.x / kBY, ty = threadIdx.x % kBY;
+  uint32_t next = blockIdx.x < n_cur ? __ldcg(cur + blockIdx.x) : 0u;
+  int turn = 0;
+  for (uint32_t item = blockIdx.x; item < n_cur; item += gridDim.x, turn ^= 1) {
+    const int bid = (int)next;
+    if (item + gridDim.x < n_cur) next = __ldcg(cur + item + gridDim.x);
     const int bw = bid / (nbx * nby);
     const int rem = bid % (nbx * nby);
     const int bxi = rem / nby, byi = rem % nby;
     const int x0 = bxi * kBX, y0 = byi * kBY;
-    const int tx = threadIdx.x / kBY, ty = threadIdx.x % kBY;
-    // load the halo'd water words (monotone: a racing update is harmless)
-    for (int i = threadIdx.x; i < 3 * (kBX + 2) * (kBY + 2); i += blockDim.x) {
-      const int k = i / ((kBX + 2) * (kBY + 2));
-      const int r2 = i % ((kBX + 2) * (kBY + 2));
-      const int hx = r2 / (kBY + 2), hy = r2 % (kBY + 2);
-      const int x = x0 + hx - 1, y = y0 + hy - 1, w = bw + k - 1;
-      uint32_t v = 0;
-      if (x >= 0 && x < g.nx && y >= 0 && y < g.ny && w >= 0 && w < g.nw) v = __ldcg(&water[widx(g, x, y, w)]);
-      s_r[k][hx][hy] = v;
-    }
     const int x = x0 + tx, y = y0 + ty;
-    const bool inside = x < g.nx && y < g.ny;
     uint32_t f = 0;
-    if (inside) f = ~occ[widx(g, x, y, bw)] & crop_mask(g, x, y, bw);
-    __syncthreads();
-    const uint32_t orig = s_r[1][tx + 1][ty + 1];
-    for (int it = 0; it < max_iters; ++it) {
-      uint32_t acc = 0;
-      const uint32_t self = s_r[1][tx + 1][ty + 1];
-      // neighbours along z of this row (words of the adjacent bricks)
-      acc |= (s_r[0][tx + 1][ty + 1] >> 31) | (s_r[2][tx + 1][ty + 1] << 31);
-  #pragma unroll
+    if (x < g.nx && y < g.ny) f = ~occ[widx(g, x, y, bw)] & crop_mask(g, x, y, bw);
+    // load the halo'd water words (monotone: a racing update is harmless), all
+    // of a thread's before the first is stored
+    constexpr int kWords = 3 * (kBX + 2) * (kBY + 2), kLoads = (kWords + kBX * kBY - 1) / (kBX * kBY);
+    uint32_t v[kLoads];
+#pragma unroll
+    for (int l = 0; l < kLoads; ++l) {
+      const int i = threadIdx.x + l * kBX * kBY;
+      const int r2 = i / 3, w = bw + (i - 3 * r2) - 1;  // a row's three words lie side by side
+      const int xx = x0 + r2 / (kBY + 2) - 1, yy = y0 + r2 % (kBY + 2) - 1;
+      v[l] = 0;
+      if (i < kWords && xx >= 0 && xx < g.nx && yy >= 0 && yy < g.ny && w >= 0 && w < g.nw)
+        v[l] = __ldcg(&water[widx(g, xx, yy, w)]);
+    }
+#pragma unroll
+    for (int l = 0; l < kLoads; ++l) {
+      const int i = threadIdx.x + l * kBX * kBY, r2 = i / 3;
+      if (i < kWords) S.r[i - 3 * r2][r2 / (kBY + 2)][r2 % (kBY + 2)] = v[l];
+    }
+    S.t[tx][ty] = f;
+    if (threadIdx.x == 0) S.queue[turn] = 0u;
+    const bool open = __syncthreads_and(f == 0xffffffffu);
+    const uint32_t orig = S.r[1][tx + 1][ty + 1];
+    const uint32_t ft = S.t[ty][tx];  // the free bits of row (ty, tx): lanes along x
+    uint32_t acc = (S.r[0][tx + 1][ty + 1] >> 31) | (S.r[2][tx + 1][ty + 1] << 31);
+#pragma unroll
+    for (int dx = -1; dx <= 1; ++dx) {
+#pragma unroll
+      for (int dy = -1; dy <= 1; ++dy) {
+        if (dx == 0 && dy == 0) continue;
+        const int l1 = (dx != 0) + (dy != 0);
+        acc |= spread(S.r[1][tx + 1 + dx][ty + 1 + dy], l1, g.conn);
+        if (spreads_z(l1, g.conn))
+          acc |= (S.r[0][tx + 1 + dx][ty + 1 + dy] >> 31) | (S.r[2][tx + 1 + dx][ty + 1 + dy] << 31);
+      }
+    }
+    uint32_t now = fill_runs(orig | (acc & f), f);
+    if (!__syncthreads_or(now != orig)) continue;  // nothing flows in: water is closed under the runs
+    bool settled = true;
+    if (open) {
+      now = 0xffffffffu;
+    } else {
+      settled = false;
+      for (int it = 0; it < max_iters; ++it) {
+        const uint32_t before = now;
+        now = fill_lanes(fill_runs(now, f), f);
+        S.t[tx][ty] = now;
+        __syncthreads();
+        S.t[ty][tx] = fill_lanes(S.t[ty][tx], ft);
+        __syncthreads();
+        now = S.t[tx][ty];
+        if (g.conn != 6) {  // the diagonals, inside the brick
+          uint32_t d = 0;
+#pragma unroll
+          for (int dx = -1; dx <= 1; ++dx)
+#pragma unroll
+            for (int dy = -1; dy <= 1; ++dy) {
+              if ((dx == 0 && dy == 0) || tx + dx < 0 || tx + dx >= kBX || ty + dy < 0 || ty + dy >= kBY) continue;
+              d |= spread(S.t[tx + dx][ty + dy], (dx != 0) + (dy != 0), g.conn);
+            }
+          now |= d & f;
+        }
+        // also the barrier between these reads of t and the next sweep's writes
+        if (!__syncthreads_or(now != before)) {
+          settled = true;
+          break;
+        }
+      }
+    }
+    // the neighbours that a change reaches
+    const uint32_t ch = now & ~orig;
+    uint32_t q = settled ? 0u : 1u << 13;
+    if (ch) {
+      water[widx(g, x, y, bw)] = now;
+#pragma unroll
       for (int dx = -1; dx <= 1; ++dx) {
-  #pragma unroll
+#pragma unroll
         for (int dy = -1; dy <= 1; ++dy) {
-          if (dx == 0 && dy == 0) continue;
           const int l1 = (dx != 0) + (dy != 0);
-          const uint32_t a = s_r[0][tx + 1 + dx][ty + 1 + dy];
-          const uint32_t c = s_r[1][tx + 1 + dx][ty + 1 + dy];
-          const uint32_t b = s_r[2][tx + 1 + dx][ty + 1 + dy];
-          if (g.conn == 6) {
-            if (l1 == 1) acc |= c;
-          } else if (g.conn == 18) {
-            acc |= (l1 == 1) ? zdil(a, c, b) : c;
-          } else {
-            acc |= zdil(a, c, b);
+          const int ox = tx + dx < 0 ? 0 : tx + dx >= kBX ? 2 : 1, oy = ty + dy < 0 ? 0 : ty + dy >= kBY ? 2 : 1;
+          const uint32_t bit = 1u << (3 * ox + oy);  // of the layer w-1; w and w+1 follow at 9 and 18
+          if ((ox != 1 || oy != 1) &&
+              (spread(ch, l1, g.conn) & ~S.r[1][tx + 1 + dx][ty + 1 + dy] & crop_mask(g, x + dx, y + dy, bw)))
+            q |= bit << 9;
+          if (spreads_z(l1, g.conn)) {
+            if ((ch & 1u) && !(S.r[0][tx + 1 + dx][ty + 1 + dy] >> 31)) q |= bit;
+            if ((ch >> 31) && !(S.r[2][tx + 1 + dx][ty + 1 + dy] & 1u)) q |= bit << 18;
           }
         }
       }
-      const uint32_t nw = inside ? fill_runs(self | (acc & f), f) | self : self;
-      const bool ch = nw != self;
-      if (ch) s_r[1][tx + 1][ty + 1] = nw;
-      if (!__syncthreads_or(ch)) break;
     }
-    const uint32_t fin = s_r[1][tx + 1][ty + 1];
-    if (inside && fin != orig) water[widx(g, x, y, bw)] = fin;
-    // the barrier also ends this brick's reads of s_r before the next item's
+    q = __reduce_or_sync(0xffffffffu, q);
+    if (ty == 0 && q) atomicOr(&S.queue[turn], q);
+    // the barrier also ends this brick's reads of r before the next item's
     // halo load
-    if (__syncthreads_or(inside && fin != orig)) {
-      if (threadIdx.x < 27) {
-        const int dz = threadIdx.x / 9 - 1, dxx = (threadIdx.x / 3) % 3 - 1, dyy = threadIdx.x % 3 - 1;
-        const int nbw = bw + dz, nbxx = bxi + dxx, nbyy = byi + dyy;
-        if (nbw >= 0 && nbw < g.nw && nbxx >= 0 && nbxx < nbx && nbyy >= 0 && nbyy < nby) {
-          const uint32_t nb = (uint32_t)((nbw * nbx + nbxx) * nby + nbyy);
-          if (atomicMax(&mark[nb], next_round) < next_round) {
-            const uint32_t slot = atomicAdd(&cnt[(round + 1) % 3], 1u);
-            if (slot < nbricks) nxt[slot] = nb;
-          }
+    __syncthreads();
+    if (threadIdx.x < 27 && ((S.queue[turn] >> threadIdx.x) & 1u)) {
+      const int dz = threadIdx.x / 9 - 1, dxx = (threadIdx.x / 3) % 3 - 1, dyy = threadIdx.x % 3 - 1;
+      const int nbw = bw + dz, nbxx = bxi + dxx, nbyy = byi + dyy;
+      if (nbw >= 0 && nbw < g.nw && nbxx >= 0 && nbxx < nbx && nbyy >= 0 && nbyy < nby) {
+        const uint32_t nb = (uint32_t)((nbw * nbx + nbxx) * nby + nbyy);
+        if (atomicMax(&mark[nb], next_round) < next_round) {
+          const uint32_t slot = atomicAdd(&cnt[(round + 1) % 3], 1u);
+          if (slot < nbricks) nxt[slot] = nb;
         }
       }
     }
@@ -283,12 +380,12 @@ __global__ void __launch_bounds__(kBX * kBY)
                         uint32_t* __restrict__ mark, uint32_t* cnt, int nbx, int nby, int max_iters, int max_rounds,
                         uint32_t* sync) {
   pdl_wait();
-  __shared__ uint32_t s_r[3][kBX + 2][kBY + 2];  // words w-1, w, w+1 of the rows with halo
+  __shared__ BrickSmem S;
   int round = 0;
   for (;;) {
     const uint32_t* cur = (round & 1) ? list_b : list_a;
     uint32_t* nxt = (round & 1) ? list_a : list_b;
-    relax_round(g, occ, water, cur, nxt, mark, cnt, round, nbx, nby, max_iters, s_r);
+    relax_round(g, occ, water, cur, nxt, mark, cnt, round, nbx, nby, max_iters, S);
     const bool ok = grid_barrier(sync);
     ++round;
     if (!ok) {
@@ -308,86 +405,127 @@ __global__ void __launch_bounds__(kBX * kBY)
 // 4 extended dam 5 extended tide 6 dry adjacent 7 ring (scratch)
 enum { kWater = 0, kDry = 1, kTide = 2, kDam = 3, kExt = 4, kExtTide = 5, kDryAdj = 6, kRing = 7, kLabels = 8 };
 
+// The label and ring passes: a thread takes kRun rows along y of one word
+// column and keeps what the last rows gave, so a word's 3x3x3 neighbourhood
+// costs its three rows' words once (9 loads a word and volume, not 27); lanes
+// lie along w, then along the next run of rows.  20.7M words: labels 883 ->
+// 330 us (896 MB that have to move: 138 us), the ring with its copy and the
+// classification 560 -> 180 us, against a thread a word.
+constexpr int kRun = 16;
+
+struct RunPos {
+  int x, y0, y1, w;  // rows y0 <= y < y1
+};
+__device__ __forceinline__ int64_t runs_of(const Geom& g) {
+  return (int64_t)g.nx * ((g.ny + kRun - 1) / kRun) * g.nw;
+}
+__device__ __forceinline__ RunPos run_pos(const Geom& g, int64_t t) {
+  const int64_t r = t / g.nw;
+  const int runs = (g.ny + kRun - 1) / kRun;
+  RunPos p;
+  p.w = (int)(t - r * g.nw);
+  p.x = (int)(r / runs);
+  p.y0 = (int)(r - (int64_t)p.x * runs) * kRun;
+  p.y1 = p.y0 + kRun < g.ny ? p.y0 + kRun : g.ny;
+  return p;
+}
+
+// Row y of a word column: the word itself and, for the columns x-1, x, x+1,
+// what it adds to the dilation of its own row and of the rows beside it.
+struct RowPart {
+  uint32_t centre, own, beside;
+};
 template <int kConn>
-__device__ __forceinline__ uint32_t dil_conn(const uint32_t* __restrict__ v, const Geom& g, int x, int y, int w) {
-  uint32_t acc = 0;
-  auto word = [&](int xx, int yy, int ww) -> uint32_t {
-    if (xx < 0 || yy < 0 || ww < 0 || xx >= g.nx || yy >= g.ny || ww >= g.nw) return 0u;
-    return v[widx(g, xx, yy, ww)];
-  };
-  const uint32_t c0 = word(x, y, w);
-  acc |= (c0 << 1) | (c0 >> 1) | (word(x, y, w - 1) >> 31) | (word(x, y, w + 1) << 31);
+__device__ __forceinline__ RowPart row_part(const uint32_t* __restrict__ v, const Geom& g, int x, int y, int w) {
+  RowPart p{0u, 0u, 0u};
+  if (y < 0 || y >= g.ny) return p;
 #pragma unroll
-  for (int dx = -1; dx <= 1; ++dx)
-#pragma unroll
-    for (int dy = -1; dy <= 1; ++dy) {
-      if (dx == 0 && dy == 0) continue;
-      const int l1 = (dx != 0) + (dy != 0);
-      if (kConn == 6 && l1 != 1) continue;
-      const uint32_t c = word(x + dx, y + dy, w);
-      if (kConn == 6 || (kConn == 18 && l1 == 2)) {
-        acc |= c;
-      } else {
-        acc |= zdil(word(x + dx, y + dy, w - 1), c, word(x + dx, y + dy, w + 1));
-      }
-    }
-  return acc;
-}
-
-__global__ void labels_kernel(Geom g, const uint32_t* __restrict__ occ, const uint32_t* __restrict__ water,
-                              uint32_t* __restrict__ lab, int64_t nwords) {
-  pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nwords) return;
-  const int w = (int)(i % g.nw);
-  const int64_t row = i / g.nw;
-  const int y = (int)(row % g.ny), x = (int)(row / g.ny);
-  const uint32_t crop = crop_mask(g, x, y, w);
-  const uint32_t o = occ[i] & crop, r = water[i] & crop;
-  uint32_t near_occ, near_w;
-  if (g.conn == 6) {
-    near_occ = dil_conn<6>(occ, g, x, y, w);
-    near_w = dil_conn<6>(water, g, x, y, w);
-  } else if (g.conn == 18) {
-    near_occ = dil_conn<18>(occ, g, x, y, w);
-    near_w = dil_conn<18>(water, g, x, y, w);
-  } else {
-    near_occ = dil_conn<26>(occ, g, x, y, w);
-    near_w = dil_conn<26>(water, g, x, y, w);
+  for (int dx = -1; dx <= 1; ++dx) {
+    if (x + dx < 0 || x + dx >= g.nx) continue;
+    const uint32_t* row = v + widx(g, x + dx, y, 0);
+    const uint32_t c = __ldg(row + w);
+    const bool own_z = kConn != 6 || dx == 0, beside_z = kConn == 26 || (kConn == 18 && dx == 0);
+    uint32_t z = c;
+    if (own_z || beside_z)
+      z = zdil(w > 0 ? __ldg(row + w - 1) : 0u, c, w + 1 < g.nw ? __ldg(row + w + 1) : 0u);
+    if (dx == 0) p.centre = c;
+    p.own |= own_z ? z : c;
+    if (kConn != 6 || dx == 0) p.beside |= beside_z ? z : c;
   }
-  const uint32_t near_w_ext = g.conn == 6 ? near_w : (g.conn == 18 ? dil_conn<26>(water, g, x, y, w) : near_w);
-  const uint32_t tide = r & near_occ;
-  const uint32_t dam0 = o & near_w;
-  const uint32_t ext = o & ~dam0 & near_w_ext;
-  const uint32_t dam = dam0 | ext;
-  const int64_t nwv = nwords;
-  lab[kWater * nwv + i] = r & ~tide;
-  lab[kTide * nwv + i] = tide;
-  lab[kDam * nwv + i] = dam;
-  lab[kExt * nwv + i] = ext;
-  lab[kDry * nwv + i] = crop & ~r & ~dam;
+  return p;
 }
 
-// 3x3x3 box dilation of src into dst (one ring of get_dam_neighborhood_signs)
-__global__ void box_dilate_kernel(Geom g, const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
-                                  int64_t nwords) {
+// The dilations here keep the centre voxel; water and occupied voxels are
+// disjoint, so that changes no label.
+template <int kConn>
+__global__ void __launch_bounds__(256)
+    labels_kernel(Geom g, const uint32_t* __restrict__ occ, const uint32_t* __restrict__ water,
+                  uint32_t* __restrict__ lab, int64_t nwords) {
   pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nwords) return;
-  const int w = (int)(i % g.nw);
-  const int64_t row = i / g.nw;
-  const int y = (int)(row % g.ny), x = (int)(row / g.ny);
-  dst[i] = (src[i] | dil_conn<26>(src, g, x, y, w)) & valid_mask(g, w);
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= runs_of(g)) return;
+  const RunPos p = run_pos(g, t);
+  // the extension takes the 3x3x3 dilation of the water, or the 6-cross for
+  // connectivity 6
+  constexpr int kExtConn = kConn == 18 ? 26 : kConn;
+  RowPart o0 = row_part<kConn>(occ, g, p.x, p.y0 - 1, p.w), o1 = row_part<kConn>(occ, g, p.x, p.y0, p.w);
+  RowPart w0 = row_part<kConn>(water, g, p.x, p.y0 - 1, p.w), w1 = row_part<kConn>(water, g, p.x, p.y0, p.w);
+  RowPart e0{}, e1{};
+  if (kExtConn != kConn) {
+    e0 = row_part<kExtConn>(water, g, p.x, p.y0 - 1, p.w);
+    e1 = row_part<kExtConn>(water, g, p.x, p.y0, p.w);
+  }
+  for (int y = p.y0; y < p.y1; ++y) {
+    const RowPart o2 = row_part<kConn>(occ, g, p.x, y + 1, p.w), w2 = row_part<kConn>(water, g, p.x, y + 1, p.w);
+    RowPart e2{};
+    if (kExtConn != kConn) e2 = row_part<kExtConn>(water, g, p.x, y + 1, p.w);
+    const int64_t i = widx(g, p.x, y, p.w);
+    const uint32_t crop = crop_mask(g, p.x, y, p.w);
+    const uint32_t o = o1.centre & crop, r = w1.centre & crop;
+    const uint32_t near_occ = o0.beside | o1.own | o2.beside, near_w = w0.beside | w1.own | w2.beside;
+    const uint32_t near_w_ext = kExtConn != kConn ? e0.beside | e1.own | e2.beside : near_w;
+    const uint32_t tide = r & near_occ;
+    const uint32_t dam0 = o & near_w;
+    const uint32_t ext = o & ~dam0 & near_w_ext;
+    const uint32_t dam = dam0 | ext;
+    lab[kWater * nwords + i] = r & ~tide;
+    lab[kTide * nwords + i] = tide;
+    lab[kDam * nwords + i] = dam;
+    lab[kExt * nwords + i] = ext;
+    lab[kDry * nwords + i] = crop & ~r & ~dam;
+    o0 = o1; o1 = o2;
+    w0 = w1; w1 = w2;
+    e0 = e1; e1 = e2;
+  }
 }
 
-__global__ void ring_classify_kernel(const uint32_t* __restrict__ ring, uint32_t* __restrict__ lab, int64_t nwords) {
+// 3x3x3 box dilation of src (one ring of get_dam_neighborhood_signs) into dst,
+// or, for the last ring, straight into the labels it decides: extended tide
+// (neither dam nor dry) and dry adjacent.
+template <bool kClassify>
+__global__ void __launch_bounds__(256)
+    box_dilate_kernel(Geom g, const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
+                      uint32_t* __restrict__ lab, int64_t nwords) {
   pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nwords) return;
-  const uint32_t n = ring[i];
-  const uint32_t dam = lab[kDam * nwords + i], dry = lab[kDry * nwords + i];
-  lab[kExtTide * nwords + i] = n & ~dam & ~dry;
-  lab[kDryAdj * nwords + i] = n & dry & ~dam;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= runs_of(g)) return;
+  const RunPos p = run_pos(g, t);
+  const uint32_t valid = valid_mask(g, p.w);
+  uint32_t s0 = row_part<26>(src, g, p.x, p.y0 - 1, p.w).own, s1 = row_part<26>(src, g, p.x, p.y0, p.w).own;
+  for (int y = p.y0; y < p.y1; ++y) {
+    const uint32_t s2 = row_part<26>(src, g, p.x, y + 1, p.w).own;
+    const int64_t i = widx(g, p.x, y, p.w);
+    const uint32_t n = (s0 | s1 | s2) & valid;
+    if (kClassify) {
+      const uint32_t dam = lab[kDam * nwords + i], dry = lab[kDry * nwords + i];
+      lab[kExtTide * nwords + i] = n & ~dam & ~dry;
+      lab[kDryAdj * nwords + i] = n & dry & ~dam;
+    } else {
+      dst[i] = n;
+    }
+    s0 = s1;
+    s1 = s2;
+  }
 }
 
 // A tile is kTileWords consecutive words: 256 threads, each warp owning
@@ -428,12 +566,43 @@ __global__ void __launch_bounds__(kTileThreads) tile_counts_kernel(const uint32_
   }
 }
 
-// One block per tile.  Each lane takes one word per chunk and ranks it in
-// the tile (warp scans of popcounts, then the warps' totals); then, for each
-// non-empty word of a chunk, the 32 lanes take its 32 bits, so the set
-// voxels' coordinates are written as one contiguous run in the word's bit
-// order -- lexicographic (x, y, z) overall.  Positions at or past `count`
-// are not written.  Needs nwords < 2^32 (word coordinates in 32 bits).
+// The 32 len voxels (x, y, z..) of len full words as 96 len consecutive values
+// from out on: 16-byte stores between the aligned ends.
+__device__ __forceinline__ void write_run(int32_t* __restrict__ out, int len, int x, int y, int z) {
+  const int lane = threadIdx.x & 31;
+  const int n = 96 * len;
+  const int head = (int)((0u - (uint32_t)((uintptr_t)out >> 2)) & 3u);
+  auto value = [&](int v, int axis) { return axis == 0 ? x : axis == 1 ? y : z + v; };
+  if (lane < head) out[lane] = value(lane / 3, lane % 3);
+  int d = head + 4 * lane, v = d / 3, axis = d - 3 * v;
+  for (; d + 4 <= n; d += 128) {  // 128 = 3 * 42 + 2
+    const int zv = z + v;
+    *reinterpret_cast<int4*>(out + d) = axis == 0   ? make_int4(x, y, zv, x)
+                                        : axis == 1 ? make_int4(y, zv, x, y)
+                                                    : make_int4(zv, x, y, zv + 1);
+    const bool wrap = axis > 0;
+    axis = wrap ? axis - 1 : 2;
+    v += wrap ? 43 : 42;
+  }
+  const int tail = (n - head) & 3;
+  if (lane < tail) {
+    const int e = n - tail + lane;
+    out[e] = value(e / 3, e % 3);
+  }
+}
+
+// One block per tile.  Each lane takes one word per chunk; the warps' totals
+// give each warp its place.  Then, in the words' order, the 32 lanes take the
+// 32 bits of each non-empty word (kRuns: but a run of full words within a row
+// is written as one block of consecutive values), so the set voxels'
+// coordinates are one contiguous list -- lexicographic (x, y, z) overall.
+// Positions at or past `count` are not written.  Needs nwords < 2^32 (word
+// coordinates in 32 bits).  kRuns is for labels with at least 4 voxels a word
+// on average, the volumes, which are bound by their writes: 405M and 231M
+// voxels 941 and 524 us without it, 828 and 483 us (5.8 TB/s) with it.  The
+// surfaces (3.3M voxels in 20.7M words), bound by instructions, take 111 us
+// with it and 89 us without (100 us with a scan of every chunk's counts).
+template <bool kRuns>
 __global__ void __launch_bounds__(kTileThreads) extract_tile_kernel(Geom g, const uint32_t* __restrict__ v,
                                                                     const int64_t* __restrict__ toff, int64_t nwords,
                                                                     int64_t count, int32_t* __restrict__ out) {
@@ -443,48 +612,56 @@ __global__ void __launch_bounds__(kTileThreads) extract_tile_kernel(Geom g, cons
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
   const int64_t base = (int64_t)blockIdx.x * kTileWords + (int64_t)warp * (kTileChunks * 32);
-  uint32_t word[kTileChunks], incl[kTileChunks];
+  uint32_t word[kTileChunks];
   uint32_t run = 0;
 #pragma unroll
   for (int c = 0; c < kTileChunks; ++c) {
     const int64_t i = base + c * 32 + lane;
     word[c] = i < nwords ? v[i] : 0u;
-    uint32_t p = (uint32_t)__popc(word[c]);
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t t = __shfl_up_sync(FULL, p, d);
-      if (lane >= d) p += t;
-    }
-    incl[c] = run + p;
-    run += __shfl_sync(FULL, p, 31);
+    run += (uint32_t)__popc(word[c]);
   }
+  run = __reduce_add_sync(FULL, run);
   if (lane == 0) s_warp[warp] = run;
   __syncthreads();
-  uint32_t before = 0;
-  for (int w = 0; w < warp; ++w) before += s_warp[w];
-  const int64_t start = toff[blockIdx.x] + before;
+  if (!run) return;
+  int64_t pos = toff[blockIdx.x];
+  for (int w = 0; w < warp; ++w) pos += s_warp[w];
 #pragma unroll
   for (int c = 0; c < kTileChunks; ++c) {
     unsigned nz = __ballot_sync(FULL, word[c] != 0u);
     if (!nz) continue;
     const uint32_t i = (uint32_t)(base + c * 32 + lane);
     const uint32_t row = i / (uint32_t)g.nw;
-    const int wz = (int)(i - row * (uint32_t)g.nw);
-    const int y = (int)(row % (uint32_t)g.ny), x = (int)(row / (uint32_t)g.ny);
-    const uint32_t excl = incl[c] - (uint32_t)__popc(word[c]);
+    const int wz = (int)(i - row * (uint32_t)g.nw) * 32 + g.vz;
+    const int y = (int)(row % (uint32_t)g.ny) + g.vy, x = (int)(row / (uint32_t)g.ny) + g.vx;
+    unsigned full = 0, row_start = 0;
+    if (kRuns) {
+      full = __ballot_sync(FULL, word[c] == FULL);
+      row_start = __ballot_sync(FULL, wz == g.vz);
+    }
     while (nz) {
       const int j = __ffs(nz) - 1;
+      const int xx = __shfl_sync(FULL, x, j), yy = __shfl_sync(FULL, y, j), zz = __shfl_sync(FULL, wz, j);
+      if (kRuns && ((full >> j) & 1u)) {
+        const unsigned stop = (~full | (row_start & ~(1u << j))) >> j;  // bit 0 is clear
+        const int len = stop ? __ffs(stop) - 1 : 32 - j;
+        if (pos + 32 * len <= count) {
+          write_run(out + 3 * pos, len, xx, yy, zz);
+          pos += 32 * len;
+          nz &= len + j < 32 ? FULL << (len + j) : 0u;
+          continue;
+        }
+      }
       nz &= nz - 1u;
       const uint32_t m = __shfl_sync(FULL, word[c], j);
-      const uint32_t e = __shfl_sync(FULL, excl, j);
-      const int xx = __shfl_sync(FULL, x, j), yy = __shfl_sync(FULL, y, j), ww = __shfl_sync(FULL, wz, j);
-      const int64_t pos = start + e + __popc(m & lt);
-      if (((m >> lane) & 1u) && pos < count) {
-        int32_t* p = out + 3 * pos;
-        p[0] = xx + g.vx;
-        p[1] = yy + g.vy;
-        p[2] = ww * 32 + lane + g.vz;
+      const int64_t o = pos + __popc(m & lt);
+      if (((m >> lane) & 1u) && o < count) {
+        int32_t* p = out + 3 * o;
+        p[0] = xx;
+        p[1] = yy;
+        p[2] = zz + lane;
       }
+      pos += __popc(m);
     }
   }
 }
@@ -690,17 +867,26 @@ extern "C" int a3d_flood_fill(const int64_t* dam_ijk, int64_t n, const a3d_flood
   A3D_REQUIRE(!(hs[0] & 1u), A3D_ERR_OVERFLOW, "a3d_flood_fill: relaxation did not converge within 2^20 rounds");
   const int rounds = (int)hs[1];
   if (rounds_out) *rounds_out = rounds;
-  const unsigned gw = (unsigned)ceil_div(nwords, 256);
-  A3D_PDL(labels_kernel, dim3(gw), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
-  // k-ring box dilation of the dam, ping-ponging ring buffers
-  uint32_t* ring_a = w.lab + (int64_t)kRing * nwords;
-  A3D_CUDA_TRY(cudaMemcpyAsync(ring_a, w.lab + (int64_t)kDam * nwords, nwords * 4, cudaMemcpyDeviceToDevice, s));
-  uint32_t* ring_b = w.ring2;
-  for (int k = 0; k < geom->k_ring; ++k) {
-    A3D_PDL(box_dilate_kernel, dim3(gw), dim3(256), 0, s, g, ring_a, ring_b, nwords);
-    uint32_t* t = ring_a; ring_a = ring_b; ring_b = t;
+  const unsigned gr = (unsigned)ceil_div((int64_t)g.nx * ceil_div(g.ny, kRun) * g.nw, 256);
+  if (conn == 6)
+    A3D_PDL(labels_kernel<6>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+  else if (conn == 18)
+    A3D_PDL(labels_kernel<18>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+  else
+    A3D_PDL(labels_kernel<26>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+  // k-ring box dilation of the dam, ping-ponging ring buffers; the last ring
+  // decides the labels, and none leaves nothing outside the dam
+  const uint32_t* ring = w.lab + (int64_t)kDam * nwords;
+  uint32_t* bufs[2] = {w.lab + (int64_t)kRing * nwords, w.ring2};
+  for (int k = 0; k + 1 < geom->k_ring; ++k) {
+    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, ring, bufs[k & 1], w.lab, nwords);
+    ring = bufs[k & 1];
   }
-  A3D_PDL(ring_classify_kernel, dim3(gw), dim3(256), 0, s, ring_a, w.lab, nwords);
+  if (geom->k_ring > 0) {
+    A3D_PDL(box_dilate_kernel<true>, dim3(gr), dim3(256), 0, s, g, ring, (uint32_t*)nullptr, w.lab, nwords);
+  } else {
+    A3D_CUDA_TRY(cudaMemsetAsync(w.lab + (int64_t)kExtTide * nwords, 0, 2 * nwords * 4, s));
+  }
   // counts per label and tile, one pass and one host read
   const int64_t ntiles = tiles_of(g);
   unsigned long long* tot = reinterpret_cast<unsigned long long*>(w.misc + 8);
@@ -728,7 +914,12 @@ extern "C" int a3d_flood_extract(const a3d_flood_geom* geom, void* workspace, si
   const uint32_t* v = w.lab + (int64_t)label * nwords;
   A3D_TRY((device_exclusive_scan<uint32_t, int64_t>(w.tcnt + (int64_t)label * ntiles, w.toff, ntiles, w.scan_tmp,
                                                      w.toff + ntiles, s)));
-  A3D_PDL(extract_tile_kernel, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, g, v, w.toff, nwords, count, out_ijk);
+  if (count >= 4 * nwords)
+    A3D_PDL(extract_tile_kernel<true>, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, g, v, w.toff, nwords, count,
+            out_ijk);
+  else
+    A3D_PDL(extract_tile_kernel<false>, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, g, v, w.toff, nwords, count,
+            out_ijk);
   return A3D_OK;
 }
 
@@ -780,13 +971,13 @@ extern "C" int a3d_ring_signs(const int64_t* dam_ijk, int64_t n_dam, const int64
     A3D_PDL(set_bits_kernel, dim3((unsigned)ceil_div(n_dry, 256)), dim3(256), 0, s, dry_ijk, n_dry, g,
             w.lab + (int64_t)kDry * nwords);
   }
-  const unsigned gw = (unsigned)ceil_div(nwords, 256);
+  const unsigned gr = (unsigned)ceil_div((int64_t)g.nx * ceil_div(g.ny, kRun) * g.nw, 256);
   uint32_t* ring_out = w.lab + (int64_t)kExtTide * nwords;
   const uint32_t* src = v_dam;
   uint32_t* bufs[2] = {w.lab + (int64_t)kRing * nwords, w.ring2};
   for (int k = 0; k < geom->k_ring; ++k) {
     uint32_t* dst = (k == geom->k_ring - 1) ? ring_out : bufs[k & 1];
-    A3D_PDL(box_dilate_kernel, dim3(gw), dim3(256), 0, s, g, src, dst, nwords);
+    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, src, dst, w.lab, nwords);
     src = dst;
   }
   if (geom->k_ring == 0)
