@@ -5,7 +5,8 @@ get_node_neighbors, none of them on the descent's path).
 
 ``octree_traverse`` runs the whole descent in one native call
 (a3d_octree_traverse): per level, one SAT any-hit query per candidate cube
-over the wide BVH, then a stable prefix-sum compaction, so the output order
+over the wide BVH (or, where voxels meet few triangles, over the list that the
+parent hands down), then a stable prefix-sum compaction, so the output order
 is the reference's (meshgrid 'ij' at ``min_level``, parents in order, 8
 children each in CUBE_CORNERS order).  Morton keys are computed by the
 native a3d_morton_encode / a3d_morton_decode kernels.
