@@ -135,7 +135,7 @@ __global__ void corner_pos_kernel(DmcIn in, float ws, float* __restrict__ x) {
 // compute them from the cube (corner_world).
 template <bool kVec>
 __global__ void corner_case_kernel(DmcIn in, uint8_t* __restrict__ cases, uint32_t* __restrict__ flag,
-                                   uint32_t* __restrict__ bad_index) {
+                                   uint32_t* __restrict__ bad_index, uint32_t* __restrict__ nprob) {
   pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= in.n) return;
@@ -162,7 +162,9 @@ __global__ void corner_case_kernel(DmcIn in, uint8_t* __restrict__ cases, uint32
   }
   if (bad) *bad_index = 1u;
   cases[i] = (uint8_t)bits;
-  flag[i] = (bits != 0u && bits != 255u) ? 1u : 0u;
+  const bool surface = bits != 0u && bits != 255u;
+  flag[i] = surface ? 1u : 0u;
+  if (surface && kCheck[bits][0] == 1) atomicAdd(nprob, 1u);
 }
 
 // copies scattered device words into one block, so that the host reads
@@ -178,29 +180,37 @@ __global__ void gather_words_kernel(WordList l, uint32_t* __restrict__ out) {
   if (k < l.n) out[k] = *l.src[k];
 }
 
-__global__ void compact_kernel(int64_t n, const uint32_t* __restrict__ flag, const uint32_t* __restrict__ off,
-                               uint32_t* __restrict__ list) {
-  pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && flag[i]) list[off[i]] = (uint32_t)i;
-}
-
 __device__ __forceinline__ uint64_t hash64(uint64_t k) {
   k ^= k >> 33; k *= 0xff51afd7ed558ccdull; k ^= k >> 33; k *= 0xc4ceb9fe1a85ec53ull; k ^= k >> 33;
   return k;
 }
 
-// Stage-B kernels run over all N cubes and read the surface-cube count Ns
-// from the device (no host round trip before the crossing count).
-__global__ void prob_insert_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, const uint32_t* __restrict__ list,
-                                   const uint8_t* __restrict__ cases, unsigned long long* __restrict__ table,
-                                   uint64_t mask) {
+// The table of the cubes whose case must be checked against a neighbour is
+// used at the size that their number (on the device) asks for: a power of two
+// of at least twice as many places, and clearing and probing it cost what they
+// hold.
+__device__ __forceinline__ uint64_t table_mask_of(uint32_t nprob) {
+  const uint64_t want = 2ull * (nprob < 32u ? 32u : nprob);
+  return (1ull << (64 - __clzll((long long)(want - 1)))) - 1;
+}
+
+__global__ void table_clear_kernel(const uint32_t* __restrict__ nprob, unsigned long long* __restrict__ table) {
   pdl_wait();
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)*ns_dev) return;
-  const uint32_t i = list[t];
-  const int c = cases[i];
-  if (kCheck[c][0] != 1) return;
+  const uint64_t size = table_mask_of(*nprob) + 1;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < size; i += (uint64_t)gridDim.x * blockDim.x)
+    table[i] = ~0ull;
+}
+
+// lists the surface cubes and enters those to be checked in the table
+__global__ void compact_kernel(DmcIn in, const uint32_t* __restrict__ flag, const uint32_t* __restrict__ off,
+                               const uint8_t* __restrict__ cases, const uint32_t* __restrict__ nprob,
+                               uint32_t* __restrict__ list, unsigned long long* __restrict__ table) {
+  pdl_wait();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= in.n || !flag[i]) return;
+  list[off[i]] = (uint32_t)i;
+  if (kCheck[cases[i]][0] != 1) return;
+  const uint64_t mask = table_mask_of(*nprob);
   const uint64_t r = (uint64_t)in.res;
   const uint64_t key = ((uint64_t)in.vox[3 * i] * r + (uint64_t)in.vox[3 * i + 1]) * r + (uint64_t)in.vox[3 * i + 2];
   uint64_t h = hash64(key) & mask;
@@ -211,12 +221,22 @@ __global__ void prob_insert_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev
   }
 }
 
+// Runs over all N cubes and reads the surface-cube count Ns from the device (no
+// host round trip before the crossing count).  The case a surface cube is
+// meshed with, and its crossing edges from its sign bits (the raw case id: an
+// edge crosses when its two corners' bits differ, the test the case id was made
+// with).
 __global__ void case_fix_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, const uint32_t* __restrict__ list,
                                 const uint8_t* __restrict__ cases, const unsigned long long* __restrict__ table,
-                                uint64_t mask, uint8_t* __restrict__ case_s) {
+                                const uint32_t* __restrict__ nprob, uint8_t* __restrict__ case_s,
+                                uint16_t* __restrict__ mask12, uint32_t* __restrict__ cnt) {
   pdl_wait();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (int64_t)*ns_dev) return;
+  if (t >= in.n) return;
+  if (t >= (int64_t)*ns_dev) {  // the scan runs over all N entries
+    cnt[t] = 0;
+    return;
+  }
   const uint32_t i = list[t];
   const int c = cases[i];
   int out = c;
@@ -224,6 +244,7 @@ __global__ void case_fix_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, c
     const int64_t ax = in.vox[3 * i] + kCheck[c][1], ay = in.vox[3 * i + 1] + kCheck[c][2],
                   az = in.vox[3 * i + 2] + kCheck[c][3];
     if (ax >= 0 && ay >= 0 && az >= 0 && ax < in.res && ay < in.res && az < in.res) {
+      const uint64_t mask = table_mask_of(*nprob);
       const uint64_t r = (uint64_t)in.res;
       const uint64_t key = ((uint64_t)ax * r + (uint64_t)ay) * r + (uint64_t)az;
       uint64_t h = hash64(key) & mask;
@@ -236,6 +257,12 @@ __global__ void case_fix_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, c
     }
   }
   case_s[t] = (uint8_t)out;
+  uint32_t m = 0;
+#pragma unroll
+  for (int e = 0; e < 12; ++e)
+    if ((((uint32_t)c >> kCE[2 * e]) ^ ((uint32_t)c >> kCE[2 * e + 1])) & 1u) m |= 1u << e;
+  mask12[t] = (uint16_t)m;
+  cnt[t] = (uint32_t)__popc(m);
 }
 
 // positions of the ends of cube edge e of a cube at voxel vx.  A unique
@@ -249,37 +276,18 @@ __device__ __forceinline__ void edge_world(const DmcIn& in, float ws, const floa
   corner_world(in, ws, vx, kCE[2 * e + 1], i1, xb);
 }
 
-// crossing edges of each surface cube from its sign bits (the raw case id:
-// an edge crosses when its two corners' bits differ, the test the case id
-// was made with)
-__global__ void cross_count_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, const uint32_t* __restrict__ list,
-                                   const uint8_t* __restrict__ cases, uint16_t* __restrict__ mask12,
-                                   uint32_t* __restrict__ cnt) {
-  pdl_wait();
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= in.n) return;
-  if (t >= (int64_t)*ns_dev) {  // the scan runs over all N entries
-    cnt[t] = 0;
-    return;
-  }
-  const uint32_t c = cases[list[t]];
-  uint32_t m = 0;
-#pragma unroll
-  for (int e = 0; e < 12; ++e)
-    if (((c >> kCE[2 * e]) ^ (c >> kCE[2 * e + 1])) & 1u) m |= 1u << e;
-  mask12[t] = (uint16_t)m;
-  cnt[t] = (uint32_t)__popc(m);
-}
-
 // Crossing entries (key, val) of the surface cubes, val = t * 12 + e in edge
 // order.  A block's entries form one contiguous range of the output (off is
 // the exclusive scan of the per-cube counts), so they are staged in shared
-// memory and written with consecutive threads on consecutive entries.
+// memory and written with consecutive threads on consecutive entries.  Each
+// entry is counted at its lower endpoint on the way, and the count it finds is
+// its place in that endpoint's group of the sort below.
 constexpr int kCrossThreads = 128;
 __global__ void __launch_bounds__(kCrossThreads)
     cross_write_kernel(DmcIn in, const uint32_t* __restrict__ ns_dev, const uint32_t* __restrict__ list,
                        const uint16_t* __restrict__ mask12, const uint32_t* __restrict__ off,
-                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t* __restrict__ group_cnt,
+                       uint32_t* __restrict__ place) {
   pdl_wait();
   __shared__ uint64_t s_key[kCrossThreads * 12];
   __shared__ uint32_t s_val[kCrossThreads * 12];
@@ -309,8 +317,10 @@ __global__ void __launch_bounds__(kCrossThreads)
   }
   __syncthreads();
   for (int k = threadIdx.x; k < cnt; k += kCrossThreads) {
-    keys[o0 + k] = s_key[k];
+    const uint64_t key = s_key[k];
+    keys[o0 + k] = key;
     vals[o0 + k] = s_val[k];
+    place[o0 + k] = atomicAdd(&group_cnt[key >> 32], 1u);  // corner_at keeps ids below num_corners
   }
 }
 
@@ -321,43 +331,30 @@ __global__ void __launch_bounds__(kCrossThreads)
 // group holds at most 24 entries and every entry finds its place by ranking
 // itself within its group.  vals grow with the input position, so the order
 // equals a stable sort by key.
-__global__ void edge_count_kernel(const uint64_t* __restrict__ keys, int64_t nc, uint64_t m,
-                                  uint32_t* __restrict__ lo_of, uint32_t* __restrict__ cnt) {
-  pdl_wait();
-  const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= nc) return;
-  const uint32_t i0 = (uint32_t)(keys[j] >> 32);
-  lo_of[j] = i0;
-  atomicAdd(&cnt[i0], 1u);
-}
-
 __global__ void edge_scatter_kernel(const uint64_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t nc,
-                                    const uint32_t* __restrict__ lo_of, const uint32_t* __restrict__ start,
-                                    uint32_t* __restrict__ fill, uint64_t* __restrict__ keys_g,
-                                    uint32_t* __restrict__ vals_g, uint32_t* __restrict__ lo_g) {
+                                    const uint32_t* __restrict__ place, const uint32_t* __restrict__ start,
+                                    uint64_t* __restrict__ keys_g, uint32_t* __restrict__ vals_g) {
   pdl_wait();
   const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nc) return;
-  const uint32_t i0 = lo_of[j];
-  const uint32_t p = start[i0] + atomicAdd(&fill[i0], 1u);
-  keys_g[p] = keys[j];
+  const uint64_t k = keys[j];
+  const uint32_t p = start[k >> 32] + place[j];
+  keys_g[p] = k;
   vals_g[p] = vals[j];
-  lo_g[p] = i0;
 }
 
 // Also writes the run-start flags of the sorted entries (entry j starts a
 // run of equal keys when j == 0 or key[j] != key[j - 1]): an entry starts
 // its run when no entry of its group has the same key and a smaller val.
 __global__ void edge_rank_kernel(const uint64_t* __restrict__ keys_g, const uint32_t* __restrict__ vals_g, int64_t nc,
-                                 const uint32_t* __restrict__ lo_g, const uint32_t* __restrict__ start,
+                                 const uint32_t* __restrict__ start,
                                  uint64_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                  uint32_t* __restrict__ run_flag) {
   pdl_wait();
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= nc) return;
-  const uint32_t i0 = lo_g[p];
-  const uint32_t b = start[i0], e = start[i0 + 1];
   const uint64_t k = keys_g[p];
+  const uint32_t b = start[k >> 32], e = start[(k >> 32) + 1];
   const uint32_t v = vals_g[p];
   uint32_t rank = 0, dup_before = 0;
   for (uint32_t q = b; q < e; ++q) {
@@ -495,6 +492,18 @@ __device__ __forceinline__ void edge_normal(const float* x0, const float* x1, fl
   const float gm = fd(fsb(s1, s0), len);
   const float sg = gm > 0.f ? 1.f : (gm < 0.f ? -1.f : 0.f);
   float u[3];
+  if ((ev[0] == 0.f) + (ev[1] == 0.f) + (ev[2] == 0.f) == 2 && len < INFINITY) {
+    // along an axis (every edge without deformation): the zeros stay what their
+    // divisions give, so each division is done for one component
+    const int ax = ev[0] != 0.f ? 0 : ev[1] != 0.f ? 1 : 2;
+    const float q = fm(fd(ax == 0 ? ev[0] : ax == 1 ? ev[1] : ev[2], len), sg);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) u[a] = a == ax ? q : fm(ev[a], sg);
+    const float un = fd(q, fmaxf(sqrtf(fm(q, q)), 1e-12f));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) n[a] = a == ax ? un : u[a];
+    return;
+  }
 #pragma unroll
   for (int a = 0; a < 3; ++a) u[a] = fm(fd(ev[a], len), sg);
   const float ul = sqrtf(fa(fa(fm(u[0], u[0]), fm(u[1], u[1])), fm(u[2], u[2])));
@@ -513,7 +522,11 @@ __device__ __forceinline__ float ldf(const float* p, int64_t i) { return __ldg(p
 // 64-B row of cube_idx, which stays in L1 for the vertex's edges, instead
 // of through the crossing's unique-edge index.  Eight 128-thread blocks per
 // SM (<= 64 registers, no spills): the gathers are latency-bound, so the
-// resident warps (32 instead of 28 at 68 registers) set the throughput.
+// resident warps (32 instead of 28 at 68 registers) set the throughput.  The
+// divisions weigh as much: without those of the second crossing (no alpha
+// weights) and of a normal's zero components 110 -> 97 us at 512^3; outputs
+// staged and written with consecutive lanes gave 7 us more on the kernel alone
+// and nothing on the call.
 __global__ void __launch_bounds__(128, 8) vd_kernel(DmcIn in, int64_t nv, const uint32_t* __restrict__ list,
                           const uint8_t* __restrict__ case_s, const uint32_t* __restrict__ vd_cube,
                           const uint8_t* __restrict__ vd_slot, const uint32_t* __restrict__ goff, EdgeData ed,
@@ -555,7 +568,8 @@ __global__ void __launch_bounds__(128, 8) vd_kernel(DmcIn in, int64_t nv, const 
       out.palpha[3 * g + a] = ue;
       out.nalpha[3 * g + a] = n[a];
       acc[a] = fa(acc[a], fm(ue, b));
-      z[k][a] = interp1(xa[a], xb[a], pw0, pw1, pden);  // the plain zero crossing
+      // the plain zero crossing: without alpha weights it is the same one
+      z[k][a] = in.alpha ? interp1(xa[a], xb[a], pw0, pw1, pden) : ue;
     }
     bsum = fa(bsum, b);
     ++g;
@@ -688,14 +702,18 @@ __device__ __forceinline__ void scatter_interp_grad(const DmcIn& in, const float
 }
 
 // One thread per dual vertex.  The slot loops are not unrolled (the kernel
-// stays small enough for the instruction cache): each pass reloads a slot's
-// corner ids, signs and weights (the cube's 64-B row of cube_idx, sdf and the
-// weights stay in L1 across the passes) and recomputes its crossings.  An
-// edge's corner ids are the cube's own ids at its two local corners.  Without
-// an L_dev gradient two passes suffice (dual vertex, then the scatter).
-// Gradient order as the forward's reverse: L_dev -> distances -> plain
-// crossings and the dual vertex -> weighted average -> interpolation
-// weights -> sdf, deform, alpha, beta.
+// stays small enough for the instruction cache): the first pass and the scatter
+// load a slot's corner ids, signs and weights (the cube's 64-B row of cube_idx,
+// sdf and the weights stay in L1 in between) and compute its crossings; the
+// L_dev passes between them read the plain crossings that the first one left in
+// shared memory.  An edge's corner ids are the cube's own ids at its two local
+// corners.  Gradient order as the forward's reverse: L_dev -> distances -> plain
+// crossings and the dual vertex -> weighted average -> interpolation weights ->
+// sdf, deform, alpha, beta.  Without alpha weights both crossings are one, and
+// their gradients are scattered together.
+// Bound by instructions: a 512^3 grid's vertices (sdf gradients, L_dev) took 146
+// us with the crossings computed anew in each of five passes, now 94.
+constexpr int kBwdThreads = 128;
 struct BwdSlot {
   int64_t i0, i1;
   float s0, s1, a0, a1, b;
@@ -717,7 +735,7 @@ __device__ __forceinline__ void bwd_slot(const DmcIn& in, float ws, const float*
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
     q.ue[a] = interp1(q.xa[a], q.xb[a], w0, w1, den);
-    q.z[a] = interp1(q.xa[a], q.xb[a], pw0, pw1, pden);
+    q.z[a] = in.alpha ? interp1(q.xa[a], q.xb[a], pw0, pw1, pden) : q.ue[a];
   }
 }
 
@@ -732,7 +750,7 @@ __device__ __forceinline__ float bwd_dist(const BwdSlot& q, const float* vd) {
   return sqrtf(d2);
 }
 
-__global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, const uint32_t* __restrict__ list,
+__global__ void __launch_bounds__(kBwdThreads, 8) vd_bwd_kernel(DmcIn in, int64_t nv, const uint32_t* __restrict__ list,
                                                      const uint8_t* __restrict__ case_s,
                                                      const uint32_t* __restrict__ vd_cube,
                                                      const uint8_t* __restrict__ vd_slot,
@@ -749,6 +767,9 @@ __global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, co
   float vx[3];
   load_voxel(in, cube, vx);
   const int64_t g0 = goff[v];
+  __shared__ float s_z[7][3][kBwdThreads];  // plain crossings
+  const int th = threadIdx.x;
+  const bool with_ldev = gr.g_ldev != nullptr;
   BwdSlot q;
   // forward: weighted average of the alpha-weighted crossings
   float acc[3] = {0.f, 0.f, 0.f}, bsum = 0.f;
@@ -759,7 +780,10 @@ __global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, co
     if (e == 15) continue;
     bwd_slot(in, ws, vx, cube, e, q);
 #pragma unroll
-    for (int a = 0; a < 3; ++a) acc[a] = fa(acc[a], fm(q.ue[a], q.b));
+    for (int a = 0; a < 3; ++a) {
+      acc[a] = fa(acc[a], fm(q.ue[a], q.b));
+      if (with_ldev) s_z[ne][a][th] = q.z[a];
+    }
     bsum = fa(bsum, q.b);
     ++ne;
   }
@@ -774,46 +798,39 @@ __global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, co
     for (int a = 0; a < 3; ++a) gvd[a] = gr.g_verts[3 * v + a] + gr.g_vd[3 * v + a];
   // L_dev backward (mad = |dist - mean|, mean = sum(dist)/ne): gD of slot
   // k = gl_k sign(D_k - mean) + gm, gm = -sum_k gl_k sign(D_k - mean) / ne
-  const bool with_ldev = gr.g_ldev != nullptr;
   float mean = 0.f, gm = 0.f;
+  auto left_dist = [&](int r) {  // bwd_dist of the stored crossing
+    float d2 = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const float dd = fsb(s_z[r][a][th], vd[a]);
+      d2 = fa(d2, fm(dd, dd));
+    }
+    return sqrtf(d2);
+  };
   if (with_ldev) {
     float msum = 0.f;
 #pragma unroll 1
-    for (int k = 0; k < 7; ++k) {
-      const int e = vd_edge(vedges, k);
-      if (e == 15) continue;
-      bwd_slot(in, ws, vx, cube, e, q);
-      msum = fa(msum, bwd_dist(q, vd));
-    }
+    for (int r = 0; r < ne; ++r) msum = fa(msum, left_dist(r));
     mean = fd(msum, (float)ne);
     float gmean = 0.f;
-    int r = 0;
 #pragma unroll 1
-    for (int k = 0; k < 7; ++k) {
-      const int e = vd_edge(vedges, k);
-      if (e == 15) continue;
-      bwd_slot(in, ws, vx, cube, e, q);
-      const float df = bwd_dist(q, vd) - mean;
+    for (int r = 0; r < ne; ++r) {
+      const float df = left_dist(r) - mean;
       const float sg = df > 0.f ? 1.f : (df < 0.f ? -1.f : 0.f);
       gmean -= gr.g_ldev[g0 + r] * sg;
-      ++r;
     }
     gm = gmean / (float)ne;
     // dist -> crossing z and the dual vertex
-    r = 0;
 #pragma unroll 1
-    for (int k = 0; k < 7; ++k) {
-      const int e = vd_edge(vedges, k);
-      if (e == 15) continue;
-      bwd_slot(in, ws, vx, cube, e, q);
-      const float D = bwd_dist(q, vd);
+    for (int r = 0; r < ne; ++r) {
+      const float D = left_dist(r);
       const float df = D - mean;
       const float sg = df > 0.f ? 1.f : (df < 0.f ? -1.f : 0.f);
       const float gD = gr.g_ldev[g0 + r] * sg + gm;
       const float invd = D > 0.f ? 1.0f / D : 0.f;
 #pragma unroll
-      for (int a = 0; a < 3; ++a) gvd[a] -= gD * ((q.z[a] - vd[a]) * invd);
-      ++r;
+      for (int a = 0; a < 3; ++a) gvd[a] -= gD * ((s_z[r][a][th] - vd[a]) * invd);
     }
   }
   // vd = sum(b ue) / (sum b + 1e-8)
@@ -836,6 +853,30 @@ __global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, co
       if (gr.g_palpha) gue[a] += gr.g_palpha[3 * (g0 + r) + a];
       gb += gvd[a] * q.ue[a] * inv_bden;
     }
+    // plain crossing z through w0 = s1, w1 = -s0 (zero without an L_dev
+    // gradient)
+    float gZ[3] = {0.f, 0.f, 0.f};
+    if (with_ldev) {
+      const float D = bwd_dist(q, vd);
+      const float df = D - mean;
+      const float sg = df > 0.f ? 1.f : (df < 0.f ? -1.f : 0.f);
+      const float gD = gr.g_ldev[g0 + r] * sg + gm;
+      const float invd = D > 0.f ? 1.0f / D : 0.f;
+#pragma unroll
+      for (int a = 0; a < 3; ++a) gZ[a] = gD * ((q.z[a] - vd[a]) * invd);
+      if (in.alpha) {
+        const float w0 = q.s1, w1 = -q.s0, den = w0 + w1;
+        float gw0, gw1;
+        scatter_interp_grad(in, gZ, q.xa, q.xb, q.z, w0, w1, den, i0, i1, gw0, gw1, gr);
+        if (gr.g_sdf) {
+          atomicAdd(&gr.g_sdf[i1], gw0);
+          atomicAdd(&gr.g_sdf[i0], -gw1);
+        }
+      } else {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) gue[a] += gZ[a];
+      }
+    }
     // ue through w0 = s1 a1, w1 = -s0 a0
     {
       const float w0 = q.s1 * q.a1, w1 = -(q.s0 * q.a0), den = w0 + w1;
@@ -850,25 +891,6 @@ __global__ void __launch_bounds__(128, 8) vd_bwd_kernel(DmcIn in, int64_t nv, co
         const float t0 = tanhf(in.alpha[8 * (int64_t)cube + c0]), t1 = tanhf(in.alpha[8 * (int64_t)cube + c1]);
         atomicAdd(&gr.g_alpha[8 * (int64_t)cube + c1], gw0 * q.s1 * in.wscale * (1.f - t1 * t1));
         atomicAdd(&gr.g_alpha[8 * (int64_t)cube + c0], -gw1 * q.s0 * in.wscale * (1.f - t0 * t0));
-      }
-    }
-    // plain crossing z through w0 = s1, w1 = -s0 (zero without an L_dev
-    // gradient)
-    if (with_ldev) {
-      const float D = bwd_dist(q, vd);
-      const float df = D - mean;
-      const float sg = df > 0.f ? 1.f : (df < 0.f ? -1.f : 0.f);
-      const float gD = gr.g_ldev[g0 + r] * sg + gm;
-      const float invd = D > 0.f ? 1.0f / D : 0.f;
-      float gZ[3];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) gZ[a] = gD * ((q.z[a] - vd[a]) * invd);
-      const float w0 = q.s1, w1 = -q.s0, den = w0 + w1;
-      float gw0, gw1;
-      scatter_interp_grad(in, gZ, q.xa, q.xb, q.z, w0, w1, den, i0, i1, gw0, gw1, gr);
-      if (gr.g_sdf) {
-        atomicAdd(&gr.g_sdf[i1], gw0);
-        atomicAdd(&gr.g_sdf[i0], -gw1);
       }
     }
     // edge normal (n_alpha) through the edge vector
@@ -1103,9 +1125,8 @@ struct DmcWs {
   float* g_vd;         // [4N,3]
   uint32_t* scan_tmp;
   uint32_t* misc;      // counters
-  uint32_t* ecnt;      // [M] edge-sort group sizes, then fill counters
+  uint32_t* ecnt;      // [M] edge-sort group sizes
   uint32_t* estart;    // [M+1] edge-sort group starts
-  uint64_t table_mask;
 };
 
 uint64_t pow2_at_least(uint64_t v) {
@@ -1116,8 +1137,7 @@ uint64_t pow2_at_least(uint64_t v) {
 
 size_t carve_dmc(DmcWs& w, Workspace& ws, int64_t n, int64_t m) {
   const int64_t n12 = 12 * n + 1;
-  const uint64_t tsize = pow2_at_least((uint64_t)(2 * n + 2));
-  w.table_mask = tsize - 1;
+  const uint64_t tsize = pow2_at_least((uint64_t)(2 * n + 2 < 64 ? 64 : 2 * n + 2));  // see table_mask_of
   w.x = ws.take<float>(3 * m);
   w.cases = ws.take<uint8_t>(n);
   w.flag = ws.take<uint32_t>(n);
@@ -1193,25 +1213,27 @@ extern "C" int a3d_dmc_prepare(const a3d_dmc_inputs* p, void* workspace, size_t 
   for (int k = 0; k < 6; ++k) counts[k] = 0;
   if (n == 0 || m == 0) return A3D_OK;
   DmcIn in = make_in(p);
-  // misc[1]: out-of-range corner ids; misc[4..6] and misc[8..14]: the words
-  // the two host reads take
+  // misc[1]: out-of-range corner ids; misc[2]: cubes to be checked; misc[4..6]
+  // and misc[8..14]: the words the two host reads take
   uint32_t* bad_index = w.misc + 1;
-  A3D_TRY(fill_async<uint32_t>(bad_index, 1, 0u, s));
+  uint32_t* nprob = w.misc + 2;
+  A3D_TRY(fill_async<uint32_t>(bad_index, 2, 0u, s));
   if (((uintptr_t)in.cidx & 15u) == 0)
-    A3D_PDL(corner_case_kernel<true>, dim3(gsz(n)), dim3(256), 0, s, in, w.cases, w.flag, bad_index);
+    A3D_PDL(corner_case_kernel<true>, dim3(gsz(n)), dim3(256), 0, s, in, w.cases, w.flag, bad_index, nprob);
   else
-    A3D_PDL(corner_case_kernel<false>, dim3(gsz(n)), dim3(256), 0, s, in, w.cases, w.flag, bad_index);
+    A3D_PDL(corner_case_kernel<false>, dim3(gsz(n)), dim3(256), 0, s, in, w.cases, w.flag, bad_index, nprob);
   A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(w.flag, w.off, n, w.scan_tmp, w.off + n, s)));
   // stage B over all N cubes with the surface count on the device
   const uint32_t* ns_dev = w.off + n;
-  A3D_PDL(compact_kernel, dim3(gsz(n)), dim3(256), 0, s, n, w.flag, w.off, w.list);
-  A3D_TRY(fill_async<unsigned long long>(w.table, (int64_t)(w.table_mask + 1), ~0ull, s));
-  A3D_PDL(prob_insert_kernel, dim3(gsz(n)), dim3(256), 0, s, in, ns_dev, w.list, w.cases, w.table, w.table_mask);
-  A3D_PDL(case_fix_kernel, dim3(gsz(n)), dim3(256), 0, s, in, ns_dev, w.list, w.cases, w.table, w.table_mask, w.case_s);
-  A3D_PDL(cross_count_kernel, dim3(gsz(n)), dim3(256), 0, s, in, ns_dev, w.list, w.cases, w.mask12, w.ccnt);
+  A3D_PDL(table_clear_kernel, dim3(num_sms() * 4), dim3(256), 0, s, nprob, w.table);
+  A3D_PDL(compact_kernel, dim3(gsz(n)), dim3(256), 0, s, in, w.flag, w.off, w.cases, nprob, w.list, w.table);
+  A3D_PDL(case_fix_kernel, dim3(gsz(n)), dim3(256), 0, s, in, ns_dev, w.list, w.cases, w.table, nprob, w.case_s,
+          w.mask12, w.ccnt);
   A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(w.ccnt, w.coff, n, w.scan_tmp, w.coff + n, s)));
+  // rid holds the entries' places in their groups until the scatter
+  A3D_TRY(fill_async<uint32_t>(w.ecnt, m, 0u, s));
   A3D_PDL(cross_write_kernel, dim3(gsz(n, kCrossThreads)), dim3(kCrossThreads), 0, s, in, ns_dev, w.list, w.mask12,
-          w.coff, w.keys, w.vals);
+          w.coff, w.keys, w.vals, w.ecnt, w.rid);
   // the one round trip before the edge sort: surface cubes, crossings and
   // the out-of-range flag
   uint32_t h3[3];
@@ -1223,16 +1245,10 @@ extern "C" int a3d_dmc_prepare(const a3d_dmc_inputs* p, void* workspace, size_t 
   counts[0] = ns;
   counts[1] = nc;  // crossing (cube, edge) entries == groups
   if (ns == 0) return A3D_OK;
-  // counting sort of the crossings by (key, val); rid, then qflag, hold the
-  // lower endpoints until the rank pass has read them
-  A3D_TRY(fill_async<uint32_t>(w.ecnt, m, 0u, s));
-  A3D_PDL(edge_count_kernel, dim3(gsz(nc)), dim3(256), 0, s, w.keys, nc, (uint64_t)m, w.rid, w.ecnt);
+  // counting sort of the crossings by (key, val)
   A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(w.ecnt, w.estart, m, w.scan_tmp, w.estart + m, s)));
-  A3D_TRY(fill_async<uint32_t>(w.ecnt, m, 0u, s));
-  A3D_PDL(edge_scatter_kernel, dim3(gsz(nc)), dim3(256), 0, s, w.keys, w.vals, nc, w.rid, w.estart, w.ecnt, w.keys2,
-          w.vals2, w.qflag);
-  A3D_PDL(edge_rank_kernel, dim3(gsz(nc)), dim3(256), 0, s, w.keys2, w.vals2, nc, w.qflag, w.estart, w.keys, w.vals,
-          w.rflag);
+  A3D_PDL(edge_scatter_kernel, dim3(gsz(nc)), dim3(256), 0, s, w.keys, w.vals, nc, w.rid, w.estart, w.keys2, w.vals2);
+  A3D_PDL(edge_rank_kernel, dim3(gsz(nc)), dim3(256), 0, s, w.keys2, w.vals2, nc, w.estart, w.keys, w.vals, w.rflag);
   A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(w.rflag, w.rid, nc, w.scan_tmp, w.misc, s)));
   // idx_map is read only at crossing (cube, edge) pairs, all of which
   // run_info_kernel writes: no clear.  The run count is in misc[0].
@@ -1413,23 +1429,62 @@ size_t carve_grad(GradWs& w, Workspace& ws, int64_t n, int64_t m) {
 // edge is listed once per cube holding it) and sums in ascending neighbour
 // order: deterministic FP64 sums.  Cube indices from one grid give a corner
 // at most one neighbour per axis and side, kept in 6 slots per corner
-// (edge_slot_kernel); when some slot is claimed by two different corners the
+// (slot_store_kernel); when some slot is claimed by two different corners the
 // neighbours are gathered from two adjacency lists instead (count, scan,
 // fill).  Both gathers give the same neighbours in the same order.
 constexpr uint32_t kNoCorner = 0xffffffffu;
 
-__global__ void edge_slot_kernel(DmcIn in, uint32_t* __restrict__ slots, uint32_t* __restrict__ conflict) {
+// positions of corners no cube names, empty slots, no conflict yet
+__global__ void slot_init_kernel(int64_t m, const float* __restrict__ deform, float* __restrict__ x,
+                                 uint32_t* __restrict__ slots, uint32_t* __restrict__ conflict) {
   pdl_wait();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= in.n * 12) return;
-  const int64_t i = t / 12;
-  const int e = (int)(t % 12);
-  const int d = kCE[2 * e] ^ kCE[2 * e + 1];
-  const int axis = d == 1 ? 0 : (d == 2 ? 1 : 2);
-  const int64_t a = corner_at(in, 8 * i + kCE[2 * e]), b = corner_at(in, 8 * i + kCE[2 * e + 1]);
-  const uint32_t oa = atomicCAS(&slots[6 * a + axis], kNoCorner, (uint32_t)b);
-  const uint32_t ob = atomicCAS(&slots[6 * b + 3 + axis], kNoCorner, (uint32_t)a);
-  if ((oa != kNoCorner && oa != (uint32_t)b) || (ob != kNoCorner && ob != (uint32_t)a)) *conflict = 1u;
+  if (t == 0) *conflict = 0u;
+  if (t < 6 * m) slots[t] = kNoCorner;
+  if (t < 3 * m) x[t] = deform ? fa(-1.0f, deform[t]) : -1.0f;
+}
+
+// The slot and the neighbour of corner c of a cube along an axis: an edge runs
+// from the corner with the axis' bit clear to the one with it set along x and z,
+// the other way along y (kCE), and the first endpoint keeps the second one in
+// its slots 0..2, the second endpoint the first one in 3..5.
+__device__ __forceinline__ int slot_of(int c, int axis) {
+  const bool set = (c >> axis) & 1;
+  return axis + ((axis == 1) == set ? 0 : 3);
+}
+
+// One thread per cube corner: the corner's position and its three neighbours in
+// the cube, by plain stores -- cubes of one grid store the same ones.  Whether
+// they did is checked afterwards: of two different values one is lost, and its
+// owner sees that.  (Claiming the 24 slots of a cube by compare-and-swap took
+// 21 us for 250,000 cubes; store and check take half of that.)
+__global__ void slot_store_kernel(DmcIn in, float ws, float* __restrict__ x, uint32_t* __restrict__ slots) {
+  pdl_wait();
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= in.n * 8) return;
+  const int64_t i = t >> 3;
+  const int c = (int)(t & 7);
+  const int64_t mi = corner_at(in, t);
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const float g = fa((float)in.vox[3 * i + a], (float)((c >> a) & 1));
+    float v = fsb(fm(g, ws), 1.0f);
+    if (in.deform) v = fa(v, in.deform[3 * mi + a]);
+    x[3 * mi + a] = v;
+    slots[6 * mi + slot_of(c, a)] = (uint32_t)corner_at(in, t ^ (1 << a));
+  }
+}
+
+__global__ void slot_check_kernel(DmcIn in, const uint32_t* __restrict__ slots, uint32_t* __restrict__ conflict) {
+  pdl_wait();
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= in.n * 8) return;
+  const int c = (int)(t & 7);
+  const int64_t mi = corner_at(in, t);
+  bool lost = false;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) lost = lost || slots[6 * mi + slot_of(c, a)] != (uint32_t)corner_at(in, t ^ (1 << a));
+  if (lost) *conflict = 1u;
 }
 
 __global__ void edge_adj_count_kernel(DmcIn in, uint32_t* __restrict__ cnt) {
@@ -2152,19 +2207,16 @@ extern "C" int a3d_dmc_corner_gradients(const a3d_dmc_inputs* p, void* workspace
   carve_grad(w, ws, n > 0 ? n : 1, m > 0 ? m : 1);
   A3D_REQUIRE(workspace && ws.ok(), A3D_ERR_WORKSPACE, "dmc_corner_gradients: workspace too small");
   if (m == 0) return A3D_OK;
-  A3D_TRY(fill_async<float>(gradients, 3 * m, 0.f, s));
-  if (n == 0) return A3D_OK;
+  if (n == 0) return fill_async<float>(gradients, 3 * m, 0.f, s);
   DmcIn in = make_in(p);
-  A3D_PDL(init_pos_kernel, dim3(gsz(m)), dim3(256), 0, s, m, p->deform, w.x, nullptr);
-  A3D_PDL(corner_pos_kernel, dim3(gsz(8 * n)), dim3(256), 0, s, in, 2.0f / (float)p->resolution, w.x);
   const int64_t nk = 12 * n;
-  A3D_TRY(fill_async<uint32_t>(w.slots, 6 * m, 0xffffffffu, s));
-  A3D_TRY(fill_async<uint32_t>(w.misc, 1, 0u, s));
-  A3D_PDL(edge_slot_kernel, dim3(gsz(nk)), dim3(256), 0, s, in, w.slots, w.misc);
+  A3D_PDL(slot_init_kernel, dim3(gsz(6 * m)), dim3(256), 0, s, m, p->deform, w.x, w.slots, w.misc);
+  A3D_PDL(slot_store_kernel, dim3(gsz(8 * n)), dim3(256), 0, s, in, 2.0f / (float)p->resolution, w.x, w.slots);
+  A3D_PDL(slot_check_kernel, dim3(gsz(8 * n)), dim3(256), 0, s, in, w.slots, w.misc);
   uint32_t conflict = 0;
   A3D_CUDA_TRY(cudaMemcpyAsync(&conflict, w.misc, sizeof(conflict), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
-  if (!conflict) {
+  if (!conflict) {  // after the read, so that it runs beside the caller's next host work
     A3D_PDL(corner_gradient_slots_kernel, dim3(gsz(m)), dim3(256), 0, s, in, w.x, w.slots, gradients);
     return A3D_OK;
   }
