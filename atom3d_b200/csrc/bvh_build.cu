@@ -73,7 +73,7 @@ struct BuildWs {
   uint32_t* visit;
   int32_t* work_a;
   int32_t* work_b;
-  uint32_t* counters;   // [kMaxLevels + 1] worklist sizes per level
+  uint32_t* counters;   // [kMaxLevels + 1] worklist sizes per level, then the first level of the grid launches
   WideNode* tmp_nodes;  // [N] wide node at the slot of its binary node
   uint32_t* lvl;        // [N] level of the wide node at a slot, kNoLevel if none
   uint32_t* lvl_alt;
@@ -114,7 +114,7 @@ size_t carve(BuildWs& w, Workspace& ws, int64_t n, int64_t m) {
   w.visit = ws.take<uint32_t>(n);
   w.work_a = ws.take<int32_t>(n);
   w.work_b = ws.take<int32_t>(n);
-  w.counters = ws.take<uint32_t>(kMaxLevels + 1);
+  w.counters = ws.take<uint32_t>(kMaxLevels + 2);
   w.tmp_nodes = ws.take<WideNode>(n);
   w.lvl = ws.take<uint32_t>(n);
   w.lvl_alt = ws.take<uint32_t>(n);
@@ -165,7 +165,7 @@ __global__ void init_kernel(const int64_t* __restrict__ face_off, int nmesh, int
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < 12 * (int64_t)nmesh) bounds[t] = (((t % 12) / 3) % 2 == 0) ? 0xffffffffu : 0u;
   if (t < 4) err[t] = 0;
-  if (t <= kMaxLevels) counters[t] = t == 0 ? (uint32_t)nmesh : 0u;
+  if (t <= kMaxLevels + 1) counters[t] = t == 0 ? (uint32_t)nmesh : 0u;
   if (t < nmesh) {
     const int64_t s = face_off[t], e = face_off[t + 1];
     if (e <= s) atomicExch(err, 1);
@@ -458,21 +458,51 @@ __device__ __forceinline__ void quantize_axis(float o, float s, float lo, float 
   qhi = (uint32_t)qh;
 }
 
-// 6. one collapse level: each worklist entry becomes a wide node at the slot
-// of its binary node; its internal children (binary node indices, which are
-// also their slots) form the next level's worklist
-__global__ void __launch_bounds__(kThreads)
-    collapse_level_kernel(int level, uint32_t* __restrict__ counters, const int32_t* __restrict__ cur,
-                          int32_t* __restrict__ nxt, int64_t n, int leaf_max, const int32_t* __restrict__ left,
-                          const int32_t* __restrict__ right, const int32_t* __restrict__ first,
-                          const int32_t* __restrict__ last, const float4* __restrict__ box_lo,
-                          const float4* __restrict__ box_hi, const uint32_t* __restrict__ dec,
-                          WideNode* __restrict__ tmp, uint32_t* __restrict__ lvl) {
-  pdl_wait();
-  const uint32_t cnt = counters[level];
-  const int nn = (int)n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x) {
-    const int b = cur[k];
+// 6. the collapse, level by level: each worklist entry becomes a wide node at
+// the slot of its binary node; its internal children (binary node indices, which
+// are also their slots) form the next level's worklist.  The first levels, while
+// they hold up to kHeadNodes nodes, are run by one block in one launch, the next
+// kGridLevels by the grid, one launch each, and what is left (nothing but the
+// ends of skewed trees) by one block again; a build of up to kHeadAll triangles
+// is one launch.  A level costs its nodes' serial chain (15 us), an empty launch
+// 2 us: against a launch a level up to kMaxLevels the build and queries of
+// 5,120 / 81,920 / 1,310,720 triangles took 743 / 1114 / 5061 instead of 788 /
+// 1154 / 5134 us (kHeadNodes 64: 755 / 1121 / 5067, 2048: 755 / 1129 / 5076).
+constexpr int kHeadThreads = 1024;
+constexpr uint32_t kHeadNodes = 256;
+constexpr int64_t kHeadAll = 2048;
+constexpr int kGridLevels = 12;
+
+struct Collapse {
+  uint32_t* counters;
+  int32_t* work[2];  // worklists of the even and the odd levels
+  int64_t n;
+  const int32_t* left;
+  const int32_t* right;
+  const int32_t* first;
+  const int32_t* last;
+  const float4* box_lo;
+  const float4* box_hi;
+  const uint32_t* dec;
+  WideNode* tmp;
+  uint32_t* lvl;
+};
+
+// this thread's nodes of a level, from `start` on, `stride` apart
+__device__ __forceinline__ void collapse_level(const Collapse& w, int level, uint32_t cnt, int64_t start,
+                                               int64_t stride) {
+  uint32_t* counters = w.counters;
+  const int32_t* cur = w.work[level & 1];
+  int32_t* nxt = w.work[(level + 1) & 1];
+  const int32_t *left = w.left, *right = w.right, *first = w.first, *last = w.last;
+  const float4 *box_lo = w.box_lo, *box_hi = w.box_hi;
+  const uint32_t* dec = w.dec;
+  WideNode* tmp = w.tmp;
+  uint32_t* lvl = w.lvl;
+  const int nn = (int)w.n;
+  for (int64_t k = start; k < cnt; k += stride) {
+    // past L1: the block that runs several levels wrote it itself
+    const int b = __ldcg(cur + k);
     int c[4];
     int nc;
     if (b >= nn) {  // a lone leaf as root (single-triangle mesh)
@@ -549,6 +579,29 @@ __global__ void __launch_bounds__(kThreads)
     tmp[slot] = nd;
     lvl[slot] = (uint32_t)level;
   }
+}
+
+// kHead: from level 0 while a level is small, noting where it stopped; else from
+// the level after the grid's to the last
+template <bool kHead>
+__global__ void __launch_bounds__(kHeadThreads) collapse_block_kernel(Collapse w, uint32_t head_nodes) {
+  pdl_wait();
+  int level = kHead ? 0 : (int)w.counters[kMaxLevels + 1] + kGridLevels;
+  for (; level < kMaxLevels; ++level) {
+    const uint32_t cnt = __ldcg(w.counters + level);
+    if (cnt == 0u || (kHead && cnt > head_nodes)) break;
+    collapse_level(w, level, cnt, threadIdx.x, kHeadThreads);
+    __syncthreads();
+  }
+  if (kHead && threadIdx.x == 0) w.counters[kMaxLevels + 1] = (uint32_t)level;
+}
+
+__global__ void __launch_bounds__(kThreads) collapse_grid_kernel(Collapse w, int step) {
+  pdl_wait();
+  const int level = (int)w.counters[kMaxLevels + 1] + step;
+  if (level >= kMaxLevels) return;
+  collapse_level(w, level, w.counters[level], (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                 (int64_t)gridDim.x * blockDim.x);
 }
 
 __global__ void depth_check_kernel(const uint32_t* counters, int32_t* err) {
@@ -712,7 +765,7 @@ int build_wide_bvh(const float* V, const int64_t* vert_off, const int32_t* F, co
                    float* bounds_out, int64_t* num_nodes_out, int32_t* status_out, BuildWs& w, cudaStream_t s) {
   const int mbits = mesh_bits_of(nmesh);
   const int bits = (64 - mbits) / 3 < 21 ? (64 - mbits) / 3 : 21;
-  const int64_t init_threads = 12ll * nmesh > kMaxLevels + 1 ? 12ll * nmesh : kMaxLevels + 1;
+  const int64_t init_threads = 12ll * nmesh > kMaxLevels + 2 ? 12ll * nmesh : kMaxLevels + 2;
   A3D_PDL(init_kernel, dim3((unsigned)ceil_div(init_threads, kThreads)), dim3(kThreads), 0, s, face_off, nmesh, n,
           w.bounds, w.err, w.counters, w.work_a);
   const unsigned g = (unsigned)ceil_div(n, kThreads);
@@ -744,17 +797,17 @@ int build_wide_bvh(const float* V, const int64_t* vert_off, const int32_t* F, co
           w.last, leaf_max, w.box_lo, w.box_hi, w.dp_cost, w.dp_dec, w.visit);
   A3D_PDL(write_tris_kernel, dim3(g), dim3(kThreads), 0, s, V, vert_off, F, face_off, w.mesh_of, order, n, tris_out);
 
-  // collapse: a fixed number of level launches (empty levels return at once)
   A3D_CUDA_TRY(cudaMemsetAsync(w.lvl, 0xff, sizeof(uint32_t) * n, s));
-  const int64_t level_blocks = (int64_t)num_sms() * 8;
-  const int64_t lb = ceil_div(n, kThreads) < level_blocks ? ceil_div(n, kThreads) : level_blocks;
-  int32_t *cur = w.work_a, *nxt = w.work_b;
-  for (int level = 0; level < kMaxLevels; ++level) {
-    A3D_PDL(collapse_level_kernel, dim3((unsigned)lb), dim3(kThreads), 0, s, level, w.counters, cur, nxt, n, leaf_max,
-            w.left, w.right, w.first, w.last, w.box_lo, w.box_hi, w.dp_dec, w.tmp_nodes, w.lvl);
-    int32_t* t = cur;
-    cur = nxt;
-    nxt = t;
+  const Collapse col{w.counters, {w.work_a, w.work_b}, n,        w.left,   w.right,     w.first,
+                     w.last,     w.box_lo,             w.box_hi, w.dp_dec, w.tmp_nodes, w.lvl};
+  A3D_PDL(collapse_block_kernel<true>, dim3(1), dim3(kHeadThreads), 0, s, col,
+          n > kHeadAll ? kHeadNodes : (uint32_t)kHeadAll);
+  if (n > kHeadAll) {
+    const int64_t level_blocks = (int64_t)num_sms() * 8;
+    const int64_t lb = ceil_div(n, kThreads) < level_blocks ? ceil_div(n, kThreads) : level_blocks;
+    for (int step = 0; step < kGridLevels; ++step)
+      A3D_PDL(collapse_grid_kernel, dim3((unsigned)lb), dim3(kThreads), 0, s, col, step);
+    A3D_PDL(collapse_block_kernel<false>, dim3(1), dim3(kHeadThreads), 0, s, col, 0u);
   }
   A3D_PDL(depth_check_kernel, dim3(1), dim3(32), 0, s, w.counters, w.err);
   // breadth-first layout: stable sort of the slots by level
