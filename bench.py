@@ -44,10 +44,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, HERE)
 
 METRIC = "UDF Mqueries/s (plain traversal, 1.31M-triangle mesh, 16M queries)"
-# DRAM read + write of one udf_task_kernel launch per query, measured by an
-# ncu capture of a 4,194,304-query launch on this mesh (1.471 GB); traffic
+# DRAM read + write of one udf_group_kernel launch per query, measured by an
+# ncu capture of a 4,194,304-query launch on this mesh (0.613 GB); traffic
 # scales with the query count (the tree stays in L2)
-DRAM_BYTES_PER_QUERY = 1.471343e9 / 4194304
+DRAM_BYTES_PER_QUERY = 0.612750e9 / 4194304
 TRAFFIC_SOURCE = "ncu dram__bytes_read.sum + dram__bytes_write.sum, 4,194,304-query capture scaled per query"
 UNIT = "Mqueries/s"
 WORKLOAD = "udf_large: icosphere L8 (1,310,720 tris) + 16 sinusoids, 16,777,216 mixed queries"
@@ -457,7 +457,7 @@ def main():
         achieved = per_q * n / (kernel_ms * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": DRAM_BYTES_PER_QUERY * n, "traffic_source": TRAFFIC_SOURCE, "peak_kind": peak_kind,
-                "bytes_per_query": per_q, "kernel": "udf_task_kernel", "kernel_ms": kernel_ms}
+                "bytes_per_query": per_q, "kernel": "udf_group_kernel", "kernel_ms": kernel_ms}
         # the tree (nodes + triangles, ~91 MB) stays in L2: the same bytes
         # against the L2 read bandwidth measured on this GPU
         l2 = l2_read_peak(dev)
