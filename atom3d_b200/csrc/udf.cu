@@ -713,6 +713,9 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
       for (int x = 1; x < kG; x <<= 1) next |= __shfl_xor_sync(FULL, next, x);
       if (at) {
         if (greedy) {
+          // every box distance overflows (infinite or huge queries): no child
+          // to descend to, so the query ends here and is re-run
+          greedy = have = q > 0;
           ref = next;
         } else if (q > 0) {
           if (sp + q - 1 > kGroupDepth && sp + q - 1 > capacity()) {

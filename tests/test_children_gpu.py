@@ -105,3 +105,28 @@ def test_flat_boxes_still_give_every_query_its_face(kind):
     for _ in range(3):
         for x, y in zip(first, b.query(q)):
             assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("leaf_max", [1, 8])
+@pytest.mark.parametrize("bounded", [False, True])
+def test_greedy_seed_ends_where_no_box_distance_is_finite(leaf_max, bounded):
+    """The greedy descent for a seed (NO_REUSE) on queries whose squared box
+    distances overflow or are NaN: the answer of the default seeding."""
+    v, f = mesh("smooth")
+    b = WideBVH(v.cuda(), f.cuda(), leaf_max=leaf_max)
+    inf, nan = float("inf"), float("nan")
+    odd = torch.tensor([[inf, 0, 0], [0, -inf, 0], [inf, inf, -inf], [1e30, 0, 0], [0, 2e19, -3e19], [3e38, 3e38, 3e38],
+                        [nan, 0, 0], [nan, nan, inf]])
+    g = torch.Generator().manual_seed(8)
+    q = torch.cat([odd, torch.rand(300, 3, generator=g) * 3 - 1.5, odd, odd[:1].expand(40, 3)]).contiguous().cuda()
+    ref = b.query(q)
+    seeding, bound = _lib.A3D_UDF_NO_REUSE, None
+    if bounded:
+        seeding |= _lib.A3D_UDF_BOUND_SEEDS
+        bound = torch.full((q.shape[0],), inf, device="cuda")
+        bound[::2] = 10.0
+    got = b.query(q, bound=bound, seeding=seeding)
+    has = ref[1] >= 0
+    assert not bool(has[:8].any()) and bool(has[8:308].all())
+    for x, y in zip((*ref[:3], ref[3][has]), (*got[:3], got[3][has])):
+        assert bool(((x == y) | ((x != x) & (y != y))).all())
