@@ -678,21 +678,28 @@ __global__ void test_bits_kernel(Geom g, const uint32_t* __restrict__ v, const i
   out[i] = r;
 }
 
-// plants the seed voxel and queues its brick for round 0 (list[0], cnt[0]);
-// status: 1 when the seed is occupied
+// Plants the seed voxel and queues its brick and the up to 26 around it for round
+// 0 (list, cnt[0]): a brick queues its neighbours for what its own visit changes,
+// which the seed never is, so those that the seed touches take it from their halo
+// in the first round.  status: 1 when the seed is occupied.  One warp.
 __global__ void seed_kernel(Geom g, const uint32_t* __restrict__ occ, uint32_t* __restrict__ water, int sx, int sy,
-                            int sz, uint32_t seed_brick, uint32_t* __restrict__ list, uint32_t* __restrict__ cnt,
+                            int sz, int nbx, int nby, uint32_t* __restrict__ list, uint32_t* __restrict__ cnt,
                             uint32_t* __restrict__ status) {
   pdl_wait();
+  const int lane = threadIdx.x;
   const int64_t i = widx(g, sx, sy, sz >> 5);
   const uint32_t bit = 1u << (sz & 31);
-  if (occ[i] & bit) {
-    status[0] = 1u;  // seed occupied
-  } else {
-    water[i] |= bit;
-    list[0] = seed_brick;
-    cnt[0] = 1u;
-    status[0] = 0u;
+  const bool occupied = (occ[i] & bit) != 0u;
+  const int bw = (sz >> 5) + lane / 9 - 1, bx = sx / kBX + (lane / 3) % 3 - 1, by = sy / kBY + lane % 3 - 1;
+  const bool queued = !occupied && lane < 27 && bw >= 0 && bw < g.nw && bx >= 0 && bx < nbx && by >= 0 && by < nby;
+  const unsigned m = __ballot_sync(0xffffffffu, queued);
+  if (queued) list[__popc(m & ((1u << lane) - 1u))] = (uint32_t)((bw * nbx + bx) * nby + by);
+  if (lane == 0) {
+    status[0] = occupied ? 1u : 0u;
+    if (!occupied) {
+      water[i] |= bit;
+      cnt[0] = (uint32_t)__popc(m);
+    }
   }
 }
 
@@ -824,12 +831,11 @@ extern "C" int a3d_flood_fill(const int64_t* dam_ijk, int64_t n, const a3d_flood
             sz = (int)(geom->seed[2] - geom->vol_lo[2]);
   A3D_REQUIRE(sx >= g.cx0 && sx <= g.cx1 && sy >= g.cy0 && sy <= g.cy1 && sz >= g.cz0 && sz <= g.cz1,
               A3D_ERR_ARGUMENT, "flood_fill: seed outside the crop");
-  // the queue of round 0 is the seed's brick; misc (queue counts included)
-  // was cleared above and mark starts at round 0 for every brick
-  const int64_t sb = ((int64_t)(sz >> 5) * nbx + sx / kBX) * nby + sy / kBY;
+  // misc (queue counts included) was cleared above and mark starts at round 0
+  // for every brick
   uint32_t* qcnt = w.misc + 2;
   A3D_CUDA_TRY(cudaMemsetAsync(w.mark, 0, nbricks * sizeof(uint32_t), s));
-  A3D_PDL(seed_kernel, dim3(1), dim3(1), 0, s, g, w.occ, w.water, sx, sy, sz, (uint32_t)sb, w.list_a, qcnt, w.misc);
+  A3D_PDL(seed_kernel, dim3(1), dim3(32), 0, s, g, w.occ, w.water, sx, sy, sz, nbx, nby, w.list_a, qcnt, w.misc);
   uint32_t seed_status = 0;
   A3D_CUDA_TRY(cudaMemcpyAsync(&seed_status, w.misc, 4, cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
