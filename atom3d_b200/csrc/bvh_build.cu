@@ -625,12 +625,15 @@ __global__ void layout_copy_kernel(const uint32_t* __restrict__ sorted_lvl, cons
   pdl_wait();
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
-  if ((sorted_lvl[r] & 0xffu) == kNoLevel) return;
+  const uint32_t level = sorted_lvl[r] & 0xffu;
+  if (level == kNoLevel) return;
   WideNode nd = tmp[sorted_slot[r]];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const uint32_t ref = nd.ref[j];
-    if (ref != 0xffffffffu && !ref_is_leaf(ref)) nd.ref[j] = newidx[ref];
+    // the inner children of the last level have no node (the status says so):
+    // an empty slot's reference, which names nothing
+    if (ref != 0xffffffffu && !ref_is_leaf(ref)) nd.ref[j] = level + 1 < kMaxLevels ? newidx[ref] : 0xffffffffu;
   }
   out[r] = nd;
 }

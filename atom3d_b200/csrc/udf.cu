@@ -152,6 +152,11 @@ struct TreeT {
     }
     return reinterpret_cast<const int4*>(nodes + ref);
   }
+  // whether the child of this reference has a disc that can be read (a leaf
+  // outside the arrays goes without; tri() records it)
+  __device__ __forceinline__ bool has_disc(uint32_t ref) const {
+    return ref_is_leaf(ref) ? !kGuard || leaf_first(ref) < num_tris : ref < num_children;
+  }
   __device__ __forceinline__ TriRec tri(uint32_t i) const {
     if (kGuard && i >= num_tris) {
       atomicOr(fault, kFaultTri);
@@ -470,7 +475,7 @@ __device__ __forceinline__ void node_child(const Tree& T, uint32_t ref, int c0, 
     }
 #pragma unroll
     for (int j = 0; j < kC; ++j)
-      if (d[j] < best && (ref_is_leaf(r[j]) || r[j] < T.num_children))
+      if (d[j] < best && T.has_disc(r[j]))
         e[j] = fmaxf(d[j], disc_dist_sq(ref_is_leaf(r[j]) ? T.children.leaf_discs + leaf_first(r[j])
                                                           : T.children.node_discs + r[j],
                                         px, py, pz));
