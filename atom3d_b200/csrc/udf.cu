@@ -1212,6 +1212,7 @@ extern "C" int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, c
   A3D_REQUIRE(num_points >= 0 && num_points < (1ll << 32), A3D_ERR_ARGUMENT, "udf: bad number of points");
   if (num_points == 0) return A3D_OK;
   A3D_REQUIRE(points && distances && face_ids && closest_points, A3D_ERR_ARGUMENT, "udf: null output");
+  A3D_REQUIRE(((uintptr_t)children & 31) == 0, A3D_ERR_ARGUMENT, "udf: child records must be 32-B aligned");
   if (sign) {
     A3D_REQUIRE(sign->face_normals && sign->faces, A3D_ERR_ARGUMENT, "udf: sign data needs face normals and faces");
     const bool all = sign->vertex_pn && sign->edge_pn && sign->he_edge_idx;
@@ -1373,6 +1374,7 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_childr
                   bvh->num_faces > 0 && bvh->num_faces < (1ll << 28),
               A3D_ERR_ARGUMENT, "batch_udf: invalid batch");
   A3D_REQUIRE(n >= 0 && n < (1ll << 40), A3D_ERR_ARGUMENT, "batch_udf: bad number of queries");
+  A3D_REQUIRE(((uintptr_t)children & 31) == 0, A3D_ERR_ARGUMENT, "batch_udf: child records must be 32-B aligned");
   A3D_REQUIRE(workspace, A3D_ERR_WORKSPACE, "batch_udf: no workspace");
   const int mbits = mesh_bits(bvh->num_meshes);
   A3D_REQUIRE(mbits <= 26, A3D_ERR_ARGUMENT, "batch_udf: too many meshes");
