@@ -63,6 +63,13 @@ _SIGNATURES: dict[str, tuple] = {
         c_int,
         [c_vp, c_i64, c_vp, c_i64, c_int, c_vp, c_i64, c_vp, c_vp, c_size, ctypes.POINTER(c_i64), c_fp, c_vp],
     ),
+    "a3d_bvh_build_children": (
+        c_int,
+        [
+            c_vp, c_i64, c_vp, c_i64, c_int, c_vp, c_i64, c_vp, c_vp, c_i64, c_vp, c_size, ctypes.POINTER(c_i64), c_fp,
+            c_vp,
+        ],
+    ),
     "a3d_mesh_normals_workspace_bytes": (c_size, [c_i64, c_i64]),
     "a3d_mesh_normals": (
         c_int,

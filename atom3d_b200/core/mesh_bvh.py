@@ -53,24 +53,39 @@ class WideBVH:
             ws = _lib.workspace(_lib.lib().a3d_bvh_build_workspace_bytes(nf), dev)
             nn = ctypes.c_int64(0)
             bounds = (ctypes.c_float * 6)()
+            # child records: decoded boxes and discs for the closest-point traversal
+            ccap = self._child_capacity(nf, self.leaf_max)
+            children = self._child_buffer(ccap, nf, dev)
             _lib.call(
-                "a3d_bvh_build", v.data_ptr(), v.shape[0], f.data_ptr(), nf, self.leaf_max, nodes.data_ptr(), cap,
-                tris.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(nn), bounds, _lib.stream_ptr(dev),
+                "a3d_bvh_build_children", v.data_ptr(), v.shape[0], f.data_ptr(), nf, self.leaf_max, nodes.data_ptr(),
+                cap, tris.data_ptr(), children.data_ptr(), ccap, ws.data_ptr(), ws.numel(), ctypes.byref(nn), bounds,
+                _lib.stream_ptr(dev),
             )
             self.num_nodes = int(nn.value)
+            if self.num_nodes > ccap:
+                children = self._child_buffer(self.num_nodes, nf, dev)
+                _lib.call("a3d_bvh_children", nodes.data_ptr(), tris.data_ptr(), self.num_nodes, None, nf,
+                          children.data_ptr(), _lib.stream_ptr(dev))
+                torch.cuda.current_stream(dev).synchronize()
             self.nodes = nodes[: self.num_nodes * 64]
             self.tris = tris
-            # child records: decoded boxes and discs for the closest-point traversal
-            self.children = torch.empty(_lib.lib().a3d_bvh_children_bytes(self.num_nodes, nf), dtype=torch.uint8,
-                                        device=dev)
-            _lib.call("a3d_bvh_children", self.nodes.data_ptr(), self.tris.data_ptr(), self.num_nodes, None, nf,
-                      self.children.data_ptr(), _lib.stream_ptr(dev))
+            self.children = children
         self.lo = [bounds[0], bounds[1], bounds[2]]
         self.hi = [bounds[3], bounds[4], bounds[5]]
         self._view = _lib.BvhView(
             self.nodes.data_ptr(), self.tris.data_ptr(), self.num_nodes, self.num_tris,
             (ctypes.c_float * 3)(*self.lo), (ctypes.c_float * 3)(*self.hi),
         )
+
+    @staticmethod
+    def _child_capacity(nf: int, leaf_max: int) -> int:
+        """Nodes to hold child records for, before the tree is known: leaves of
+        up to 8 triangles make about nf / 12 nodes, of one triangle nf / 3."""
+        return nf // (8 if leaf_max >= 8 else 2) + 64
+
+    @staticmethod
+    def _child_buffer(nodes: int, nf: int, dev) -> torch.Tensor:
+        return torch.empty(_lib.lib().a3d_bvh_children_bytes(nodes, nf), dtype=torch.uint8, device=dev)
 
     @property
     def view(self) -> _lib.BvhView:
@@ -99,9 +114,9 @@ class WideBVH:
             if b.shape[0] != n:
                 raise ValueError("bound must have one entry per query")
         _lib.call(
-            "a3d_udf_children", ctypes.byref(self._view), self.children.data_ptr(), p.data_ptr(), n, dist.data_ptr(), fid.data_ptr(), cp.data_ptr(),
-            _lib.ptr(uvw), ctypes.byref(sign) if sign is not None else None, _lib.ptr(b), _lib.ptr(stats), flags,
-            ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev),
+            "a3d_udf_children", ctypes.byref(self._view), self.children.data_ptr(), p.data_ptr(), n, dist.data_ptr(),
+            fid.data_ptr(), cp.data_ptr(), _lib.ptr(uvw), ctypes.byref(sign) if sign is not None else None,
+            _lib.ptr(b), _lib.ptr(stats), flags, ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev),
         )
         return dist, fid, cp, uvw
 

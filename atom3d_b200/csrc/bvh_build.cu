@@ -33,6 +33,7 @@
 #include <math.h>
 #include <string.h>
 
+#include "bvh_children.cuh"
 #include "bvh_layout.cuh"
 #include "bvh_sah.cuh"
 #include "primitives.cuh"
@@ -842,7 +843,16 @@ extern "C" size_t a3d_bvh_build_workspace_bytes(int64_t num_faces) {
 extern "C" int a3d_bvh_build(const float* vertices, int64_t num_vertices, const int32_t* faces, int64_t num_faces,
                              int leaf_max, void* nodes_out, int64_t node_capacity, void* tris_out, void* workspace,
                              size_t workspace_bytes, int64_t* num_nodes_out, float* bounds_out,
-                             a3d_stream_t stream_) {
+                             a3d_stream_t stream) {
+  return a3d_bvh_build_children(vertices, num_vertices, faces, num_faces, leaf_max, nodes_out, node_capacity, tris_out,
+                                nullptr, 0, workspace, workspace_bytes, num_nodes_out, bounds_out, stream);
+}
+
+extern "C" int a3d_bvh_build_children(const float* vertices, int64_t num_vertices, const int32_t* faces,
+                                      int64_t num_faces, int leaf_max, void* nodes_out, int64_t node_capacity,
+                                      void* tris_out, void* children_out, int64_t children_capacity, void* workspace,
+                                      size_t workspace_bytes, int64_t* num_nodes_out, float* bounds_out,
+                                      a3d_stream_t stream_) {
   cudaStream_t s = (cudaStream_t)stream_;
   A3D_REQUIRE(num_faces > 0 && num_vertices > 0, A3D_ERR_ARGUMENT, "bvh_build: empty mesh");
   A3D_REQUIRE(num_faces < (1ll << 28), A3D_ERR_ARGUMENT, "bvh_build: more than 2^28 faces");
@@ -850,6 +860,8 @@ extern "C" int a3d_bvh_build(const float* vertices, int64_t num_vertices, const 
               "bvh_build: null pointer");
   A3D_REQUIRE(((uintptr_t)nodes_out & 63) == 0 && ((uintptr_t)tris_out & 15) == 0, A3D_ERR_ARGUMENT,
               "bvh_build: nodes must be 64-B and triangles 16-B aligned");
+  A3D_REQUIRE(!children_out || (((uintptr_t)children_out & 31) == 0 && children_capacity > 0), A3D_ERR_ARGUMENT,
+              "bvh_build: child records must be 32-B aligned and have a capacity");
   const int64_t n = num_faces;
   A3D_REQUIRE(node_capacity >= n, A3D_ERR_WORKSPACE, "bvh_build: node capacity must be at least num_faces");
   Workspace ws(workspace, workspace_bytes);
@@ -861,6 +873,9 @@ extern "C" int a3d_bvh_build(const float* vertices, int64_t num_vertices, const 
   A3D_PDL(single_offsets_kernel, dim3(1), dim3(32), 0, s, w.face_off, w.vert_off, n, num_vertices);
   A3D_TRY(build_wide_bvh(vertices, w.vert_off, faces, w.face_off, 1, n, leaf_max, (WideNode*)nodes_out,
                          (TriRec*)tris_out, nullptr, nullptr, w.count, nullptr, w, s));
+  // before the wait below, so that they are as finished as the tree when this returns
+  if (children_out)
+    A3D_TRY(launch_children(nodes_out, tris_out, children_capacity, w.count, true, n, children_out, s));
   uint32_t hb[12];
   int32_t herr[4];
   int64_t count = 0;

@@ -35,13 +35,21 @@ __device__ __forceinline__ float warp_max(float v) { return -warp_min(-v); }
 // to the last of its rightmost one.
 __global__ void __launch_bounds__(kChildThreads)
     child_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris, int64_t num_nodes,
-                const int64_t* __restrict__ num_nodes_dev, int64_t num_tris, BoxRec* __restrict__ boxes,
-                 DiscRec* __restrict__ node_discs, DiscRec* __restrict__ leaf_discs) {
+                 const int64_t* __restrict__ num_nodes_dev, bool by_count, int64_t num_tris, void* children) {
   pdl_wait();
   const int lane = threadIdx.x & 31;
-  // num_nodes is a capacity when the count is on the device: nodes past it
-  // have no boxes and no disc, the leaves under them still do
+  // num_nodes is a capacity when the count is on the device.  The records are
+  // laid out for it (nodes past it have no boxes and no disc, the leaves under
+  // them still do), or, by_count, for the count, and left out if they do not fit
   const int64_t count = num_nodes_dev != nullptr ? *num_nodes_dev : num_nodes;
+  if (by_count) {
+    if (count > num_nodes) return;
+    num_nodes = count;
+  }
+  const ChildRecs cr(children, num_nodes);
+  BoxRec* __restrict__ boxes = const_cast<BoxRec*>(cr.boxes);
+  DiscRec* __restrict__ node_discs = const_cast<DiscRec*>(cr.node_discs);
+  DiscRec* __restrict__ leaf_discs = const_cast<DiscRec*>(cr.leaf_discs);
   const int64_t warps = (int64_t)gridDim.x * (kChildThreads / 32);
   for (int64_t w = ((int64_t)blockIdx.x * kChildThreads + threadIdx.x) >> 5; w < 4 * count; w += warps) {
     const WideNode* nd = nodes + (w >> 2);
@@ -156,6 +164,17 @@ __global__ void __launch_bounds__(kChildThreads)
 }
 
 }  // namespace
+
+int launch_children(const void* nodes, const void* tris, int64_t num_nodes, const int64_t* num_nodes_device,
+                    bool by_count, int64_t num_tris, void* children_out, cudaStream_t s) {
+  A3D_REQUIRE(((uintptr_t)children_out & 31) == 0, A3D_ERR_ARGUMENT, "bvh_children: records must be 32-B aligned");
+  const int64_t want = ceil_div(4 * num_nodes, kChildThreads / 32);
+  const int64_t cap = (int64_t)num_sms() * 32;
+  A3D_PDL(child_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(kChildThreads), 0, s, (const WideNode*)nodes,
+          (const TriRec*)tris, num_nodes, num_nodes_device, by_count, num_tris, children_out);
+  return A3D_OK;
+}
+
 }  // namespace a3d
 
 using namespace a3d;
@@ -169,12 +188,5 @@ extern "C" int a3d_bvh_children(const void* nodes, const void* tris, int64_t num
                              int64_t num_tris, void* children_out, a3d_stream_t stream) {
   A3D_REQUIRE(nodes && tris && children_out && num_nodes > 0 && num_tris > 0, A3D_ERR_ARGUMENT,
               "bvh_children: invalid bvh");
-  A3D_REQUIRE(((uintptr_t)children_out & 31) == 0, A3D_ERR_ARGUMENT, "bvh_children: records must be 32-B aligned");
-  const ChildRecs cr(children_out, num_nodes);
-  const int64_t want = ceil_div(4 * num_nodes, kChildThreads / 32);
-  const int64_t cap = (int64_t)num_sms() * 32;
-  A3D_PDL(child_kernel, dim3((unsigned)(want < cap ? want : cap)), dim3(kChildThreads), 0, (cudaStream_t)stream,
-          (const WideNode*)nodes, (const TriRec*)tris, num_nodes, num_nodes_device, num_tris,
-          const_cast<BoxRec*>(cr.boxes), const_cast<DiscRec*>(cr.node_discs), const_cast<DiscRec*>(cr.leaf_discs));
-  return A3D_OK;
+  return launch_children(nodes, tris, num_nodes, num_nodes_device, false, num_tris, children_out, (cudaStream_t)stream);
 }

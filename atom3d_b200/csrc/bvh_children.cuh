@@ -54,6 +54,12 @@ struct ChildRecs {
         leaf_discs(node_discs + num_nodes) {}
 };
 
+// Launches the pass that writes the records of a finished tree.  num_nodes: the
+// tree's nodes, or a capacity with the count in *num_nodes_device; laid out for
+// num_nodes or, by_count, for the count (nothing is written past the capacity).
+int launch_children(const void* nodes, const void* tris, int64_t num_nodes, const int64_t* num_nodes_device,
+                    bool by_count, int64_t num_tris, void* children_out, cudaStream_t s);
+
 // Rounding allowance of a disc distance, relative to |q| (q the query
 // relative to the disc's centre): the bound's own error (about 10 ulp) and
 // that of the triangle tests it stands in for (the point they evaluate lies

@@ -81,6 +81,19 @@ int a3d_bvh_children(const void* nodes, const void* tris, int64_t num_nodes,
                   const int64_t* num_nodes_device, int64_t num_tris, void* children_out,
                   a3d_stream_t stream);
 
+/* a3d_bvh_build with the tree's child records, written before the call's own
+ * wait: the tree and its records are finished when it returns.  children_out
+ * (nullable): a3d_bvh_children_bytes(children_capacity, num_faces) bytes, 32-B
+ * aligned; the records are laid out for *num_nodes_out nodes.  A tree of more
+ * than children_capacity nodes gets none (a3d_bvh_children writes them then). */
+int a3d_bvh_build_children(const float* vertices, int64_t num_vertices,
+                  const int32_t* faces, int64_t num_faces, int leaf_max,
+                  void* nodes_out, int64_t node_capacity, void* tris_out,
+                  void* children_out, int64_t children_capacity,
+                  void* workspace, size_t workspace_bytes, int64_t* num_nodes_out,
+                  float* bounds_out /* host, 6 floats: lo xyz, hi xyz */,
+                  a3d_stream_t stream);
+
 /* ---- pseudo-normal precompute for the SDF sign -------------------------- */
 /* Replaces MeshBVH._precompute_face_normals and
  * MeshBVH._precompute_pseudo_normal_data (atom3d/core/mesh_bvh.py:129-232).
