@@ -50,12 +50,14 @@ __global__ void __launch_bounds__(kChildThreads)
   BoxRec* __restrict__ boxes = const_cast<BoxRec*>(cr.boxes);
   DiscRec* __restrict__ node_discs = const_cast<DiscRec*>(cr.node_discs);
   DiscRec* __restrict__ leaf_discs = const_cast<DiscRec*>(cr.leaf_discs);
+  const DiscRec no_disc{0.f, 0.f, 0.f, INFINITY, 0.f, 0.f, 1.f, INFINITY};
+  if (blockIdx.x == 0 && threadIdx.x == 0) leaf_discs[num_tris] = no_disc;
   const int64_t warps = (int64_t)gridDim.x * (kChildThreads / 32);
   for (int64_t w = ((int64_t)blockIdx.x * kChildThreads + threadIdx.x) >> 5; w < 4 * count; w += warps) {
     const WideNode* nd = nodes + (w >> 2);
     const int c = (int)(w & 3);
     BoxRec box{INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY, 0xffffffffu, 0u};
-    DiscRec disc{0.f, 0.f, 0.f, INFINITY, 0.f, 0.f, 1.f, INFINITY};
+    DiscRec disc = no_disc;
     int64_t leaf_at = -1, node_at = -1;
     if (c < (int)(nd->meta >> 24)) {
       const uint32_t r = nd->ref[c];
@@ -68,7 +70,9 @@ __global__ void __launch_bounds__(kChildThreads)
       box.hx = dequant(nd->q[3], c, sx, nd->ox);
       box.hy = dequant(nd->q[4], c, sy, nd->oy);
       box.hz = dequant(nd->q[5], c, sz, nd->oz);
-      box.ref = r;
+      box.ref = (ref_is_leaf(r) ? leaf_first(r) + leaf_count(r) <= (uint64_t)num_tris : r < (uint64_t)count)
+                    ? r
+                    : make_leaf_ref((uint32_t)num_tris, 1u);
       for (int x = 1; x < 4; ++x) box.ties |= nd->ref[c ^ x] < r ? 1u << (x - 1) : 0u;
       if (ref_is_leaf(r)) {
         if (leaf_first(r) < (uint64_t)num_tris) leaf_at = leaf_first(r);
@@ -181,7 +185,7 @@ using namespace a3d;
 
 extern "C" size_t a3d_bvh_children_bytes(int64_t num_nodes, int64_t num_tris) {
   return (size_t)(num_nodes > 0 ? num_nodes : 0) * (4 * sizeof(BoxRec) + sizeof(DiscRec)) +
-         (size_t)(num_tris > 0 ? num_tris : 0) * sizeof(DiscRec);
+         (size_t)(num_tris > 0 ? num_tris + 1 : 1) * sizeof(DiscRec);
 }
 
 extern "C" int a3d_bvh_children(const void* nodes, const void* tris, int64_t num_nodes, const int64_t* num_nodes_device,

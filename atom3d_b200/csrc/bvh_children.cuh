@@ -20,8 +20,10 @@
 //                           dequant() gives, so box distances are the same)
 //   uint32 ref, ties        the node's reference, 0xffffffff for no child;
 //                           bit x - 1 set when sibling c ^ x's is smaller
+//                           (a reference to no node or triangle of the tree
+//                           is stored as the leaf of one triangle at num_tris)
 // DiscRec (32 B, one load), one per wide node and one per leaf, the latter at
-// the place of the leaf's first triangle:
+// the place of the leaf's first triangle, and one more at num_tris:
 //   float cx, cy, cz, rho   centre and radius of the disc
 //   float nx, ny, nz, h     unit normal and half thickness
 // rho and h are widened by their rounding error; rho = +inf for no disc.

@@ -133,7 +133,9 @@ __device__ __forceinline__ TriRec load_tri(const TriRec* tris, uint32_t i) {
 // The arrays a traversal reads.  With kGuard (batches, whose node count is
 // only known on the device) a node or triangle index outside the arrays is
 // recorded in *fault (kFaultNode / kFaultTri) and replaced by 0, so no
-// access leaves them whatever the tree holds.
+// access leaves them whatever the tree holds.  The child records hold no
+// reference outside the arrays (child_kernel): a bad one is there the leaf at
+// num_tris, which has a disc of its own and is recorded by the triangle read.
 constexpr uint32_t kFaultNode = 1u, kFaultTri = 2u;
 
 template <bool kGuard>
@@ -151,11 +153,6 @@ struct TreeT {
       ref = 0;
     }
     return reinterpret_cast<const int4*>(nodes + ref);
-  }
-  // whether the child of this reference has a disc that can be read (a leaf
-  // outside the arrays goes without; tri() records it)
-  __device__ __forceinline__ bool has_disc(uint32_t ref) const {
-    return ref_is_leaf(ref) ? !kGuard || leaf_first(ref) < num_tris : ref < num_children;
   }
   __device__ __forceinline__ TriRec tri(uint32_t i) const {
     if (kGuard && i >= num_tris) {
@@ -475,7 +472,7 @@ __device__ __forceinline__ void node_child(const Tree& T, uint32_t ref, int c0, 
     }
 #pragma unroll
     for (int j = 0; j < kC; ++j)
-      if (d[j] < best && T.has_disc(r[j]))
+      if (d[j] < best && (ref_is_leaf(r[j]) || r[j] < T.num_children))
         e[j] = fmaxf(d[j], disc_dist_sq(ref_is_leaf(r[j]) ? T.children.leaf_discs + leaf_first(r[j])
                                                           : T.children.node_discs + r[j],
                                         px, py, pz));
