@@ -598,45 +598,13 @@ __device__ __forceinline__ int parity_vote(int k, float coalesce, Hit hit) {
   return ((sc < 0 ? -sc : sc) % 2) == 1 ? 1 : 0;
 }
 
-// one ray with deep local buffers, for the rays that outgrow the shared ones
-__device__ __noinline__ int parity_slow(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris, V3 o,
-                                        V3 d, float max_t, float coalesce, uint32_t* __restrict__ overflow) {
-  float ts[kParityCap];
-  int8_t sg[kParityCap];
-  const Ray r = make_ray(o, d);
-  int k = 0;
-  bool lost = false;
-  if (!all_hits(nodes, tris, r, max_t, [&](float th, const Tri&, int s) {
-        // insertion by t keeps the buffer sorted
-        if (k >= kParityCap) {
-          lost = true;
-          return;
-        }
-        int j = k;
-        while (j > 0 && ts[j - 1] > th) {
-          ts[j] = ts[j - 1];
-          sg[j] = sg[j - 1];
-          --j;
-        }
-        ts[j] = th;
-        sg[j] = (int8_t)s;
-        ++k;
-      }))
-    lost = true;
-  if (lost) atomicExch(overflow, 1u);
-  return parity_vote(k, coalesce, [&](int j, float& t, int& s) {
-    t = ts[j];
-    s = sg[j];
-  });
-}
-
 // One (direction, point) ray a lane, directions outermost so that a warp's rays
 // are parallel; phases as in ray_nearest_kernel, visits in any order.  A ray's
-// hits (t, the sign bit for hits from the front) and stack stay in shared
-// memory; one that outgrows either is done again by parity_slow.  votes[i]
-// (zeroed before) counts the point's odd rays.  100,000 points, 8 directions,
-// 200,000 triangles: 1.38 ms with a thread per point and its directions in
-// turn, 0.55 ms so.
+// first hits (t, the sign bit for hits from the front) and stack entries stay in
+// shared memory, the rest in local memory; the hits of a ray with more than
+// kParityHits are sorted by the whole warp.  votes[i] (zeroed before) counts the
+// point's odd rays.  100,000 points, 8 directions, 200,000 triangles: 1.38 ms
+// with a thread per point and its directions in turn, 0.55 ms so.
 constexpr int kParityHits = 12;
 constexpr int kParityStack = 24;
 
@@ -644,8 +612,10 @@ struct ParitySmem {
   uint32_t stack[kParityStack][32];
   float hits[kParityHits][32];
   uint2 own[32];
-  float trid[kMaxLeafTris * kTriRow];
+  float trid[kMaxLeafTris * kTriRow];  // between leaf steps: the hits to sort
+  float sorted[kParityCap];
 };
+static_assert(kMaxLeafTris * kTriRow >= kParityCap, "a ray's hits fit the leaf step's results");
 
 __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
     ray_parity_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
@@ -660,12 +630,19 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
   const int64_t rays = n * ndir;
   const float lim = max_t * kPruneSlack;
   int64_t pos = 0, end = 0;
-  bool exhausted = false, live = false, slow = false;
+  bool exhausted = false, live = false, lost = false;
   int64_t i = 0;
   int dir = 0, sp = 0, nh = 0;
   uint32_t ref = kNoItem;
   Ray r{};
+  float more_hits[kParityCap - kParityHits];
+  uint32_t more_stack[kAllDepth - kParityStack];
 
+  auto pop = [&]() -> uint32_t {
+    if (sp == 0) return kNoItem;
+    --sp;
+    return sp < kParityStack ? S.stack[sp][lane] : more_stack[sp - kParityStack];
+  };
   auto distribute = [&](unsigned want) {
     while (want) {
       if (pos >= end) {
@@ -689,7 +666,6 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
         r = make_ray(ld3(pts, i), ld3(dirs, dir));
         sp = 0;
         nh = 0;
-        slow = false;
         ref = 0u;
         live = true;
       }
@@ -714,12 +690,12 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
           if (tc[c] <= lim) {
             if (next != kNoItem) {
               if (sp < kParityStack) S.stack[sp++][lane] = next;
-              else slow = true;
+              else if (sp < kAllDepth) more_stack[sp++ - kParityStack] = next;
+              else lost = true;
             }
             next = rc[c];
           }
-        if (next == kNoItem && sp > 0) next = S.stack[--sp][lane];
-        ref = slow ? kNoItem : next;
+        ref = next == kNoItem ? pop() : next;
       }
     }
     // (b) leaf step
@@ -764,42 +740,66 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
           const float t = S.trid[k * kTriRow + lane];
           if (t < INFINITY) {
             if (nh < kParityHits) S.hits[nh++][lane] = t;
-            else slow = true;
+            else if (nh < kParityCap) more_hits[nh++ - kParityHits] = t;
+            else lost = true;
           }
         }
-        ref = !slow && sp > 0 ? S.stack[--sp][lane] : kNoItem;
+        ref = pop();
       }
       __syncwarp();
     }
     // (c) finished rays vote, new ones
-    if (live && ref == kNoItem) {
-      int vote;
-      if (slow) {
-        vote = parity_slow(nodes, tris, r.o, r.d, max_t, coalesce, overflow);
-      } else {
-        // insertion sort by t
-        for (int k = 1; k < nh; ++k) {
-          const float t = S.hits[k][lane];
-          int j = k;
-          while (j > 0 && fabsf(S.hits[j - 1][lane]) > fabsf(t)) {
-            S.hits[j][lane] = S.hits[j - 1][lane];
-            --j;
-          }
-          S.hits[j][lane] = t;
+    const bool done = live && ref == kNoItem;
+    bool vote = false;
+    if (done && nh <= kParityHits) {
+      // insertion sort by t
+      for (int k = 1; k < nh; ++k) {
+        const float t = S.hits[k][lane];
+        int j = k;
+        while (j > 0 && fabsf(S.hits[j - 1][lane]) > fabsf(t)) {
+          S.hits[j][lane] = S.hits[j - 1][lane];
+          --j;
         }
-        vote = parity_vote(nh, coalesce, [&](int j, float& t, int& sg) {
-          const float h = S.hits[j][lane];
-          t = fabsf(h);
-          sg = h < 0.f ? -1 : 1;
-        });
+        S.hits[j][lane] = t;
       }
+      vote = parity_vote(nh, coalesce, [&](int j, float& t, int& sg) {
+        const float h = S.hits[j][lane];
+        t = fabsf(h);
+        sg = h < 0.f ? -1 : 1;
+      });
+    }
+    for (unsigned m = __ballot_sync(FULL, done && nh > kParityHits); m; m &= m - 1u) {
+      // the warp sorts one ray's hits: each goes to its rank
+      const int o = __ffs(m) - 1, k = __shfl_sync(FULL, nh, o);
+      if (lane == o)
+        for (int j = kParityHits; j < k; ++j) S.trid[j] = more_hits[j - kParityHits];
+      if (lane < kParityHits) S.trid[lane] = S.hits[lane][o];
+      __syncwarp();
+      for (int e = lane; e < k; e += 32) {
+        const float t = S.trid[e];
+        int rank = 0;
+        for (int j = 0; j < k; ++j) {
+          const float u = fabsf(S.trid[j]);
+          rank += u < fabsf(t) || (u == fabsf(t) && j < e) ? 1 : 0;
+        }
+        S.sorted[rank] = t;
+      }
+      __syncwarp();
+      if (lane == o)
+        vote = parity_vote(k, coalesce, [&](int j, float& t, int& sg) {
+          t = fabsf(S.sorted[j]);
+          sg = S.sorted[j] < 0.f ? -1 : 1;
+        });
+      __syncwarp();
+    }
+    if (done) {
       if (vote) atomicAdd(&votes[i], 1);
       live = false;
-      slow = false;
     }
     const unsigned free_lanes = __ballot_sync(FULL, !live);
     if (!exhausted || pos < end) distribute(free_lanes);
   }
+  if (lost) atomicExch(overflow, 1u);  // more hits or stack entries than a ray keeps
 }
 
 }  // namespace
