@@ -247,9 +247,17 @@ inline int radix_items(int64_t n) {
 inline int64_t radix_num_tiles(int64_t n) {
   return ceil_div(n > 0 ? n : 1, (int64_t)radix_items(n) * kRsThreads);
 }
-// uint32 elements of scratch needed by radix_sort_pairs
+// uint32 elements of scratch needed by radix_sort_pairs, for n keys and for any
+// smaller sort (just below a change of the keys a thread, fewer keys take more
+// tiles), so that a workspace for n serves every smaller call
 inline size_t radix_sort_scratch_elems(int64_t n) {
-  const int64_t h = 256 * radix_num_tiles(n);
+  int64_t tiles = radix_num_tiles(n);
+  for (int items = 2; items < kRsMaxItems; items *= 2) {
+    const int64_t below = items == 2 ? kRsFuseTiles * 2 * kRsThreads : (int64_t)items * kRsThreads * 296 - 1;
+    const int64_t t = radix_num_tiles(below);
+    if (n > below && tiles < t) tiles = t;
+  }
+  const int64_t h = 256 * tiles;
   return (size_t)h + scan_workspace_elems(h);
 }
 
