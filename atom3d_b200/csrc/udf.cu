@@ -517,8 +517,14 @@ __device__ __forceinline__ void node_child(const Tree& T, uint32_t ref, int c0, 
 // leaf (or test their seed triangle).  Every query keeps the nearest-first
 // order of traverse(), so results and ties are those of a single walk.
 constexpr int kGroupWarps = 4;
-constexpr int kGroupDepth = 24;  // stack entries of a query in shared memory
-constexpr int kSpillCap = 64;    // further entries in the workspace
+// stack entries of a query in shared memory, and further ones in the workspace
+// where it has room.  The boxes alone prune less, so that stacks go deeper:
+// 1,048,576 queries (1,310,720 triangles) without room in the workspace, where a
+// query with more entries is run again, took 105 ms at 24 entries, 36.7 at 32
+// and 25.6 at 40
+template <bool kRecords>
+constexpr int kGroupDepth = kRecords ? 24 : 40;
+constexpr int kSpillCap = 64;
 constexpr int kMaxPool = 64;
 constexpr uint32_t kReuseSpan = 64;  // a group's previous result seeds a query this close in the sorted order
 // resident blocks an SM (48 registers at 4 lanes, 64 at 2, no spills in the
@@ -531,9 +537,9 @@ constexpr int kGroupBlocks = kG == 4 ? 10 : 8;
 template <int kG>
 constexpr int kNodeGroups = kG == 4 ? 5 : 10;
 
-template <int kG>
+template <int kG, bool kRecords>
 struct GroupSmem {
-  uint2 stack[32 / kG][kGroupDepth];
+  uint2 stack[32 / kG][kGroupDepth<kRecords>];
   uint2 own[32 / kG];                     // a leaf step's queries: first triangle less its first task, first lane
   float trid[32 / kG * kMaxLeafTris];     // distances by task
 };
@@ -552,10 +558,11 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
   pdl_wait();
   constexpr int kC = 4 / kG;  // children a lane
   constexpr unsigned lead = kG == 4 ? 0x11111111u : 0x55555555u, gmask = (1u << kG) - 1u;
-  __shared__ GroupSmem<kG> smem[kGroupWarps];
+  constexpr int kDepth = kGroupDepth<kRecords>;
+  __shared__ GroupSmem<kG, kRecords> smem[kGroupWarps];
   const int lane = threadIdx.x & 31, c = lane & (kG - 1), base = lane & ~(kG - 1);
   const unsigned FULL = 0xffffffffu;
-  GroupSmem<kG>& S = smem[threadIdx.x >> 5];
+  GroupSmem<kG, kRecords>& S = smem[threadIdx.x >> 5];
   uint2* stack = S.stack[lane / kG];
   // persistent warps: pools of consecutive (sorted) queries are taken from a
   // global counter; inside a pool, groups take queries as they finish
@@ -573,16 +580,16 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
   int sp = 0;
   unsigned long long rounds = 0;
 
-  // entry i >= kGroupDepth of the query's stack, in the workspace, and the
-  // stack's capacity: kGroupDepth, and kSpillCap more where the workspace has
+  // entry i >= kDepth of the query's stack, in the workspace, and the
+  // stack's capacity: kDepth, and kSpillCap more where the workspace has
   // room for this group
   auto spill_at = [&](int i) -> uint2* {
     const uint32_t owner = (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / kG;
-    return spill + (size_t)owner * kSpillCap + (i - kGroupDepth);
+    return spill + (size_t)owner * kSpillCap + (i - kDepth);
   };
   auto capacity = [&]() -> int {
     const uint32_t owner = (blockIdx.x * (kGroupWarps * 32) + threadIdx.x) / kG;
-    return owner < spill_owners ? kGroupDepth + kSpillCap : kGroupDepth;
+    return owner < spill_owners ? kDepth + kSpillCap : kDepth;
   };
 
   auto start = [&](uint32_t knew) {
@@ -647,7 +654,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
     while (__any_sync(FULL, need)) {
       uint2 t = make_uint2(0u, 0x7f800000u);
       const int i = sp - 1 - c;
-      if (need && i >= 0) t = i < kGroupDepth ? stack[i] : *spill_at(i);
+      if (need && i >= 0) t = i < kDepth ? stack[i] : *spill_at(i);
       const bool good = need && i >= 0 && __uint_as_float(t.y) < best_sq;
       const unsigned gm = (__ballot_sync(FULL, good) >> base) & gmask;
       const int f = __ffs(gm) - 1;
@@ -720,7 +727,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
           greedy = have = q > 0;
           ref = next;
         } else if (q > 0) {
-          if (sp + q - 1 > kGroupDepth && sp + q - 1 > capacity()) {
+          if (sp + q - 1 > kDepth && sp + q - 1 > capacity()) {
             // no room: the deep-stack kernel re-runs the query
             phase = kAbandon;
             have = false;
@@ -729,7 +736,7 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
             for (int j = 0; j < kC; ++j) {
               const int i = sp + q - 1 - rank[j];
               if (ok[j] && rank[j] > 0) {
-                if (i < kGroupDepth) stack[i] = make_uint2(r[j], __float_as_uint(e[j]));
+                if (i < kDepth) stack[i] = make_uint2(r[j], __float_as_uint(e[j]));
                 else *spill_at(i) = make_uint2(r[j], __float_as_uint(e[j]));
               }
             }
@@ -1099,19 +1106,25 @@ int launch_groups(const TreeT<kBatch>& T, const float* pts, int64_t n, const uin
 // meshes with 8.7M: 23.8 against 25.0 with their build; 300k: 0.86 against
 // 0.83; 100k: 0.44 against 0.38).
 constexpr int64_t kPairMin = 2 << 20;
+// The same for the boxes alone, where a query tests ten times the triangles, which
+// two lanes a query spread over the warp: 300k / 1M / 4M queries 10.4 / 27.5 / 103
+// ms at four lanes, 10.4 / 25.3 / 81 at two against 1,310,720 triangles, 0.94 /
+// 2.84 / 9.10 and 0.92 / 2.53 / 8.00 against 20,480.
+constexpr int64_t kPairMinBoxes = 3 << 18;
+
+inline bool two_lanes(bool records, int64_t n) { return n >= (records ? kPairMin : kPairMinBoxes); }
 
 template <bool kSign, bool kStats, bool kBatch>
 int launch_udf(const TreeT<kBatch>& T, const float* pts, int64_t n, const uint32_t* perm, bool coherent,
                const float* bound, const QueryOut& out, const SignArgs& sg, unsigned long long* stats, UdfWs& w,
                uint32_t seeding, const MeshSel& sel, TaskShape shape, cudaStream_t s) {
   if (coherent) {
-    if (T.num_children > 0u) {
-      A3D_TRY(n >= kPairMin
-                  ? (launch_groups<2, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
-                  : (launch_groups<4, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s)));
-    } else {
-      A3D_TRY((launch_groups<4, false, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s)));
-    }
+    const bool records = T.num_children > 0u, two = two_lanes(records, n);
+    A3D_TRY(
+        records && two ? (launch_groups<2, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
+        : records ? (launch_groups<4, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
+        : two ? (launch_groups<2, false, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
+              : (launch_groups<4, false, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s)));
   } else {
     if constexpr (!kBatch) {
       A3D_PDL((udf_kernel<kStats>), dim3((unsigned)ceil_div(n, kUdfThreads)), dim3(kUdfThreads), 0, s, T, pts, n, 1,
