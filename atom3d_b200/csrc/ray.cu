@@ -14,6 +14,7 @@
 // distance exceeds the current bound by a relative 2e-6, so pruning never
 // drops a hit.  A triangle miss is +inf (the reference uses a 1e10 sentinel,
 // which a max_t above 1e10 would count as a hit).
+#include <float.h>
 #include <math.h>
 
 #include "bvh_layout.cuh"
@@ -31,6 +32,11 @@ constexpr int kRayDeep = 256;    // local-memory stack of the re-run kernel
 constexpr int kAllDepth = 192;   // node stack of the all-hit traversals
 constexpr int kParityCap = 256;  // hits per (point, direction) kept by the parity kernel
 constexpr float kPruneSlack = 1.000002f;
+
+// The largest entry distance of a box that can hold a hit before t.  Finite: a
+// missed child and an empty slot, whose reference names nothing, have the entry
+// distance +inf, which no t admits.
+__device__ __forceinline__ float prune_limit(float t) { return fminf(t * kPruneSlack, FLT_MAX); }
 
 struct V3 {
   float x, y, z;
@@ -199,7 +205,7 @@ __device__ bool nearest(const WideNode* __restrict__ nodes, const TriRec* __rest
         cswap(tc[0], rc[0], tc[2], rc[2]);
         cswap(tc[1], rc[1], tc[3], rc[3]);
         cswap(tc[1], rc[1], tc[2], rc[2]);
-        const float lim = mint * kPruneSlack;
+        const float lim = prune_limit(mint);
         int q = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) q += tc[c] <= lim ? 1 : 0;
@@ -348,7 +354,7 @@ __global__ void __launch_bounds__(kRayThreads, kRayBlocks)
         cswap(tc[0], rc[0], tc[2], rc[2]);
         cswap(tc[1], rc[1], tc[3], rc[3]);
         cswap(tc[1], rc[1], tc[2], rc[2]);
-        const float lim = mint * kPruneSlack;
+        const float lim = prune_limit(mint);
         int q = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) q += tc[c] <= lim ? 1 : 0;
@@ -484,7 +490,7 @@ __device__ bool all_hits(const WideNode* __restrict__ nodes, const TriRec* __res
   uint32_t stack[kAllDepth];
   int sp = 0;
   stack[sp++] = 0u;
-  const float lim = max_t * kPruneSlack;
+  const float lim = prune_limit(max_t);
   bool ok = true;
   while (sp > 0) {
     const uint32_t ref = stack[--sp];
@@ -628,7 +634,7 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
   const unsigned FULL = 0xffffffffu;
   ParitySmem& S = smem[threadIdx.x >> 5];
   const int64_t rays = n * ndir;
-  const float lim = max_t * kPruneSlack;
+  const float lim = prune_limit(max_t);
   int64_t pos = 0, end = 0;
   bool exhausted = false, live = false, lost = false;
   int64_t i = 0;
@@ -638,10 +644,12 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
   float more_hits[kParityCap - kParityHits];
   uint32_t more_stack[kAllDepth - kParityStack];
 
+  const uint32_t* deep = more_stack;
+
   auto pop = [&]() -> uint32_t {
     if (sp == 0) return kNoItem;
     --sp;
-    return sp < kParityStack ? S.stack[sp][lane] : more_stack[sp - kParityStack];
+    return sp < kParityStack ? S.stack[sp][lane] : deep[sp - kParityStack];
   };
   auto distribute = [&](unsigned want) {
     while (want) {
