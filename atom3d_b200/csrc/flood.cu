@@ -24,7 +24,7 @@
 //     being updated is safe; rounds repeat until no brick is dirty;
 //   * labels and the k-ring dilation are word-parallel passes over runs of
 //     rows (the last ring decides its labels itself); one pass
-//     counts every label per tile of kTileWords words (and in total), and a
+//     counts every label per tile of consecutive words (and in total), and a
 //     label's coordinates are written by one block per tile after a scan of
 //     that label's tile counts (words are ranked inside the tile).
 #include <limits.h>
@@ -411,22 +411,31 @@ enum { kWater = 0, kDry = 1, kTide = 2, kDam = 3, kExt = 4, kExtTide = 5, kDryAd
 // lie along w, then along the next run of rows.  20.7M words: labels 883 ->
 // 330 us (896 MB that have to move: 138 us), the ring with its copy and the
 // classification 560 -> 180 us, against a thread a word.
-constexpr int kRun = 16;
+// Runs are shorter while there would be fewer than kRunThreads of them, down to
+// kRunMin rows, which a volume of a few thousand words waits for (44^3: labels
+// 21 us at 16 rows, 5 at 2).
+constexpr int kRun = 16, kRunMin = 2;
+constexpr int64_t kRunThreads = 1 << 16;
 
 struct RunPos {
   int x, y0, y1, w;  // rows y0 <= y < y1
 };
-__device__ __forceinline__ int64_t runs_of(const Geom& g) {
-  return (int64_t)g.nx * ((g.ny + kRun - 1) / kRun) * g.nw;
+__host__ __device__ inline int64_t runs_of(const Geom& g, int run) {
+  return (int64_t)g.nx * ((g.ny + run - 1) / run) * g.nw;
 }
-__device__ __forceinline__ RunPos run_pos(const Geom& g, int64_t t) {
+inline int run_length(const Geom& g) {
+  int run = kRun;
+  while (run > kRunMin && runs_of(g, run) < kRunThreads) run >>= 1;
+  return run;
+}
+__device__ __forceinline__ RunPos run_pos(const Geom& g, int run, int64_t t) {
   const int64_t r = t / g.nw;
-  const int runs = (g.ny + kRun - 1) / kRun;
+  const int runs = (g.ny + run - 1) / run;
   RunPos p;
   p.w = (int)(t - r * g.nw);
   p.x = (int)(r / runs);
-  p.y0 = (int)(r - (int64_t)p.x * runs) * kRun;
-  p.y1 = p.y0 + kRun < g.ny ? p.y0 + kRun : g.ny;
+  p.y0 = (int)(r - (int64_t)p.x * runs) * run;
+  p.y1 = p.y0 + run < g.ny ? p.y0 + run : g.ny;
   return p;
 }
 
@@ -460,11 +469,11 @@ __device__ __forceinline__ RowPart row_part(const uint32_t* __restrict__ v, cons
 template <int kConn>
 __global__ void __launch_bounds__(256)
     labels_kernel(Geom g, const uint32_t* __restrict__ occ, const uint32_t* __restrict__ water,
-                  uint32_t* __restrict__ lab, int64_t nwords) {
+                  uint32_t* __restrict__ lab, int64_t nwords, int run) {
   pdl_wait();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= runs_of(g)) return;
-  const RunPos p = run_pos(g, t);
+  if (t >= runs_of(g, run)) return;
+  const RunPos p = run_pos(g, run, t);
   // the extension takes the 3x3x3 dilation of the water, or the 6-cross for
   // connectivity 6
   constexpr int kExtConn = kConn == 18 ? 26 : kConn;
@@ -505,11 +514,11 @@ __global__ void __launch_bounds__(256)
 template <bool kClassify>
 __global__ void __launch_bounds__(256)
     box_dilate_kernel(Geom g, const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
-                      uint32_t* __restrict__ lab, int64_t nwords) {
+                      uint32_t* __restrict__ lab, int64_t nwords, int run) {
   pdl_wait();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= runs_of(g)) return;
-  const RunPos p = run_pos(g, t);
+  if (t >= runs_of(g, run)) return;
+  const RunPos p = run_pos(g, run, t);
   const uint32_t valid = valid_mask(g, p.w);
   uint32_t s0 = row_part<26>(src, g, p.x, p.y0 - 1, p.w).own, s1 = row_part<26>(src, g, p.x, p.y0, p.w).own;
   for (int y = p.y0; y < p.y1; ++y) {
@@ -528,27 +537,31 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// A tile is kTileWords consecutive words: 256 threads, each warp owning
-// kTileWords / 8 consecutive words in chunks of 32 (one word per lane).
+// A tile is kTileThreads * kChunks consecutive words, 256 threads: each warp owns
+// an eighth of them in chunks of 32 (one word per lane).  Volumes take 8 chunks;
+// below kTileSmall words one, since a warp writes its words one after the other
+// (44^3, two volume labels: 94 us at 8 chunks, 18 at 1).
 constexpr int kTileThreads = 256;
-constexpr int kTileWords = 2048;
-constexpr int kTileChunks = kTileWords / kTileThreads;  // chunks of 32 words per warp
+constexpr int kTileChunks = 8;
+constexpr int64_t kTileSmall = 1 << 18;
+__host__ __device__ inline int tile_chunks(int64_t nwords) { return nwords < kTileSmall ? 1 : kTileChunks; }
 
 // set voxels of every label per tile (label-major [kRing][ntiles]) and per
 // label in total
+template <int kChunks>
 __global__ void __launch_bounds__(kTileThreads) tile_counts_kernel(const uint32_t* __restrict__ lab, int64_t nwords,
                                                                    int64_t ntiles, uint32_t* __restrict__ tcnt,
                                                                    unsigned long long* __restrict__ tot) {
   pdl_wait();
   __shared__ uint32_t s_part[kRing][kTileThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t base = (int64_t)blockIdx.x * kTileWords;
+  const int64_t base = (int64_t)blockIdx.x * (kTileThreads * kChunks);
 #pragma unroll 1
   for (int k = 0; k < kRing; ++k) {
     const uint32_t* v = lab + (int64_t)k * nwords;
     uint32_t c = 0;
 #pragma unroll
-    for (int j = 0; j < kTileChunks; ++j) {
+    for (int j = 0; j < kChunks; ++j) {
       const int64_t i = base + (int64_t)j * kTileThreads + threadIdx.x;
       if (i < nwords) c += (uint32_t)__popc(v[i]);
     }
@@ -602,7 +615,7 @@ __device__ __forceinline__ void write_run(int32_t* __restrict__ out, int len, in
 // voxels 941 and 524 us without it, 828 and 483 us (5.8 TB/s) with it.  The
 // surfaces (3.3M voxels in 20.7M words), bound by instructions, take 111 us
 // with it and 89 us without (100 us with a scan of every chunk's counts).
-template <bool kRuns>
+template <bool kRuns, int kChunks>
 __global__ void __launch_bounds__(kTileThreads) extract_tile_kernel(Geom g, const uint32_t* __restrict__ v,
                                                                     const int64_t* __restrict__ toff, int64_t nwords,
                                                                     int64_t count, int32_t* __restrict__ out) {
@@ -611,11 +624,11 @@ __global__ void __launch_bounds__(kTileThreads) extract_tile_kernel(Geom g, cons
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  const int64_t base = (int64_t)blockIdx.x * kTileWords + (int64_t)warp * (kTileChunks * 32);
-  uint32_t word[kTileChunks];
+  const int64_t base = (int64_t)blockIdx.x * (kTileThreads * kChunks) + (int64_t)warp * (kChunks * 32);
+  uint32_t word[kChunks];
   uint32_t run = 0;
 #pragma unroll
-  for (int c = 0; c < kTileChunks; ++c) {
+  for (int c = 0; c < kChunks; ++c) {
     const int64_t i = base + c * 32 + lane;
     word[c] = i < nwords ? v[i] : 0u;
     run += (uint32_t)__popc(word[c]);
@@ -627,7 +640,7 @@ __global__ void __launch_bounds__(kTileThreads) extract_tile_kernel(Geom g, cons
   int64_t pos = toff[blockIdx.x];
   for (int w = 0; w < warp; ++w) pos += s_warp[w];
 #pragma unroll
-  for (int c = 0; c < kTileChunks; ++c) {
+  for (int c = 0; c < kChunks; ++c) {
     unsigned nz = __ballot_sync(FULL, word[c] != 0u);
     if (!nz) continue;
     const uint32_t i = (uint32_t)(base + c * 32 + lane);
@@ -756,7 +769,20 @@ struct FloodWs {
   uint32_t* misc;    // [0] seed status [2..4] queue counts (round % 3) [8..21] label totals (u64)
 };
 
-int64_t tiles_of(const Geom& g) { return ceil_div((int64_t)g.nx * g.ny * g.nw, kTileWords); }
+int64_t tiles_of(const Geom& g) {
+  const int64_t nwords = (int64_t)g.nx * g.ny * g.nw;
+  return ceil_div(nwords, kTileThreads * tile_chunks(nwords));
+}
+
+// voxels of every label per tile (w.tcnt) and in total (tot)
+int launch_tile_counts(const FloodWs& w, int64_t nwords, int64_t ntiles, unsigned long long* tot, cudaStream_t s) {
+  const dim3 g((unsigned)ntiles), b(kTileThreads);
+  if (tile_chunks(nwords) == 1)
+    A3D_PDL(tile_counts_kernel<1>, g, b, 0, s, w.lab, nwords, ntiles, w.tcnt, tot);
+  else
+    A3D_PDL(tile_counts_kernel<kTileChunks>, g, b, 0, s, w.lab, nwords, ntiles, w.tcnt, tot);
+  return A3D_OK;
+}
 
 size_t carve_flood(FloodWs& w, Workspace& ws, const Geom& g) {
   const int64_t nwords = (int64_t)g.nx * g.ny * g.nw;
@@ -873,30 +899,31 @@ extern "C" int a3d_flood_fill(const int64_t* dam_ijk, int64_t n, const a3d_flood
   A3D_REQUIRE(!(hs[0] & 1u), A3D_ERR_OVERFLOW, "a3d_flood_fill: relaxation did not converge within 2^20 rounds");
   const int rounds = (int)hs[1];
   if (rounds_out) *rounds_out = rounds;
-  const unsigned gr = (unsigned)ceil_div((int64_t)g.nx * ceil_div(g.ny, kRun) * g.nw, 256);
+  const int run = run_length(g);
+  const unsigned gr = (unsigned)ceil_div(runs_of(g, run), 256);
   if (conn == 6)
-    A3D_PDL(labels_kernel<6>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+    A3D_PDL(labels_kernel<6>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords, run);
   else if (conn == 18)
-    A3D_PDL(labels_kernel<18>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+    A3D_PDL(labels_kernel<18>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords, run);
   else
-    A3D_PDL(labels_kernel<26>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords);
+    A3D_PDL(labels_kernel<26>, dim3(gr), dim3(256), 0, s, g, w.occ, w.water, w.lab, nwords, run);
   // k-ring box dilation of the dam, ping-ponging ring buffers; the last ring
   // decides the labels, and none leaves nothing outside the dam
   const uint32_t* ring = w.lab + (int64_t)kDam * nwords;
   uint32_t* bufs[2] = {w.lab + (int64_t)kRing * nwords, w.ring2};
   for (int k = 0; k + 1 < geom->k_ring; ++k) {
-    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, ring, bufs[k & 1], w.lab, nwords);
+    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, ring, bufs[k & 1], w.lab, nwords, run);
     ring = bufs[k & 1];
   }
   if (geom->k_ring > 0) {
-    A3D_PDL(box_dilate_kernel<true>, dim3(gr), dim3(256), 0, s, g, ring, (uint32_t*)nullptr, w.lab, nwords);
+    A3D_PDL(box_dilate_kernel<true>, dim3(gr), dim3(256), 0, s, g, ring, (uint32_t*)nullptr, w.lab, nwords, run);
   } else {
     A3D_CUDA_TRY(cudaMemsetAsync(w.lab + (int64_t)kExtTide * nwords, 0, 2 * nwords * 4, s));
   }
   // counts per label and tile, one pass and one host read
   const int64_t ntiles = tiles_of(g);
   unsigned long long* tot = reinterpret_cast<unsigned long long*>(w.misc + 8);
-  A3D_PDL(tile_counts_kernel, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, w.lab, nwords, ntiles, w.tcnt, tot);
+  A3D_TRY(launch_tile_counts(w, nwords, ntiles, tot, s));
   unsigned long long h[kRing];
   A3D_CUDA_TRY(cudaMemcpyAsync(h, tot, sizeof(h), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
@@ -920,12 +947,18 @@ extern "C" int a3d_flood_extract(const a3d_flood_geom* geom, void* workspace, si
   const uint32_t* v = w.lab + (int64_t)label * nwords;
   A3D_TRY((device_exclusive_scan<uint32_t, int64_t>(w.tcnt + (int64_t)label * ntiles, w.toff, ntiles, w.scan_tmp,
                                                      w.toff + ntiles, s)));
-  if (count >= 4 * nwords)
-    A3D_PDL(extract_tile_kernel<true>, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, g, v, w.toff, nwords, count,
-            out_ijk);
-  else
-    A3D_PDL(extract_tile_kernel<false>, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, g, v, w.toff, nwords, count,
-            out_ijk);
+  const dim3 gt((unsigned)ntiles), bt(kTileThreads);
+  const bool runs = count >= 4 * nwords;
+  if (tile_chunks(nwords) == 1) {
+    if (runs)
+      A3D_PDL((extract_tile_kernel<true, 1>), gt, bt, 0, s, g, v, w.toff, nwords, count, out_ijk);
+    else
+      A3D_PDL((extract_tile_kernel<false, 1>), gt, bt, 0, s, g, v, w.toff, nwords, count, out_ijk);
+  } else if (runs) {
+    A3D_PDL((extract_tile_kernel<true, kTileChunks>), gt, bt, 0, s, g, v, w.toff, nwords, count, out_ijk);
+  } else {
+    A3D_PDL((extract_tile_kernel<false, kTileChunks>), gt, bt, 0, s, g, v, w.toff, nwords, count, out_ijk);
+  }
   return A3D_OK;
 }
 
@@ -977,20 +1010,21 @@ extern "C" int a3d_ring_signs(const int64_t* dam_ijk, int64_t n_dam, const int64
     A3D_PDL(set_bits_kernel, dim3((unsigned)ceil_div(n_dry, 256)), dim3(256), 0, s, dry_ijk, n_dry, g,
             w.lab + (int64_t)kDry * nwords);
   }
-  const unsigned gr = (unsigned)ceil_div((int64_t)g.nx * ceil_div(g.ny, kRun) * g.nw, 256);
+  const int run = run_length(g);
+  const unsigned gr = (unsigned)ceil_div(runs_of(g, run), 256);
   uint32_t* ring_out = w.lab + (int64_t)kExtTide * nwords;
   const uint32_t* src = v_dam;
   uint32_t* bufs[2] = {w.lab + (int64_t)kRing * nwords, w.ring2};
   for (int k = 0; k < geom->k_ring; ++k) {
     uint32_t* dst = (k == geom->k_ring - 1) ? ring_out : bufs[k & 1];
-    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, src, dst, w.lab, nwords);
+    A3D_PDL(box_dilate_kernel<false>, dim3(gr), dim3(256), 0, s, g, src, dst, w.lab, nwords, run);
     src = dst;
   }
   if (geom->k_ring == 0)
     A3D_CUDA_TRY(cudaMemcpyAsync(ring_out, v_dam, nwords * 4, cudaMemcpyDeviceToDevice, s));
   const int64_t ntiles = tiles_of(g);
   unsigned long long* tot = reinterpret_cast<unsigned long long*>(w.misc + 8);
-  A3D_PDL(tile_counts_kernel, dim3((unsigned)ntiles), dim3(kTileThreads), 0, s, w.lab, nwords, ntiles, w.tcnt, tot);
+  A3D_TRY(launch_tile_counts(w, nwords, ntiles, tot, s));
   unsigned long long h = 0;
   A3D_CUDA_TRY(cudaMemcpyAsync(&h, tot + kExtTide, sizeof(h), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
