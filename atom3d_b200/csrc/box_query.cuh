@@ -225,10 +225,13 @@ struct BoxSmem {
   uint8_t task[32 * kMaxLeafTris];  // a leaf step's tests: lane | position in its leaf << 5
 };
 
-// boxes a warp takes: all warps get some while there are few
+// Boxes a warp takes: all warps get some while there are few, down to one each,
+// since a warp's time is that of all its boxes' steps (1,000 boxes of some 150
+// pairs each, 1,310,720 triangles: count and write pass 377 + 655 us at 32 boxes a
+// warp, 253 + 301 at one; a thread a box 448 + 488).
 __host__ __device__ inline int64_t box_items(int64_t n, int64_t warps) {
-  const int64_t per = ceil_div(ceil_div(n, warps), 32) * 32;
-  return per < 32 ? 32 : per > kBoxItems ? kBoxItems : per;
+  const int64_t per = ceil_div(n, warps);
+  return per <= 32 ? (per < 1 ? 1 : per) : per > kBoxItems ? kBoxItems : ceil_div(per, 32) * 32;
 }
 
 // A query Q of the walk (its members are the state of the lane's box):
@@ -418,7 +421,7 @@ __device__ __forceinline__ void box_walk_all(const WideNode* __restrict__ nodes,
 }
 // blocks of box_walk_all over at most n items
 inline int64_t box_blocks(int64_t n, int sms) {
-  const int64_t want = ceil_div(n, 32 * kBoxWarps), cap = (int64_t)sms * kBoxBlocks;
+  const int64_t want = ceil_div(n, kBoxWarps), cap = (int64_t)sms * kBoxBlocks;
   return want < cap ? want : cap;
 }
 
