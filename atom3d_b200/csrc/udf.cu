@@ -999,14 +999,20 @@ __global__ void query_morton_kernel(const float* __restrict__ pts, int64_t n, fl
 
 constexpr int kStatusWords = 8;
 
-// Queries are Morton-sorted from kSortMin on.  Below it what the sorted order
-// saves (L1 misses, a seed from the neighbour) does not pay for the sort, even
-// for queries in random order: 100,000 / 1M / 2M / 4M queries in random order
-// against 1,310,720 triangles take 0.59 / 3.14 / 5.77 / 10.8 ms unsorted and
-// 0.75 / 3.26 / 5.55 / 8.85 ms sorted, against 20,480 rough triangles 0.25 /
-// 1.49 / 2.85 / 5.07 and 0.28 / 1.46 / 2.66 / 4.23.  Below kSortFine 8 bits an
-// axis (three passes) order as well as 10 (four), above 10 gain about 1%.
-constexpr int64_t kSortMin = 3 << 19;
+// Queries are Morton-sorted from kSortMin on, those without child records from
+// kSortMinBoxes on.  Below it what the sorted order saves (L1 misses, a seed from
+// the neighbour) does not pay for the sort, even for queries in random order.  ms,
+// unsorted / sorted, with records:
+//                                       300k         700k         1M           1.3M
+//   1,310,720 triangles, uniform      1.64 / 1.68  3.47 / 3.32  4.82 / 4.46  6.16 / 5.62
+//   the same, half of them near it     1.20 / 1.32  2.45 / 2.53  3.31 / 3.43  4.22 / 4.18
+//   20,480 rough triangles, uniform   0.70 / 0.68  1.49 / 1.38  2.08 / 1.92  2.68 / 2.44
+//   1,000,000 scattered triangles     0.51 / 0.51  1.18 / 1.07  1.69 / 1.47  2.20 / 1.87
+// (the last at 1M, sorted, without records and discs: 1.62) and by boxes alone
+// (the first mesh, two lanes, 1M) 26.0 / 30.4 and 14.7 / 19.1.  Below kSortFine 8
+// bits an axis (three passes) order as well as 10 (four), above 10 gain about 1%.
+constexpr int64_t kSortMin = 7 << 17, kSortMinBoxes = 3 << 19;
+inline bool sorted_queries(bool records, int64_t n) { return n >= (records ? kSortMin : kSortMinBoxes); }
 constexpr int64_t kSortFine = 8 << 20;
 
 struct UdfWs {
@@ -1243,7 +1249,7 @@ extern "C" int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, c
   }
   const int64_t n = num_points;
   const uint32_t* perm = nullptr;
-  const bool sort = (flags & A3D_UDF_SORT_QUERIES) != 0 && n >= kSortMin;
+  const bool sort = (flags & A3D_UDF_SORT_QUERIES) != 0 && sorted_queries(children != nullptr, n);
   if (sort) {
     const float ext[3] = {bvh->hi[0] - bvh->lo[0], bvh->hi[1] - bvh->lo[1], bvh->hi[2] - bvh->lo[2]};
     float emax = fmaxf(ext[0], fmaxf(ext[1], ext[2]));
@@ -1414,7 +1420,7 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_childr
     const int64_t cn = n - base < kBatchChunk ? n - base : kBatchChunk;
     const float* pts = points + 3 * base;
     const uint32_t* perm = nullptr;  // the caller's order (mesh by mesh) when there are few
-    if (cn >= kSortMin) {
+    if (sorted_queries(T.num_children > 0u, cn)) {
       A3D_PDL(batch_query_morton_kernel, dim3((unsigned)ceil_div(cn, 256)), dim3(256), 0, s, pts, cn, base, qoff,
               bvh->num_meshes, bvh->bounds, bits, w.keys, w.vals);
       bool alt = false;

@@ -12,8 +12,9 @@ from test_children_gpu import mesh, plain_query
 
 pytestmark = pytest.mark.gpu
 
-# from here on: two lanes without records, sorting, two lanes with records
-SIZES = [(3 << 18) + 3, (3 << 19) + 3, (2 << 20) + 3]
+# from here on: two lanes without records, sorting with them, sorting without,
+# two lanes with records
+SIZES = [(3 << 18) + 3, (7 << 17) + 3, (3 << 19) + 3, (2 << 20) + 3]
 
 
 @pytest.mark.parametrize("kind", ["soup", "cube", "infinite vertex", "flattened"])
