@@ -1120,12 +1120,14 @@ constexpr int64_t kPairMinBoxes = 3 << 18;
 
 inline bool two_lanes(bool records, int64_t n) { return n >= (records ? kPairMin : kPairMinBoxes); }
 
+// n queries with the kernel of a call of `like` (n itself, but for the
+// autotuner's samples)
 template <bool kSign, bool kStats, bool kBatch>
-int launch_udf(const TreeT<kBatch>& T, const float* pts, int64_t n, const uint32_t* perm, bool coherent,
+int launch_udf(const TreeT<kBatch>& T, const float* pts, int64_t n, int64_t like, const uint32_t* perm, bool coherent,
                const float* bound, const QueryOut& out, const SignArgs& sg, unsigned long long* stats, UdfWs& w,
                uint32_t seeding, const MeshSel& sel, TaskShape shape, cudaStream_t s) {
   if (coherent) {
-    const bool records = T.num_children > 0u, two = two_lanes(records, n);
+    const bool records = T.num_children > 0u, two = two_lanes(records, like);
     A3D_TRY(
         records && two ? (launch_groups<2, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
         : records ? (launch_groups<4, true, kStats, kBatch>(T, pts, n, perm, bound, stats, w, seeding, sel, shape, s))
@@ -1284,17 +1286,17 @@ extern "C" int a3d_udf_children(const a3d_bvh_view* bvh, const void* children, c
   }
   if (sign) {
     if (stats)
-      A3D_TRY((launch_udf<true, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+      A3D_TRY((launch_udf<true, true, false>(T, points, n, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
                                              shape, s)));
     else
-      A3D_TRY((launch_udf<true, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+      A3D_TRY((launch_udf<true, false, false>(T, points, n, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
                                               shape, s)));
   } else {
     if (stats)
-      A3D_TRY((launch_udf<false, true, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+      A3D_TRY((launch_udf<false, true, false>(T, points, n, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
                                               shape, s)));
     else
-      A3D_TRY((launch_udf<false, false, false>(T, points, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
+      A3D_TRY((launch_udf<false, false, false>(T, points, n, n, perm, coherent, bound, out, sg, stats, w, seeding, sel,
                                                shape, s)));
   }
   if (stats) {
@@ -1326,6 +1328,9 @@ extern "C" int a3d_udf_backward(const float* points, int64_t num_points, const f
 namespace a3d {
 namespace {
 
+// blocks an SM of a tuning that takes all that fit, whatever the kernel (32: an
+// SM's most), so that calls of another size are not held to one kernel's count
+constexpr int kAllBlocks = 32;
 // queries per traversal launch of a batch (bounds the scratch: ~380 MB)
 constexpr int64_t kBatchChunk = 1ll << 24;
 
@@ -1382,8 +1387,10 @@ size_t batch_udf_bytes(int64_t n) {
   return base + (size_t)spill_owner_bound(c) * kSpillCap * sizeof(uint2) + 512;
 }
 
+// like: the size of the call whose order and kernel are used (0: this one's own,
+// launch by launch); the autotuner times its samples with those of the whole call
 int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_children, const float* points,
-              const int64_t* qoff, int64_t n, float* distances, int32_t* face_ids, float* closest_points,
+              const int64_t* qoff, int64_t n, int64_t like, float* distances, int32_t* face_ids, float* closest_points,
               float* uvw, TaskShape shape, unsigned long long* stats,
               void* workspace, size_t workspace_bytes, cudaStream_t s) {
   A3D_REQUIRE(bvh && bvh->nodes && bvh->tris && bvh->roots && bvh->bounds && bvh->num_meshes > 0 &&
@@ -1418,9 +1425,10 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_childr
   const SignArgs sg{nullptr, nullptr, nullptr, nullptr, nullptr};
   for (int64_t base = 0; base < n; base += kBatchChunk) {
     const int64_t cn = n - base < kBatchChunk ? n - base : kBatchChunk;
+    const int64_t as = like > 0 ? like : cn;
     const float* pts = points + 3 * base;
     const uint32_t* perm = nullptr;  // the caller's order (mesh by mesh) when there are few
-    if (sorted_queries(T.num_children > 0u, cn)) {
+    if (sorted_queries(T.num_children > 0u, as)) {
       A3D_PDL(batch_query_morton_kernel, dim3((unsigned)ceil_div(cn, 256)), dim3(256), 0, s, pts, cn, base, qoff,
               bvh->num_meshes, bvh->bounds, bits, w.keys, w.vals);
       bool alt = false;
@@ -1434,10 +1442,10 @@ int batch_udf(const a3d_bvh_batch* bvh, const void* children, int64_t num_childr
     const QueryOut out{distances + base, face_ids + base, closest_points + 3 * base, uvw ? uvw + 3 * base : nullptr};
     const MeshSel sel{qoff, bvh->roots, bvh->num_meshes, base};
     if (stats)
-      A3D_TRY((launch_udf<false, true, true>(T, pts, cn, perm, true, nullptr, out, sg, stats, w, kSeedReuse, sel,
+      A3D_TRY((launch_udf<false, true, true>(T, pts, cn, as, perm, true, nullptr, out, sg, stats, w, kSeedReuse, sel,
                                              shape, s)));
     else
-      A3D_TRY((launch_udf<false, false, true>(T, pts, cn, perm, true, nullptr, out, sg, stats, w, kSeedReuse, sel,
+      A3D_TRY((launch_udf<false, false, true>(T, pts, cn, as, perm, true, nullptr, out, sg, stats, w, kSeedReuse, sel,
                                               shape, s)));
   }
   if (stats) A3D_CUDA_TRY(cudaMemcpyAsync(stats + 2, w.nrerun + 4, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
@@ -1520,7 +1528,7 @@ extern "C" int a3d_batch_udf_children(const a3d_bvh_batch* bvh, const void* chil
     if (tuning->pool > 0) shape.pool = tuning->pool;
     shape.blocks_per_sm = tuning->blocks_per_sm;
   }
-  return a3d::batch_udf(bvh, children, num_children, points, query_offsets, num_queries, distances, face_ids,
+  return a3d::batch_udf(bvh, children, num_children, points, query_offsets, num_queries, 0, distances, face_ids,
                         closest_points, uvw, shape, stats, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
@@ -1560,15 +1568,22 @@ extern "C" int a3d_batch_autotune_children(const a3d_bvh_batch* bvh, const void*
   const int64_t th = ns > (int64_t)bvh->num_meshes + 1 ? ns : (int64_t)bvh->num_meshes + 1;
   A3D_PDL(sample_queries_kernel, dim3((unsigned)ceil_div(th, 256)), dim3(256), 0, s, points, stride, query_offsets,
           bvh->num_meshes, t.pts, ns, t.qoff);
+  // order and kernel of the call that is tuned for (of its first launch), and the
+  // blocks of that kernel an SM holds
+  const int64_t like = num_queries < kBatchChunk ? num_queries : kBatchChunk;
+  const bool records = children != nullptr && num_children > 0, two = two_lanes(records, like);
   int occ = 0;
-  A3D_TRY((group_blocks_per_sm<2, true, false, true>(&occ)));
+  A3D_TRY((records && two ? group_blocks_per_sm<2, true, false, true>(&occ)
+           : records      ? group_blocks_per_sm<4, true, false, true>(&occ)
+           : two          ? group_blocks_per_sm<2, false, false, true>(&occ)
+                          : group_blocks_per_sm<4, false, false, true>(&occ)));
   const int pools[4] = {32, 64, 128, 256};
   const int bpss[3] = {occ, occ * 3 / 4, occ / 2};
   cudaEvent_t e0, e1;
   A3D_CUDA_TRY(cudaEventCreate(&e0));
   A3D_CUDA_TRY(cudaEventCreate(&e1));
   float best_t = INFINITY;
-  a3d_udf_tuning bt{64, occ, 0, 0};
+  a3d_udf_tuning bt{64, kAllBlocks, 0, 0};
   int rc = A3D_OK;
   for (int pi = 0; pi < 4 && rc == A3D_OK; ++pi) {
     for (int bi = 0; bi < 3 && rc == A3D_OK; ++bi) {
@@ -1579,8 +1594,8 @@ extern "C" int a3d_batch_autotune_children(const a3d_bvh_batch* bvh, const void*
       for (int rep = 0; rep < 3 && rc == A3D_OK; ++rep) {
         if (rep == 1 && cudaEventRecord(e0, s) != cudaSuccess) rc = A3D_ERR_CUDA;
         if (rc == A3D_OK)
-          rc = batch_udf(bvh, children, num_children, t.pts, t.qoff, ns, t.dist, t.fid, t.cp, nullptr, shape, nullptr,
-                         t.udf_ws, t.udf_bytes, s);
+          rc = batch_udf(bvh, children, num_children, t.pts, t.qoff, ns, like, t.dist, t.fid, t.cp, nullptr, shape,
+                         nullptr, t.udf_ws, t.udf_bytes, s);
       }
       float ms = 0.f;
       if (rc == A3D_OK && (cudaEventRecord(e1, s) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
@@ -1590,7 +1605,7 @@ extern "C" int a3d_batch_autotune_children(const a3d_bvh_batch* bvh, const void*
       ms *= 0.5f;
       if (ms < best_t) {
         best_t = ms;
-        bt = a3d_udf_tuning{pools[pi], bps, 0, 0};
+        bt = a3d_udf_tuning{pools[pi], bi == 0 ? kAllBlocks : bps, 0, 0};
       }
     }
   }

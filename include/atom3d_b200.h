@@ -574,8 +574,9 @@ int a3d_batch_udf_children(const a3d_bvh_batch* bvh, const void* children, int64
                         const a3d_udf_tuning* tuning, unsigned long long* stats, void* workspace,
                         size_t workspace_bytes, a3d_stream_t stream);
 /* Times the traversal's launch shapes on every ceil(Q/sample)-th query
- * (sample <= 16,777,216) and returns the fastest (host-synchronous; not
- * inside stream capture). */
+ * (sample <= 16,777,216), with the kernel and the query order that a call of
+ * all Q takes, and returns the fastest (blocks_per_sm 32: as many as fit).
+ * Host-synchronous; not inside stream capture. */
 size_t a3d_batch_autotune_workspace_bytes(int64_t sample_queries, int32_t num_meshes);
 int a3d_batch_autotune(const a3d_bvh_batch* bvh, const float* points, const int64_t* query_offsets,
                        int64_t num_queries, int64_t sample_queries, void* workspace,
