@@ -5,7 +5,7 @@ kernel and in the two-lane one (from 2,097,152 queries on)."""
 import pytest
 import torch
 
-from atom3d_b200 import _lib, synthetic
+from atom3d_b200 import MeshBVH, _lib, synthetic
 from atom3d_b200.batch import BatchedMeshBVH
 
 pytestmark = pytest.mark.gpu
@@ -30,3 +30,24 @@ def test_leaf_outside_the_arrays_is_recorded(queries):
     q[half:] += 4.0
     bb.udf(q, [half, queries - half])
     assert bb.query_status()["faults"] == FAULT_TRI
+
+
+def test_tree_above_the_level_limit_is_reported_and_safe():
+    """Triangles over 100 octaves make a tree deeper than the collapse's level
+    limit.  The build's status says so; a query without reading it stays inside
+    the arrays, says so too, and answers for the other mesh of the batch."""
+    g = torch.Generator().manual_seed(4)
+    s = torch.exp2(-100 * torch.rand(60_000, 1, 1, generator=g, dtype=torch.float64))
+    deep = (s * (1 + torch.rand(60_000, 3, 3, generator=g, dtype=torch.float64))).reshape(-1, 3).float().cuda()
+    v, f = synthetic.displaced_sphere(3, 8, 0.05, 1)
+    meshes = [(deep, torch.arange(180_000, dtype=torch.int32).reshape(-1, 3).cuda()), (v.cuda(), f.cuda())]
+    bb = BatchedMeshBVH(meshes, build=False)
+    bb.build()
+    with pytest.raises(RuntimeError):
+        bb.check()
+    q = torch.zeros(6000, 3, device="cuda")
+    q[:3000] = torch.exp2(-140 * torch.rand(3000, 1, generator=g)).cuda()
+    q[3000:] = torch.rand(3000, 3, generator=g).cuda() * 3 - 1.5
+    dist, _, _ = bb.udf(q, [3000, 3000])
+    assert bb.query_status()["faults"] == FAULT_TRI
+    assert torch.equal(dist[3000:], MeshBVH(v.cuda(), f.cuda()).udf(q[3000:]))
