@@ -394,23 +394,21 @@ struct CountQuery {
   uint32_t* longs;
   unsigned long long* misc;
   uint32_t i = 0, c = 0;
-  __device__ __forceinline__ uint32_t begin(int64_t k, float* mn, float* mx) {
+  __device__ __forceinline__ void begin(int64_t k, float* mn, float* mx) {
     i = (uint32_t)k;
     c = 0;
     load_box(bmin, bmax, k, mn, mx);
-    return kNoRef;
   }
-  __device__ __forceinline__ bool leaf(uint32_t mask, uint32_t first) {
+  __device__ __forceinline__ void leaf(uint32_t mask, uint32_t first) {
     for (uint32_t m = mask; m && c < (uint32_t)kPairsKept; m &= m - 1u) {
       kept[(int64_t)kPairsKept * i + c] = first + (uint32_t)__ffs((int)m) - 1u;
       ++c;
       mask &= mask - 1u;
     }
     c += (uint32_t)__popc(mask);
-    return false;
   }
-  __device__ __forceinline__ void done(int status) {
-    if (status == 2) {
+  __device__ __forceinline__ void done(bool overflow) {
+    if (overflow) {
       spill[atomicAdd(misc, 1ull)] = i;
       c = 0;
     } else if (c > (uint32_t)kPairsKept) {
@@ -482,20 +480,18 @@ struct WriteQuery {
   int32_t* out_face;
   uint32_t i = 0;
   int64_t o = 0, end = 0;
-  __device__ __forceinline__ uint32_t begin(int64_t k, float* mn, float* mx) {
+  __device__ __forceinline__ void begin(int64_t k, float* mn, float* mx) {
     i = w.longs[k];
     o = w.offs[i];
     end = w.offs[i + 1];
     load_box(bmin, bmax, i, mn, mx);
-    return kNoRef;
   }
-  __device__ __forceinline__ bool leaf(uint32_t mask, uint32_t first) {
+  __device__ __forceinline__ void leaf(uint32_t mask, uint32_t first) {
     for (; mask; mask &= mask - 1u)
       put_pair<kSlots>(tris, num_slots, i, first + (uint32_t)__ffs((int)mask) - 1u, o++, end, out_box, out_face,
                        w.misc + 2);
-    return false;
   }
-  __device__ __forceinline__ void done(int) {}
+  __device__ __forceinline__ void done(bool) {}
 };
 
 // the boxes with more pairs than were kept: the walk again

@@ -235,11 +235,9 @@ __host__ __device__ inline int64_t box_items(int64_t n, int64_t warps) {
 }
 
 // A query Q of the walk (its members are the state of the lane's box):
-//   begin(i, mn, mx)   the box of item i; returns a leaf reference to test
-//                      before the walk, or kNoRef
-//   leaf(mask, first)  bit k: triangle first + k passed SAT; returns true to
-//                      stop
-//   done(status)       as box_traverse: 0 finished, 1 stopped, 2 overflow
+//   begin(i, mn, mx)   the box of item i
+//   leaf(mask, first)  bit k: triangle first + k passed SAT
+//   done(overflow)     the walk is over, or outgrew its stack
 
 // pruning box of a lane
 struct PruneBox {
@@ -346,7 +344,7 @@ __device__ __forceinline__ void box_walk(const WideNode* __restrict__ nodes, con
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  bool live = false, over = false, stop = false;
+  bool live = false, over = false;
   int sp = 0;
   uint32_t ref = kNoRef;
   PruneBox pb{};
@@ -357,16 +355,12 @@ __device__ __forceinline__ void box_walk(const WideNode* __restrict__ nodes, con
       const int64_t i = pos + __popc(want & lt);
       if (!live && i < end) {
         float mn[3], mx[3];
-        const uint32_t first = q.begin(i, mn, mx);
+        q.begin(i, mn, mx);
         pb = set_box(S, mn, mx);
         sp = 0;
         ref = 0u;
-        if (first != kNoRef) {
-          S.stack[sp++][lane] = 0u;
-          ref = first;
-        }
         live = true;
-        over = stop = false;
+        over = false;
       }
       pos = pos + __popc(want) < end ? pos + __popc(want) : end;
       __syncwarp();
@@ -399,13 +393,13 @@ __device__ __forceinline__ void box_walk(const WideNode* __restrict__ nodes, con
     if (__any_sync(FULL, cnt > 0u)) {
       const uint32_t mask = leaf_step(tris, cnt, leaf_first(ref), pb, S);
       if (cnt > 0u) {
-        stop = mask && q.leaf(mask, leaf_first(ref));
-        ref = !stop && sp > 0 ? S.stack[--sp][lane] : kNoRef;
+        if (mask) q.leaf(mask, leaf_first(ref));
+        ref = sp > 0 ? S.stack[--sp][lane] : kNoRef;
       }
     }
     // (d) finished boxes
     if (live && ref == kNoRef) {
-      q.done(over ? 2 : stop ? 1 : 0);
+      q.done(over);
       live = false;
     }
   }

@@ -11,10 +11,7 @@ constexpr int kChildThreads = 256;
 // subtrees above this have no disc: at that size a patch is curved and the
 // axis-aligned box serves as well, and the pass over every level's triangles
 // stays short
-#ifndef A3D_DISC_MAX_TRIS
-#define A3D_DISC_MAX_TRIS 4096
-#endif
-constexpr int64_t kDiscMaxTris = A3D_DISC_MAX_TRIS;
+constexpr int64_t kDiscMaxTris = 4096;
 constexpr int kMaxDescent = 64;  // wide levels of any tree the builder finishes
 
 __device__ __forceinline__ float warp_sum(float v) {

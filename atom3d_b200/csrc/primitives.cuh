@@ -400,18 +400,8 @@ __global__ void __launch_bounds__(kRsThreads, kRsBlocks<K>)
 template <typename K, int kItems, bool kFused>
 int radix_pass(const K* kin, const uint32_t* vin, K* kout, uint32_t* vout, int64_t n, int shift, uint32_t* hist,
                uint32_t* tmp, int64_t nt, cudaStream_t s) {
-  const size_t smem = sizeof(RsSmem<K, kItems>);
-  if (smem > 48 * 1024) {
-    // opt in above 48 KB, once per device
-    static bool done[kMaxDevices] = {false};
-    int dev = 0;
-    A3D_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= kMaxDevices || !done[dev]) {
-      A3D_CUDA_TRY(cudaFuncSetAttribute(rs_downsweep_kernel<K, kItems, kFused>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      if (dev >= 0 && dev < kMaxDevices) done[dev] = true;
-    }
-  }
+  constexpr size_t smem = sizeof(RsSmem<K, kItems>);
+  static_assert(smem <= 48 * 1024, "above 48 KB the kernel needs an opt-in per device");
   A3D_PDL((rs_upsweep_kernel<K, kItems, kFused>), dim3((unsigned)nt), dim3(kRsThreads), 0, s, kin, n, shift, hist, nt);
   if (!kFused) A3D_TRY((device_exclusive_scan<uint32_t, uint32_t>(hist, hist, 256 * nt, tmp, (uint32_t*)nullptr, s)));
   A3D_PDL((rs_downsweep_kernel<K, kItems, kFused>), dim3((unsigned)nt), dim3(kRsThreads), smem, s, kin, vin, kout,

@@ -826,21 +826,20 @@ extern "C" size_t a3d_ray_workspace_bytes(int64_t num_rays) {
 }
 
 namespace {
-// resident blocks of a persistent kernel, queried once per device; slot: one
-// per kernel
-template <typename Kernel>
-int blocks_per_sm(Kernel kernel, int* out, int slot) {
-  static int cached[2][kMaxDevices] = {};
+// resident blocks of a persistent kernel, queried once per device
+template <auto kKernel>
+int blocks_per_sm(int* out) {
+  static int cached[kMaxDevices] = {};
   int dev = 0;
   A3D_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev >= 0 && dev < kMaxDevices && cached[slot][dev] > 0) {
-    *out = cached[slot][dev];
+  if (dev >= 0 && dev < kMaxDevices && cached[dev] > 0) {
+    *out = cached[dev];
     return A3D_OK;
   }
   int b = 0;
-  A3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, kRayThreads, 0));
+  A3D_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kKernel, kRayThreads, 0));
   b = b < 1 ? 1 : b;
-  if (dev >= 0 && dev < kMaxDevices) cached[slot][dev] = b;
+  if (dev >= 0 && dev < kMaxDevices) cached[dev] = b;
   *out = b;
   return A3D_OK;
 }
@@ -886,7 +885,7 @@ extern "C" int a3d_ray_nearest(const a3d_bvh_view* bvh, const float* rays_o, con
   const TriRec* tris = (const TriRec*)bvh->tris;
   const RayOut out{hit, t, face_ids, hit_points, normals, uvw};
   int bps = 0;
-  A3D_TRY(blocks_per_sm(ray_nearest_kernel, &bps, 0));
+  A3D_TRY(blocks_per_sm<ray_nearest_kernel>(&bps));
   const int64_t warps = (int64_t)num_sms() * bps * kRayWarps;
   const int64_t pool = ray_pool(num_rays, warps);
   const int64_t want = ceil_div(ceil_div(num_rays, pool), kRayWarps), cap = warps / kRayWarps;
@@ -946,7 +945,7 @@ extern "C" int a3d_ray_parity_votes(const a3d_bvh_view* bvh, const float* points
   A3D_REQUIRE(points && dirs && votes, A3D_ERR_ARGUMENT, "ray_parity: null pointer");
   A3D_CUDA_TRY(cudaMemsetAsync(votes, 0, (size_t)num_points * sizeof(int32_t), s));
   int bps = 0;
-  A3D_TRY(blocks_per_sm(ray_parity_kernel, &bps, 1));
+  A3D_TRY(blocks_per_sm<ray_parity_kernel>(&bps));
   const int64_t rays = num_points * num_dirs, warps = (int64_t)num_sms() * bps * kRayWarps;
   const int64_t pool = ray_pool(rays, warps);
   const int64_t want = ceil_div(ceil_div(rays, pool), kRayWarps), cap = warps / kRayWarps;
