@@ -694,13 +694,15 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
       // a child is dropped by e (box and disc), visited in order of d (the box
       // alone), so the discs change which children are visited, never their
       // order; rank: the child's place in (distance, ref) order among the
-      // qualifying ones, by the distances' bits, which are never negative
+      // qualifying ones, by the distances' bits, which are never negative.  A
+      // greedy descent takes any child there is, also where every distance
+      // overflows (infinite or huge queries), so it always ends at a leaf
       bool ok[kC];
       int key[kC], rank[kC], q = 0;
       uint32_t next = 0u;
 #pragma unroll
       for (int j = 0; j < kC; ++j) {
-        ok[j] = e[j] < best_sq || (greedy && d[j] < INFINITY);
+        ok[j] = e[j] < best_sq || (greedy && r[j] != 0xffffffffu);
         key[j] = ok[j] ? __float_as_int(d[j]) : 0x7f800000;
         q += __popc((__ballot_sync(FULL, ok[j]) >> base) & gmask);
       }
@@ -722,9 +724,6 @@ __global__ void __launch_bounds__(kGroupWarps * 32, kGroupBlocks<kG>)
       for (int x = 1; x < kG; x <<= 1) next |= __shfl_xor_sync(FULL, next, x);
       if (at) {
         if (greedy) {
-          // every box distance overflows (infinite or huge queries): no child
-          // to descend to, so the query ends here and is re-run
-          greedy = have = q > 0;
           ref = next;
         } else if (q > 0) {
           if (sp + q - 1 > kDepth && sp + q - 1 > capacity()) {
