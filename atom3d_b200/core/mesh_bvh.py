@@ -5,8 +5,10 @@ Keeps the reference's constructor and query signatures
 computation runs in libatom3d_b200.so on the GPU:
 
 * construction: pseudo-normal precompute (a3d_mesh_normals) and the GPU
-  wide-BVH build (a3d_bvh_build) instead of the reference's host SAH build;
-* ``udf`` / ``sdf``: one fused traversal launch (a3d_udf), sign included;
+  wide-BVH build (a3d_bvh_build_children) instead of the reference's host SAH
+  build;
+* ``udf`` / ``sdf``: one native call (a3d_udf_children), traversal and outputs,
+  sign included;
 * ``udf(return_grad=True)``: a torch.autograd.Function whose backward is the
   hand-written adjoint kernel (a3d_udf_backward) for points and vertices;
 * ``intersect_aabb``: SAT any-hit over the BVH (mode 0, a3d_aabb_hit) and

@@ -237,7 +237,8 @@ __device__ __forceinline__ unsigned rs_peers(uint32_t d) {
 }
 
 // keys a thread of a sort of n keys: the fused form's tiles up to 131,072
-// keys, above it two tiles an SM up to 16
+// keys, above it two tiles an SM up to 16 (of 148: scratch sizes are asked for
+// without a device)
 inline int radix_items(int64_t n) {
   if (n <= kRsFuseTiles * 2 * kRsThreads) return 2;
   int items = kRsMaxItems;
