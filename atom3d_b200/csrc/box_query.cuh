@@ -90,10 +90,9 @@ __device__ __forceinline__ bool sat_half(const float4& a, const float4& b, const
       fminf(fminf(v0y, v1y), v2y) > fa(hy, eps) || fmaxf(fmaxf(v0y, v1y), v2y) < fsb(-hy, eps) ||
       fminf(fminf(v0z, v1z), v2z) > fa(hz, eps) || fmaxf(fmaxf(v0z, v1z), v2z) < fsb(-hz, eps))
     return false;
-  // 0, or NaN with an operand that is not finite (short chains: a walk waits for it)
-  const float z0 = fmaf(v0x, 0.f, fmaf(v0y, 0.f, v0z * 0.f)), z1 = fmaf(v1x, 0.f, fmaf(v1y, 0.f, v1z * 0.f));
-  const float z2 = fmaf(v2x, 0.f, fmaf(v2y, 0.f, v2z * 0.f)), z3 = fmaf(hx, 0.f, fmaf(hy, 0.f, hz * 0.f));
-  const float z = (z0 + z1) + (z2 + z3);
+  // 0, or NaN with an operand that is not finite or a sum that overflows, which
+  // the general form decides the same (short chains: a walk waits for it)
+  const float z = (((v0x + v0y) + (v0z + v1x)) + ((v1y + v1z) + (v2x + v2y)) + ((v2z + hx) + (hy + hz))) * 0.f;
   if (!(z == 0.f)) return sat_general(v0x, v0y, v0z, v1x, v1y, v1z, v2x, v2y, v2z, hx, hy, hz);
   const float e0x = fsb(v1x, v0x), e0y = fsb(v1y, v0y), e0z = fsb(v1z, v0z);
   {  // plane: normal = cross(e0, v2 - v0)

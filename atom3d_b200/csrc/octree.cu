@@ -68,7 +68,7 @@ __device__ __forceinline__ void cube_box(int x, int y, int z, const LevelGeom& g
 constexpr uint32_t kNoHint = 0xffffffffu;
 constexpr uint32_t kHintBit = 0x80000000u;
 constexpr int kListMax = 32;  // triangles of a list
-constexpr int64_t kListMin = 1 << 14;  // candidates of the collecting level
+constexpr int64_t kListFull = 1 << 14;  // candidates that fill the chip
 
 // candidate k of this level: either cube k of the full min_level grid
 // (meshgrid 'ij': x slowest, z fastest) or child (k & 7) of parent k >> 3
@@ -525,15 +525,15 @@ extern "C" int a3d_octree_traverse(const a3d_bvh_view* bvh, const float* grid_lo
     const dim3 gk((unsigned)ceil_div(ncand, kSatThreads)), bk(kSatThreads);
     // Lists are collected at the first level that has, by the usual count of
     // four hit children a parent, at most eight triangles a hit voxel, where a
-    // walk finds a whole list in few steps.  (The voxel's box meets two or three
-    // times that many triangles' boxes.)  The collecting walk costs more than the
-    // one it replaces, so two levels must be left to gain by it, and the level
-    // must fill the chip: smaller ones are bound by one walk's latency.  (128^3,
-    // 20,480 rough triangles, collected at 5,000 candidates: 554 instead of 513
-    // us; 512^3, 1,310,720 triangles, collected for the last level alone: 975
-    // instead of 913.)
+    // walk finds a whole list in few steps, or two on a level too small to fill
+    // the chip, which waits for its longest walk.  (The voxel's box meets two or
+    // three times that many triangles' boxes.)  The collecting walk costs more than
+    // the one it replaces, so two levels must be left to gain by it.  (us, no lists
+    // / eight triangles at every size and for one level / so: 128^3, 1,280 triangles
+    // 260 / 240 / 249, 20,480 rough ones 513 / 555 / 520, 5,000 large ones 457 / 540
+    // / 455; 512^3, 1,310,720 triangles 921 / 978 / 922.)
     const bool collect = !have_lists && !first_level && level + 2 <= max_level && margin >= 0.0f &&
-                         ncand >= kListMin && bvh->num_tris <= 4 * ncand;
+                         bvh->num_tris <= (ncand >= kListFull ? 4 : 1) * ncand;
     if (have_lists && last_level)
       A3D_PDL(octree_list_kernel<false>, gk, bk, 0, s, nodes, tris, lv);
     else if (have_lists)
