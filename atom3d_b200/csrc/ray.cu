@@ -444,24 +444,18 @@ __global__ void __launch_bounds__(64)
   }
 }
 
-// The remaining outputs of each ray; out.t holds t and out.face the triangle
-// record on entry.
-__global__ void __launch_bounds__(256)
-    ray_finish_kernel(const TriRec* __restrict__ tris, const float* __restrict__ face_normals,
-                      const float* __restrict__ ro, const float* __restrict__ rd, int64_t n, RayOut out) {
-  pdl_wait();
-  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t best = (uint32_t)out.face[i];
+// the outputs of ray i but t, for the nearest hit (t, best)
+__device__ __forceinline__ void write_ray(const TriRec* __restrict__ tris, const float* __restrict__ face_normals,
+                                          V3 o, V3 d, int64_t i, float t, uint32_t best, const RayOut& out) {
   const bool hit = best != 0xffffffffu;
   out.hit[i] = hit ? 1 : 0;
   V3 p{0.f, 0.f, 0.f}, nrm{0.f, 0.f, 0.f}, bc{0.f, 0.f, 0.f};
   int32_t face = -1;
   if (hit) {
-    const Tri t = load_tri(tris, best);
-    face = t.face;
-    p = vpoint(ld3(ro, i), ld3(rd, i), out.t[i]);
-    if (out.uvw) bc = tri_bary(t, p, true);
+    const Tri tr = load_tri(tris, best);
+    face = tr.face;
+    p = vpoint(o, d, t);
+    if (out.uvw) bc = tri_bary(tr, p, true);
     if (face_normals) nrm = ld3(face_normals, face);
   }
   out.face[i] = face;
@@ -480,6 +474,43 @@ __global__ void __launch_bounds__(256)
     out.uvw[3 * i + 1] = bc.y;
     out.uvw[3 * i + 2] = bc.z;
   }
+}
+
+// The remaining outputs of each ray; out.t holds t and out.face the triangle
+// record on entry.
+__global__ void __launch_bounds__(256)
+    ray_finish_kernel(const TriRec* __restrict__ tris, const float* __restrict__ face_normals,
+                      const float* __restrict__ ro, const float* __restrict__ rd, int64_t n, RayOut out) {
+  pdl_wait();
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  write_ray(tris, face_normals, ld3(ro, i), ld3(rd, i), i, out.t[i], (uint32_t)out.face[i], out);
+}
+
+// A whole ray a thread, outputs included, for trees of one node (up to some 24
+// triangles): a walk is the root and at most four leaves, and the hand-over
+// between lanes and two more passes cost more than lanes that wait.  us a call,
+// three passes / this, 300,000 and 2M rays: one triangle 48 / 40 and 97 / 75, a
+// cube's twelve 61 / 53 and 161 / 152, twenty of a sphere 64 / 57 and 161 / 167;
+// with three nodes (a cube of 48) 72 / 79 and 192 / 285.
+constexpr int64_t kRayWholeNodes = 1;
+
+__global__ void __launch_bounds__(kRayThreads)
+    ray_whole_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
+                         const float* __restrict__ face_normals, const float* __restrict__ ro,
+                         const float* __restrict__ rd, int64_t n, float max_t, RayOut out,
+                         uint32_t* __restrict__ overflow) {
+  pdl_wait();
+  const int64_t i = (int64_t)blockIdx.x * kRayThreads + threadIdx.x;
+  if (i >= n) return;
+  const Ray r = make_ray(ld3(ro, i), ld3(rd, i));
+  float mint = max_t;
+  uint32_t best = 0xffffffffu;
+  LocalStack st;
+  st.sp = 0;
+  if (!nearest(nodes, tris, r, mint, best, st)) atomicExch(overflow, 1u);
+  out.t[i] = mint;
+  write_ray(tris, face_normals, r.o, r.d, i, mint, best, out);
 }
 
 // All hits of one ray in traversal order; `emit(t, tri)` for each
@@ -884,6 +915,11 @@ extern "C" int a3d_ray_nearest(const a3d_bvh_view* bvh, const float* rays_o, con
   const WideNode* nodes = (const WideNode*)bvh->nodes;
   const TriRec* tris = (const TriRec*)bvh->tris;
   const RayOut out{hit, t, face_ids, hit_points, normals, uvw};
+  if (bvh->num_nodes <= kRayWholeNodes) {
+    A3D_PDL(ray_whole_kernel, dim3((unsigned)ceil_div(num_rays, kRayThreads)), dim3(kRayThreads), 0, s, nodes,
+            tris, face_normals, rays_o, rays_d, num_rays, max_t, out, w.status + 1);
+    return A3D_OK;
+  }
   int bps = 0;
   A3D_TRY(blocks_per_sm<ray_nearest_kernel>(&bps));
   const int64_t warps = (int64_t)num_sms() * bps * kRayWarps;
