@@ -531,8 +531,12 @@ extern "C" int a3d_octree_traverse(const a3d_bvh_view* bvh, const float* grid_lo
     // the one it replaces, so two levels must be left to gain by it.  (us, no lists
     // / eight triangles at every size and for one level / so: 128^3, 1,280 triangles
     // 260 / 240 / 249, 20,480 rough ones 513 / 555 / 520, 5,000 large ones 457 / 540
-    // / 455; 512^3, 1,310,720 triangles 921 / 978 / 922.)
+    // / 455; 512^3, 1,310,720 triangles 921 / 978 / 922.)  A tree of one node makes
+    // none: its walk is as short as a list (1024^3, a cube's twelve triangles 752
+    // us with lists, 684 without, 512^3 334 and 320; twenty of a sphere 440 and 432
+    // at 1024^3).
     const bool collect = !have_lists && !first_level && level + 2 <= max_level && margin >= 0.0f &&
+                         bvh->num_nodes > 1 &&
                          bvh->num_tris <= (ncand >= kListFull ? 4 : 1) * ncand;
     if (have_lists && last_level)
       A3D_PDL(octree_list_kernel<false>, gk, bk, 0, s, nodes, tris, lv);
