@@ -276,15 +276,21 @@ __device__ __forceinline__ void child_overlap(const WideNode* __restrict__ nodes
 // One leaf step: the cnt triangles (0: none) from first on of every lane's box.
 // Each lane compares its triangles' own boxes with its box (about a third of
 // them meet it); the rest of the test, five times as long, is spread evenly
-// over the lanes.  Returns the mask of the lane's triangles that pass SAT.
+// over the lanes.  Where the triangles of all lanes make one round of tests, or
+// most of the last step's passed (dense), the comparison costs more than it
+// saves and is left out (1,000 boxes of 342 pairs, 1,310,720 triangles: 994 ->
+// 781 us a call; 5,000 boxes that each hold half of 100,000 triangles 74.9 ->
+// 56.8 ms, 101 with a thread a box).  Returns the mask of the lane's triangles
+// that pass SAT.
 __device__ __forceinline__ uint32_t leaf_step(const TriRec* __restrict__ tris, uint32_t cnt, uint32_t first,
-                                              const PruneBox& pb, BoxSmem& S) {
+                                              const PruneBox& pb, BoxSmem& S, bool& dense) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  uint32_t near = 0;
+  const bool all = dense || __reduce_add_sync(FULL, cnt) <= 32u;
+  uint32_t near = all ? (1u << cnt) - 1u : 0u;
   const float4* p = reinterpret_cast<const float4*>(tris + first);
-  for (uint32_t k = 0; k < cnt; ++k, p += 4) {
+  for (uint32_t k = all ? cnt : 0u; k < cnt; ++k, p += 4) {
     const float4 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
     if (!(fminf(fminf(a.x, b.x), c.x) > pb.ux || fmaxf(fmaxf(a.x, b.x), c.x) < pb.lx ||
           fminf(fminf(a.y, b.y), c.y) > pb.uy || fmaxf(fmaxf(a.y, b.y), c.y) < pb.ly ||
@@ -305,6 +311,7 @@ __device__ __forceinline__ uint32_t leaf_step(const TriRec* __restrict__ tris, u
   }
   __syncwarp();
   uint32_t hits = 0;  // bit j: the j-th near triangle passes
+  uint32_t passed = 0;
   for (uint32_t t0 = 0; t0 < total; t0 += 32) {
     const uint32_t t = t0 + (uint32_t)lane;
     const uint32_t w = t < total ? S.task[t] : 0u;
@@ -317,9 +324,11 @@ __device__ __forceinline__ uint32_t leaf_step(const TriRec* __restrict__ tris, u
       pass = sat_half(a, b, c, S.box[0][o], S.box[1][o], S.box[2][o], S.box[3][o], S.box[4][o], S.box[5][o]);
     }
     const unsigned r = __ballot_sync(FULL, pass);
+    passed += (uint32_t)__popc(r);
     if (off + num > t0 && off < t0 + 32u) hits |= off >= t0 ? r >> (off - t0) : r << (t0 - off);
   }
   __syncwarp();
+  dense = passed > 0u && 4u * passed >= 3u * total;
   uint32_t mask = 0;
   for (uint32_t m = near; m; m &= m - 1u, hits >>= 1)
     if (hits & 1u) mask |= m & (0u - m);
@@ -343,7 +352,7 @@ __device__ __forceinline__ void box_walk(const WideNode* __restrict__ nodes, con
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  bool live = false, over = false;
+  bool live = false, over = false, dense = false;
   int sp = 0;
   uint32_t ref = kNoRef;
   PruneBox pb{};
@@ -390,7 +399,7 @@ __device__ __forceinline__ void box_walk(const WideNode* __restrict__ nodes, con
     // (c) leaf step
     const uint32_t cnt = live && (int)ref < 0 && ref != kNoRef ? leaf_count(ref) : 0u;
     if (__any_sync(FULL, cnt > 0u)) {
-      const uint32_t mask = leaf_step(tris, cnt, leaf_first(ref), pb, S);
+      const uint32_t mask = leaf_step(tris, cnt, leaf_first(ref), pb, S, dense);
       if (cnt > 0u) {
         if (mask) q.leaf(mask, leaf_first(ref));
         ref = sp > 0 ? S.stack[--sp][lane] : kNoRef;
