@@ -301,23 +301,6 @@ __global__ void __launch_bounds__(kClipThreads)
                                 coffs[m], faults, S);
 }
 
-// Walks the tree for box i on one thread; visit(slot, triangle, k) takes its
-// k-th SAT pair.  Returns the traversal status (2 = overflow); *count = pairs.
-template <typename Visit>
-__device__ __forceinline__ int box_pairs(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
-                                         const float* __restrict__ bmin, const float* __restrict__ bmax, int64_t i,
-                                         LcStack& st, uint32_t* count, Visit&& visit) {
-  const float mnx = bmin[3 * i], mny = bmin[3 * i + 1], mnz = bmin[3 * i + 2];
-  const float mxx = bmax[3 * i], mxy = bmax[3 * i + 1], mxz = bmax[3 * i + 2];
-  uint32_t k = 0;
-  const int r = box_traverse(nodes, tris, mnx, mny, mnz, mxx, mxy, mxz, st, [&](const TriRec& t, uint32_t slot) {
-    if (sat_test(t, mnx, mny, mnz, mxx, mxy, mxz)) visit(slot, k++);
-    return false;
-  });
-  *count = k;
-  return r;
-}
-
 // The count pass keeps each box's first kPairsKept pairs, one 32-byte sector:
 // the write pass copies them, and walks the tree again only for the boxes with
 // more (listed by the count pass): 20 + 66 us for 933,270 voxels of 3.07 pairs
@@ -341,20 +324,18 @@ struct PairsWs {
   uint32_t* counts;
   int64_t* offs;
   int64_t* scan_tmp;
-  uint32_t* spill;
   uint32_t* kept;   // [n][kPairsKept] triangle records
   uint32_t* longs;  // boxes with more pairs than are kept
-  unsigned long long* misc;  // [0] spill count, [1] overflow, [2] guard faults, [3] boxes in longs
+  unsigned long long* misc;  // [0] overflow, [1] guard faults, [2] boxes in longs
 };
 
 size_t carve_pairs(PairsWs& w, Workspace& ws, int64_t n) {
   w.counts = ws.take<uint32_t>(n);
   w.offs = ws.take<int64_t>(n + 1);
   w.scan_tmp = ws.take<int64_t>((int64_t)scan_workspace_elems(n));
-  w.spill = ws.take<uint32_t>(n);
   w.kept = ws.take<uint32_t>(n * kPairsKept);
   w.longs = ws.take<uint32_t>(n);
-  w.misc = ws.take<unsigned long long>(4);
+  w.misc = ws.take<unsigned long long>(3);
   return ws.used;
 }
 
@@ -389,7 +370,6 @@ struct CountQuery {
   const float* bmax;
   uint32_t* counts;
   uint8_t* hit;
-  uint32_t* spill;
   uint32_t* kept;
   uint32_t* longs;
   unsigned long long* misc;
@@ -408,12 +388,8 @@ struct CountQuery {
     c += (uint32_t)__popc(mask);
   }
   __device__ __forceinline__ void done(bool overflow) {
-    if (overflow) {
-      spill[atomicAdd(misc, 1ull)] = i;
-      c = 0;
-    } else if (c > (uint32_t)kPairsKept) {
-      longs[atomicAdd(misc + 3, 1ull)] = i;
-    }
+    if (overflow) atomicExch(misc, 1ull);
+    if (c > (uint32_t)kPairsKept) longs[atomicAdd(misc + 2, 1ull)] = i;
     counts[i] = c;
     if (hit) hit[i] = c > 0;
   }
@@ -427,27 +403,6 @@ __global__ void __launch_bounds__(kBoxThreads, kBoxBlocks)
   const int64_t pos = ((int64_t)blockIdx.x * kBoxWarps + (threadIdx.x >> 5)) * per;
   CountQuery q = query;
   box_walk(nodes, tris, pos, pos + per < n ? pos + per : n, smem[threadIdx.x >> 5], q);
-}
-
-__global__ void pairs_count_spill_kernel(const WideNode* __restrict__ nodes, const TriRec* __restrict__ tris,
-                                         CountQuery q) {
-  pdl_wait();
-  const uint64_t m = q.misc[0];
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (uint64_t)gridDim.x * blockDim.x) {
-    const int64_t i = q.spill[t];
-    LcStack st;
-    st.sp = 0;
-    uint32_t c = 0;
-    const int r = box_pairs(nodes, tris, q.bmin, q.bmax, i, st, &c, [&](uint32_t slot, uint32_t k) {
-      if (k < (uint32_t)kPairsKept) q.kept[kPairsKept * i + k] = slot;
-    });
-    if (r == 2) {
-      atomicExch(q.misc + 1, 1ull);
-      c = 0;
-    }
-    q.counts[i] = c;
-    if (q.hit) q.hit[i] = c > 0;
-  }
 }
 
 // the boxes whose pairs were all kept, one a thread
@@ -466,7 +421,7 @@ __global__ void pairs_copy_kernel(const TriRec* __restrict__ tris, int64_t num_s
   const uint32_t r[kPairsKept] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
   for (int k = 0; k < kPairsKept; ++k)
-    if (k < (int)c) put_pair<kSlots>(tris, num_slots, i, r[k], o + k, end, out_box, out_face, w.misc + 2);
+    if (k < (int)c) put_pair<kSlots>(tris, num_slots, i, r[k], o + k, end, out_box, out_face, w.misc + 1);
 }
 
 template <bool kSlots>
@@ -489,7 +444,7 @@ struct WriteQuery {
   __device__ __forceinline__ void leaf(uint32_t mask, uint32_t first) {
     for (; mask; mask &= mask - 1u)
       put_pair<kSlots>(tris, num_slots, i, first + (uint32_t)__ffs((int)mask) - 1u, o++, end, out_box, out_face,
-                       w.misc + 2);
+                       w.misc + 1);
   }
   __device__ __forceinline__ void done(bool) {}
 };
@@ -501,22 +456,7 @@ __global__ void __launch_bounds__(kBoxThreads, kBoxBlocks)
   pdl_wait();
   __shared__ BoxSmem smem[kBoxWarps];
   WriteQuery<kSlots> q = query;
-  box_walk_all(nodes, q.tris, (int64_t)q.w.misc[3], smem[threadIdx.x >> 5], q);
-}
-
-template <bool kSlots>
-__global__ void pairs_write_spill_kernel(const WideNode* __restrict__ nodes, WriteQuery<kSlots> q) {
-  pdl_wait();
-  const uint64_t m = q.w.misc[0];
-  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m; t += (uint64_t)gridDim.x * blockDim.x) {
-    const int64_t i = q.w.spill[t], o = q.w.offs[i], end = q.w.offs[i + 1];
-    LcStack st;
-    st.sp = 0;
-    uint32_t c;
-    box_pairs(nodes, q.tris, q.bmin, q.bmax, i, st, &c, [&](uint32_t slot, uint32_t k) {
-      put_pair<kSlots>(q.tris, q.num_slots, i, slot, o + k, end, q.out_box, q.out_face, q.w.misc + 2);
-    });
-  }
+  box_walk_all(nodes, q.tris, (int64_t)q.w.misc[2], smem[threadIdx.x >> 5], q);
 }
 
 template <bool kSlots>
@@ -528,7 +468,6 @@ int launch_write(const a3d_bvh_view* bvh, const float* bmin, const float* bmax, 
   A3D_PDL(pairs_copy_kernel<kSlots>, dim3((unsigned)ceil_div(n, 256)), dim3(256), 0, s, tris, bvh->num_tris, n, w,
           out_box, out_face);
   A3D_PDL(pairs_write_kernel<kSlots>, dim3((unsigned)box_blocks(n, num_sms())), dim3(kBoxThreads), 0, s, nodes, q);
-  A3D_PDL(pairs_write_spill_kernel<kSlots>, dim3(num_sms() * 4), dim3(64), 0, s, nodes, q);
   return A3D_OK;
 }
 
@@ -571,23 +510,22 @@ extern "C" int a3d_aabb_pairs_count(const a3d_bvh_view* bvh, const float* box_mi
   PairsWs w;
   carve_pairs(w, ws, n);
   A3D_REQUIRE(workspace && ws.ok(), A3D_ERR_WORKSPACE, "aabb_pairs: workspace too small");
-  A3D_CUDA_TRY(cudaMemsetAsync(w.misc, 0, 4 * sizeof(unsigned long long), s));
+  A3D_CUDA_TRY(cudaMemsetAsync(w.misc, 0, 3 * sizeof(unsigned long long), s));
   // modes 2-3: the hit mask comes from the clip
   uint8_t* h = mode == 1 ? hit : nullptr;
   const WideNode* nodes = (const WideNode*)bvh->nodes;
   const TriRec* tris = (const TriRec*)bvh->tris;
   const int64_t per = box_items(n, (int64_t)num_sms() * kBoxBlocks * kBoxWarps);
-  const CountQuery q{box_min, box_max, w.counts, h, w.spill, w.kept, w.longs, w.misc};
+  const CountQuery q{box_min, box_max, w.counts, h, w.kept, w.longs, w.misc};
   A3D_PDL(pairs_count_kernel, dim3((unsigned)ceil_div(n, per * kBoxWarps)), dim3(kBoxThreads), 0, s, nodes, tris, n,
           per, q);
-  A3D_PDL(pairs_count_spill_kernel, dim3(num_sms() * 4), dim3(64), 0, s, nodes, tris, q);
   A3D_TRY((device_exclusive_scan<uint32_t, int64_t>(w.counts, w.offs, n, w.scan_tmp, w.offs + n, s)));
-  unsigned long long misc[4];
+  unsigned long long misc[3];
   int64_t total = 0;
   A3D_CUDA_TRY(cudaMemcpyAsync(misc, w.misc, sizeof(misc), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaMemcpyAsync(&total, w.offs + n, sizeof(total), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
-  A3D_REQUIRE(misc[1] == 0, A3D_ERR_OVERFLOW, "aabb_pairs: traversal stack overflow");
+  A3D_REQUIRE(misc[0] == 0, A3D_ERR_OVERFLOW, "aabb_pairs: traversal stack overflow");
   *num_candidates_out = total;
   return A3D_OK;
 }
@@ -615,13 +553,13 @@ extern "C" int a3d_aabb_pairs_clip(const a3d_bvh_view* bvh, const float* box_min
   if (num_candidates == 0) return A3D_OK;
   A3D_TRY(launch_write<true>(bvh, box_min, box_max, n, w, (int32_t*)c.cand_box, (int32_t*)c.cand_slot, s));
   A3D_PDL(clip_flags_kernel, dim3((unsigned)ceil_div(num_candidates, kClipThreads)), dim3(kClipThreads), 0, s, (const TriRec*)bvh->tris,
-          box_min, box_max, c.cand_box, c.cand_slot, num_candidates, c.flags, hit, n, bvh->num_tris, w.misc + 2);
+          box_min, box_max, c.cand_box, c.cand_slot, num_candidates, c.flags, hit, n, bvh->num_tris, w.misc + 1);
   A3D_TRY((device_exclusive_scan<uint32_t, int64_t>(c.flags, c.coffs, num_candidates, c.scan_tmp,
                                                      c.coffs + num_candidates, s)));
   int64_t total = 0;
   unsigned long long faults = 0;
   A3D_CUDA_TRY(cudaMemcpyAsync(&total, c.coffs + num_candidates, sizeof(total), cudaMemcpyDeviceToHost, s));
-  A3D_CUDA_TRY(cudaMemcpyAsync(&faults, w.misc + 2, sizeof(faults), cudaMemcpyDeviceToHost, s));
+  A3D_CUDA_TRY(cudaMemcpyAsync(&faults, w.misc + 1, sizeof(faults), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
   A3D_REQUIRE(faults == 0, A3D_ERR_OVERFLOW, "aabb_pairs_clip: a candidate index guard fired");
   *num_pairs_out = total;
@@ -657,13 +595,13 @@ extern "C" int a3d_aabb_pairs_write(const a3d_bvh_view* bvh, const float* box_mi
     const unsigned g = (unsigned)ceil_div(num_candidates, kClipThreads);
     if (mode == 2)
       A3D_PDL(clip_emit_kernel<2>, dim3(g), dim3(kClipThreads), 0, s, (const TriRec*)bvh->tris, box_min, box_max, c.cand_box,
-              c.cand_slot, num_candidates, c.flags, c.coffs, out, n, bvh->num_tris, w.misc + 2);
+              c.cand_slot, num_candidates, c.flags, c.coffs, out, n, bvh->num_tris, w.misc + 1);
     else
       A3D_PDL(clip_emit_kernel<3>, dim3(g), dim3(kClipThreads), 0, s, (const TriRec*)bvh->tris, box_min, box_max, c.cand_box,
-              c.cand_slot, num_candidates, c.flags, c.coffs, out, n, bvh->num_tris, w.misc + 2);
+              c.cand_slot, num_candidates, c.flags, c.coffs, out, n, bvh->num_tris, w.misc + 1);
   }
   unsigned long long faults = 0;
-  A3D_CUDA_TRY(cudaMemcpyAsync(&faults, w.misc + 2, sizeof(faults), cudaMemcpyDeviceToHost, s));
+  A3D_CUDA_TRY(cudaMemcpyAsync(&faults, w.misc + 1, sizeof(faults), cudaMemcpyDeviceToHost, s));
   A3D_CUDA_TRY(cudaStreamSynchronize(s));
   A3D_REQUIRE(faults == 0, A3D_ERR_OVERFLOW, "aabb_pairs_write: an output index guard fired");
   return A3D_OK;
