@@ -534,10 +534,16 @@ extern "C" int a3d_octree_traverse(const a3d_bvh_view* bvh, const float* grid_lo
     // / 455; 512^3, 1,310,720 triangles 921 / 978 / 922.)  A tree of one node makes
     // none: its walk is as short as a list (1024^3, a cube's twelve triangles 752
     // us with lists, 684 without, 512^3 334 and 320; twenty of a sphere 440 and 432
-    // at 1024^3).
+    // at 1024^3).  Far from the origin and in tiny grids the margin is of a cell's
+    // size and lists get longer: it counts with the cell, and takes half of one at
+    // most (256^3, 81,920 triangles, a margin of one / two finest cells: 470 / 486 us
+    // without lists, 514 / 618 when it did not count, 469 / 488 so; 512^3, 20,480
+    // triangles: 742 / 749, 508 / 558, 508 / 559).
+    const double near = margin / fmin(g.cell[0], fmin(g.cell[1], g.cell[2]));
     const bool collect = !have_lists && !first_level && level + 2 <= max_level && margin >= 0.0f &&
-                         bvh->num_nodes > 1 &&
-                         bvh->num_tris <= (ncand >= kListFull ? 4 : 1) * ncand;
+                         bvh->num_nodes > 1 && near <= 0.5 &&
+                         (double)bvh->num_tris * (1.0 + near) * (1.0 + near) <=
+                             (ncand >= kListFull ? 4.0 : 1.0) * (double)ncand;
     if (have_lists && last_level)
       A3D_PDL(octree_list_kernel<false>, gk, bk, 0, s, nodes, tris, lv);
     else if (have_lists)
