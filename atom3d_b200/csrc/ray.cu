@@ -787,8 +787,10 @@ __global__ void __launch_bounds__(kRayThreads, kParityBlocks)
       }
       __syncwarp();
     }
-    // (c) finished rays vote, new ones
+    // (c) finished rays vote, new ones; without one the rest is passed by, which a
+    // call of few rays waits for
     const bool done = live && ref == kNoItem;
+    if (!__any_sync(FULL, done)) continue;
     bool vote = false;
     if (done && nh <= kParityHits) {
       // insertion sort by t
