@@ -281,17 +281,18 @@ __device__ __forceinline__ void child_overlap(const WideNode* __restrict__ nodes
 // Each lane compares its triangles' own boxes with its box (about a third of
 // them meet it); the rest of the test, five times as long, is spread evenly
 // over the lanes.  Where the triangles of all lanes make one round of tests, or
-// most of the last step's passed (dense), the comparison costs more than it
-// saves and is left out (1,000 boxes of 342 pairs, 1,310,720 triangles: 994 ->
-// 781 us a call; 5,000 boxes that each hold half of 100,000 triangles 74.9 ->
-// 56.8 ms, 101 with a thread a box).  Returns the mask of the lane's triangles
-// that pass SAT.
+// three quarters of the last step's passed (dense), the comparison costs more
+// than it saves and is left out (1,000 boxes of 342 pairs, 1,310,720 triangles:
+// 994 -> 772 us a call; 5,000 boxes that each hold a quarter of 100,000
+// triangles 74.9 -> 57.2 ms, 101 with a thread a box).  Returns the mask of the
+// lane's triangles that pass SAT.
 __device__ __forceinline__ uint32_t leaf_step(const TriRec* __restrict__ tris, uint32_t cnt, uint32_t first,
                                               const PruneBox& pb, BoxSmem& S, bool& dense) {
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  const bool all = dense || __reduce_add_sync(FULL, cnt) <= 32u;
+  const uint32_t tris_here = __reduce_add_sync(FULL, cnt);
+  const bool all = dense || tris_here <= 32u;
   uint32_t near = all ? (1u << cnt) - 1u : 0u;
   const float4* p = reinterpret_cast<const float4*>(tris + first);
   for (uint32_t k = all ? cnt : 0u; k < cnt; ++k, p += 4) {
@@ -332,7 +333,7 @@ __device__ __forceinline__ uint32_t leaf_step(const TriRec* __restrict__ tris, u
     if (off + num > t0 && off < t0 + 32u) hits |= off >= t0 ? r >> (off - t0) : r << (t0 - off);
   }
   __syncwarp();
-  dense = passed > 0u && 4u * passed >= 3u * total;
+  dense = 4u * passed >= 3u * tris_here;
   uint32_t mask = 0;
   for (uint32_t m = near; m; m &= m - 1u, hits >>= 1)
     if (hits & 1u) mask |= m & (0u - m);
